@@ -2340,6 +2340,57 @@ int32_t ttg_matmat(const ttg_tensor* A, const ttg_tensor* B, ttg_tensor* out)
 // contract_inner_step chain of the product with itself.  The product stays
 // on the device (the reference avoids holding it for host-memory reasons;
 // it is sum_k r_k^A r_k^x m_k r_{k+1}^A r_{k+1}^x doubles of HBM here).
+// Buffers of the inner-product chain of the TTs a and b (ttg_inner.cu): env
+// (doubles of one environment), the scratch [partials | T | value and barrier
+// word] and the largest tile count of one product.
+struct InnerSizes
+{
+  int64_t env = 1, tmp = 1, tiles = 1;
+  int64_t scratch() const { return 2 * kInnerSlices * env + a32(tmp) + 32; }
+};
+
+static InnerSizes inner_sizes(const CoreSlot* a, const CoreSlot* b, int d)
+{
+  InnerSizes z;
+  auto t16 = [](int64_t n) { return (n + 15) / 16; };
+  for (int k = 0; k < d; ++k)
+  {
+    const int64_t n = a[k].n;
+    z.env = std::max({z.env, static_cast<int64_t>(a[k].r) * b[k].r,
+                      static_cast<int64_t>(a[k].rp) * b[k].rp});
+    z.tmp = std::max(z.tmp, b[k].r * n * a[k].rp);
+    z.tiles = std::max({z.tiles, t16(b[k].r) * t16(n * a[k].rp),
+                        std::min<int64_t>(kInnerSlices, (b[k].r * n + 31) / 32) * t16(a[k].rp) *
+                          t16(b[k].rp)});
+  }
+  z.env = a32(z.env);
+  return z;
+}
+
+// Runs the chain on the plan's scratch (sized by InnerSizes) over the cores
+// in `arena` and waits for the value.
+static int32_t run_inner(ttg_plan& P, const double* arena, const CoreSlot* SA, const CoreSlot* SB,
+                         int d, const InnerSizes& z, cudaStream_t st, const char* op, double* out)
+{
+  double* scratch = reinterpret_cast<double*>(static_cast<char*>(P.dev.p) + P.off_scratch);
+  double* tail = scratch + P.scratch_stride - 8;  // value, then the barrier word
+  GridBar* bar = reinterpret_cast<GridBar*>(tail + 1);
+  TTG_CUDA(launch_inner(arena, SA, SB, d, static_cast<int>(std::min<int64_t>(z.tiles, INT32_MAX)),
+                        std::max(device().sms, 1), scratch, z.env, bar, tail, st));
+  g_launches += 1;
+  struct
+  {
+    double v;
+    GridBar bar;
+  } got{};
+  TTG_CUDA(cudaMemcpyAsync(&got, tail, sizeof(got), cudaMemcpyDeviceToHost, st));
+  TTG_CUDA(cudaStreamSynchronize(st));
+  if (got.bar.err)
+    return fail(TTG_ERR_TIMEOUT, std::string(op) + ": a grid barrier wait timed out");
+  *out = got.v;
+  return TTG_OK;
+}
+
 int32_t ttg_frob_norm_apply(const ttg_tensor* a, const ttg_tensor* x, double* out)
 {
   g_err.clear();
@@ -2372,16 +2423,8 @@ int32_t ttg_frob_norm_apply(const ttg_tensor* a, const ttg_tensor* x, double* ou
   if (int32_t st = build_apply_plan(P, A, X, false, nullptr))
     return st;
   const TTInfo ty = P.tts[P.out_tts[0]];
-  int64_t env = 1, tmp = 1;
-  for (int k = 0; k < ty.d; ++k)
-  {
-    const CoreSlot& c = P.slots[ty.first + k];
-    env = std::max(env, static_cast<int64_t>(c.r) * c.r);
-    env = std::max(env, static_cast<int64_t>(c.rp) * c.rp);
-    tmp = std::max(tmp, static_cast<int64_t>(c.r) * c.n * c.rp);
-  }
-  env = a32(env);
-  P.scratch_stride = 2 * env + a32(tmp) + 32;
+  const InnerSizes z = inner_sizes(&P.slots[ty.first], &P.slots[ty.first], ty.d);
+  P.scratch_stride = z.scratch();
   if (int32_t st = layout_and_alloc(P))
     return st;
   cudaStream_t st = lib_stream();
@@ -2390,16 +2433,11 @@ int32_t ttg_frob_norm_apply(const ttg_tensor* a, const ttg_tensor* x, double* ou
   if (int32_t e = plan_run(P, st))
     return e;
   char* d = static_cast<char*>(P.dev.p);
-  double* scratch = reinterpret_cast<double*>(d + P.off_scratch);
   const CoreSlot* S = reinterpret_cast<const CoreSlot*>(d + P.off_slots);
-  launch_inner(reinterpret_cast<double*>(d + P.off_arena), S + ty.first, S + ty.first, ty.d,
-               scratch, env, scratch + P.scratch_stride - 8, st);
-  g_launches += 1;
-  TTG_CUDA(cudaGetLastError());
   double v = 0.0;
-  TTG_CUDA(cudaMemcpyAsync(&v, scratch + P.scratch_stride - 8, sizeof(double),
-                           cudaMemcpyDeviceToHost, st));
-  TTG_CUDA(cudaStreamSynchronize(st));
+  if (int32_t e = run_inner(P, reinterpret_cast<double*>(d + P.off_arena), S + ty.first,
+                            S + ty.first, ty.d, z, st, op, &v))
+    return e;
   *out = std::sqrt(std::max(v, 0.0));
   return TTG_OK;
 }
@@ -2578,15 +2616,8 @@ int32_t ttg_inner(const ttg_tensor* a, const ttg_tensor* b, double* out)
   P.shapes = {A, B};
   add_tensor(P, A, true, nullptr);
   add_tensor(P, B, true, nullptr);
-  int64_t env = 1, tmp = 1;
-  for (int k = 0; k < A.d; ++k)
-  {
-    env = std::max(env, static_cast<int64_t>(A.r[k + 1]) * B.r[k + 1]);
-    env = std::max(env, static_cast<int64_t>(A.r[k]) * B.r[k]);
-    tmp = std::max(tmp, static_cast<int64_t>(B.r[k]) * A.mode(k) * A.r[k + 1]);
-  }
-  env = a32(env);
-  P.scratch_stride = 2 * env + a32(tmp) + 32;
+  const InnerSizes z = inner_sizes(&P.slots[P.tts[0].first], &P.slots[P.tts[1].first], A.d);
+  P.scratch_stride = z.scratch();
   P.grid = 1;
   P.job_kind = -1;
   if (int32_t st = layout_and_alloc(P))
@@ -2594,18 +2625,11 @@ int32_t ttg_inner(const ttg_tensor* a, const ttg_tensor* b, double* out)
   cudaStream_t st = lib_stream();
   if (int32_t e = plan_upload(P, st))
     return e;
-  char* d = static_cast<char*>(P.dev.p);
-  TTG_CUDA(cudaMemcpyAsync(d, d + P.off_pristine, P.prefix_bytes, cudaMemcpyDeviceToDevice, st));
-  double* scratch = reinterpret_cast<double*>(d + P.off_scratch);
+  // The chain only reads the cores: straight from the uploaded copy.
+  const char* d = static_cast<const char*>(P.dev.p) + P.off_pristine;
   const CoreSlot* S = reinterpret_cast<const CoreSlot*>(d + P.off_slots);
-  launch_inner(reinterpret_cast<double*>(d + P.off_arena), S + P.tts[0].first,
-               S + P.tts[1].first, A.d, scratch, env, scratch + P.scratch_stride - 8, st);
-  g_launches += 1;
-  TTG_CUDA(cudaGetLastError());
-  TTG_CUDA(cudaMemcpyAsync(out, scratch + P.scratch_stride - 8, sizeof(double),
-                           cudaMemcpyDeviceToHost, st));
-  TTG_CUDA(cudaStreamSynchronize(st));
-  return TTG_OK;
+  return run_inner(P, reinterpret_cast<const double*>(d + P.off_arena), S + P.tts[0].first,
+                   S + P.tts[1].first, A.d, z, st, "inner", out);
 }
 
 int32_t ttg_device_fp64_peak(double* tflops)

@@ -1,0 +1,122 @@
+// inner (algebra/tt_inner.hpp:33-47): the left-to-right environment chain of
+// contract_inner_step (detail/contract.hpp:155-205) over the whole grid.
+//
+// Per core two dependent products, a grid barrier after each:
+//   T (rb x n rap)  = E^T right_unfold(ca)
+//   E' (rap x rbp)  = T_as(rb n x rap)^T left_unfold(cb)
+// in 16 x 16 FP64 tiles, one per CTA and turn.  E' has few tiles and a long
+// inner dimension, so it is cut into up to kInnerSlices ranges of it, one
+// partial E' each; the next core's T adds the partials, in a fixed order, as
+// it loads E.  What bounds it is the FP64 pipe (2 FMAs per clock per SM),
+// then the 2 d barriers: d = 32, n = 4, rank 96 takes 0.36 GFLOP = 0.29 ms at
+// the chip's FP64 rate; one CTA for the whole chain took 61.7 ms.
+#include <cstdint>
+
+#include <cuda_runtime.h>
+
+#include "ttg_gemm_grid.cuh"
+#include "ttg_gridbar.cuh"
+#include "ttg_kernels.h"
+
+namespace ttg
+{
+namespace
+{
+
+constexpr int kInnerThreads = 256;
+constexpr long long kInnerWaitCycles = 4000000000ll;  // ~2 s
+
+// Slices of the inner dimension K of an (M x N) environment: enough tiles
+// for the grid, at most kInnerSlices, none shorter than a 32-deep slab.
+__host__ __device__ inline int inner_slices(int M, int N, int K, int grid)
+{
+  const int64_t tiles = static_cast<int64_t>((M + 15) / 16) * ((N + 15) / 16);
+  int64_t s = grid / tiles;
+  s = s < (K + 31) / 32 ? s : (K + 31) / 32;
+  s = s < kInnerSlices ? s : kInnerSlices;
+  return s < 1 ? 1 : static_cast<int>(s);
+}
+
+__global__ void __launch_bounds__(kInnerThreads)
+  inner_kernel(const double* __restrict__ ar, const CoreSlot* __restrict__ SA,
+               const CoreSlot* __restrict__ SB, int d, double* scratch, int64_t env_cap, GridBar* bar,
+               double* out)
+{
+  __shared__ double sm[GridTile<1>::kDoubles];
+  const int P = static_cast<int>(gridDim.x), me = static_cast<int>(blockIdx.x);
+  double* E = scratch;
+  double* En = scratch + kInnerSlices * env_cap;
+  double* T = scratch + 2 * kInnerSlices * env_cap;
+  int slices = 0;  // partials of E; 0: the 1 x 1 start
+  for (int k = 0; k < d; ++k)
+  {
+    const int ra = SA[k].r, n = SA[k].n, rap = SA[k].rp;
+    const int rb = SB[k].r, rbp = SB[k].rp;
+    const double* ca = ar + SA[k].off;
+    const double* cb = ar + SB[k].off;
+    const int64_t w = static_cast<int64_t>(n) * rap;
+    const int tn = static_cast<int>((w + 15) / 16);
+    const int t1 = ((rb + 15) / 16) * tn;
+    for (int t = me; t < t1; t += P)
+      grid_tile<1>((t / tn) * 16, (t % tn) * 16, rb, static_cast<int>(w), 0, ra,
+                   [&](int b, int a) {
+                     if (slices == 0)
+                       return 1.0;
+                     const double* e = E + static_cast<int64_t>(a) * rb + b;
+                     double v = __ldcg(e);
+                     for (int s = 1; s < slices; ++s)
+                       v += __ldcg(e + s * env_cap);
+                     return v;
+                   },
+                   [&](int a, int j) { return ca[a * w + j]; },
+                   [&](int b, int j, double v) { T[b * w + j] = v; }, sm, false, false);
+    if (!grid_barrier(bar, P, kInnerWaitCycles))
+      return;
+    const int K = rb * n;
+    slices = inner_slices(rap, rbp, K, P);
+    const int per = (K + slices - 1) / slices;
+    const int tm = (rap + 15) / 16, tn2 = (rbp + 15) / 16;
+    for (int t = me; t < tm * tn2 * slices; t += P)
+    {
+      const int s = t / (tm * tn2), q = t % (tm * tn2);
+      const int k0 = s * per, k1 = k0 + per < K ? k0 + per : K;
+      double* Es = En + s * env_cap;
+      grid_tile<1>((q / tn2) * 16, (q % tn2) * 16, rap, rbp, k0, k1,
+                   [&](int a, int p) { return __ldcg(T + static_cast<int64_t>(p) * rap + a); },
+                   [&](int p, int b) { return cb[static_cast<int64_t>(p) * rbp + b]; },
+                   [&](int a, int b, double v) { Es[static_cast<int64_t>(a) * rbp + b] = v; }, sm,
+                   false, false);
+    }
+    if (!grid_barrier(bar, P, kInnerWaitCycles))
+      return;
+    double* x = E;
+    E = En;
+    En = x;
+  }
+  if (me == 0 && threadIdx.x == 0)
+  {
+    double v = __ldcg(E);
+    for (int s = 1; s < slices; ++s)
+      v += __ldcg(E + s * env_cap);
+    *out = v;
+  }
+}
+
+}  // namespace
+
+cudaError_t launch_inner(const double* ar, const CoreSlot* SA, const CoreSlot* SB, int d, int tiles,
+                         int sms, double* scratch, int64_t env_cap, GridBar* bar, double* out,
+                         cudaStream_t stream)
+{
+  int grid = tiles < sms ? tiles : sms;
+  if (grid < 1)
+    grid = 1;
+  cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(GridBar), stream);
+  if (e != cudaSuccess)
+    return e;
+  void* args[] = {&ar, &SA, &SB, &d, &scratch, &env_cap, &bar, &out};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(inner_kernel), dim3(grid),
+                                     dim3(kInnerThreads), args, 0, stream);
+}
+
+}  // namespace ttg

@@ -124,13 +124,12 @@ enum JobKind : int32_t
   kJobDmrg = 9,           // two-site DMRG rounding, same pairing
 };
 
-// Grid barrier word of the whole-GPU kernel (zeroed before each launch).
+// Grid barrier word of a cooperative kernel (zeroed before each launch):
+// arrivals so far, and whether a wait gave up.
 struct GridBar
 {
   unsigned int count;
-  unsigned int gen;
   int err;
-  int pad;
 };
 
 // Whole-GPU rounding of a few large TTs (wide_round_kernel): the arena,

@@ -13,8 +13,6 @@
 //   fused_matvec/matmat_core         detail/fused_apply_core.hpp:33-272
 //   matvec_core / matmat_core        apply/tt_matrix_apply.hpp:40-224
 //   eval_at / eval_batch             algebra/tt_eval.hpp:32-112
-//   inner (contract_inner_step)      algebra/tt_inner.hpp:33-47,
-//                                    detail/contract.hpp:155-205
 #include <cuda_runtime.h>
 
 #include "ttg_device.cuh"
@@ -1601,40 +1599,6 @@ __global__ void __launch_bounds__(kThreads) eval_kernel(const double* __restrict
   }
 }
 
-// inner (algebra/tt_inner.hpp:33-47): one CTA runs the left-to-right
-// environment chain of contract_inner_step (detail/contract.hpp:155-205).
-__global__ void __launch_bounds__(kThreads) inner_kernel(const double* __restrict__ ar,
-                                                         const CoreSlot* __restrict__ SA,
-                                                         const CoreSlot* __restrict__ SB, int d,
-                                                         double* scratch, int64_t env_cap,
-                                                         double* out)
-{
-  __shared__ CtaShared sh;
-  double* E = scratch;
-  double* En = scratch + env_cap;
-  double* tmp = scratch + 2 * env_cap;
-  if (threadIdx.x == 0)
-    E[0] = 1.0;
-  __syncthreads();
-  for (int k = 0; k < d; ++k)
-  {
-    const int ra = SA[k].r, n = SA[k].n, rap = SA[k].rp;
-    const int rb = SB[k].r, rbp = SB[k].rp;
-    const double* ca = ar + SA[k].off;
-    const double* cb = ar + SB[k].off;
-    // tmp (rb x n*rap) = E^T * right_unfold(ca).
-    cta_gemm(rb, n * rap, ra, View{E, 1, rb}, View{ca, static_cast<int64_t>(n) * rap, 1}, tmp,
-             static_cast<int64_t>(n) * rap, 1, sh);
-    // En (rap x rbp) = tmp_as^T (rap x rb*n) * left_unfold(cb) (rb*n x rbp).
-    cta_gemm(rap, rbp, rb * n, View{tmp, 1, rap}, View{cb, rbp, 1}, En, rbp, 1, sh);
-    double* t = E;
-    E = En;
-    En = t;
-  }
-  if (threadIdx.x == 0)
-    *out = E[0];
-}
-
 void launch_round(const RoundJob& job, int grid, int ctas_per_sm, cudaStream_t stream)
 {
   const size_t smem = sizeof(double) * static_cast<size_t>(job.smem_doubles);
@@ -1676,12 +1640,6 @@ void launch_eval(const double* ar, const CoreSlot* S, int d, const int* idx, int
 {
   const size_t smem = static_cast<size_t>(kWarps) * 2 * rcap * sizeof(double);
   eval_kernel<<<grid, kThreads, smem, stream>>>(ar, S, d, idx, M, out, rcap, bad);
-}
-
-void launch_inner(const double* ar, const CoreSlot* SA, const CoreSlot* SB, int d,
-                  double* scratch, int64_t env_cap, double* out, cudaStream_t stream)
-{
-  inner_kernel<<<1, kThreads, 0, stream>>>(ar, SA, SB, d, scratch, env_cap, out);
 }
 
 // Eight independent DFMA chains per thread (operands from kernel

@@ -32,6 +32,7 @@
 
 #include "ttg_device.cuh"
 #include "ttg_device_df.cuh"
+#include "ttg_gridbar.cuh"
 #include "ttg_job.h"
 #include "ttg_kernels.h"
 #include "ttg_ozaki.cuh"
@@ -40,57 +41,12 @@
 namespace ttg
 {
 
-// Bounded barrier of the `count` CTAs of a team (the whole grid, or a group
-// of it), by generation counter.  All CTAs are co-resident (cooperative
-// launch).  Returns false once any CTA of the team timed out (after
-// `limit` clock cycles of waiting).
-__device__ bool grid_sync(GridBar* gb, unsigned int count, long long limit)
-{
-  __shared__ int ok_sh;
-  __syncthreads();
-  if (threadIdx.x == 0)
-  {
-    int ok = 1;
-    volatile unsigned int* genp = &gb->gen;
-    volatile int* errp = &gb->err;
-    const unsigned int g = *genp;
-    __threadfence();
-    if (atomicAdd(&gb->count, 1u) == count - 1)
-    {
-      atomicExch(&gb->count, 0u);
-      __threadfence();
-      atomicAdd(&gb->gen, 1u);
-    }
-    else
-    {
-      const long long t0 = clock64();
-      while (*genp == g)
-      {
-        if (*errp)
-          break;
-        if (clock64() - t0 > limit)
-        {
-          atomicExch(&gb->err, 1);
-          break;
-        }
-        __nanosleep(64);
-      }
-    }
-    __threadfence();
-    if (*errp)
-      ok = 0;
-    ok_sh = ok;
-  }
-  __syncthreads();
-  return ok_sh != 0;
-}
-
 // The team's barrier.  job.stall_waits (set only by the failure-path tests)
 // counts one CTA more than the team holds, so that no barrier ever
 // completes and every wait runs out after job.wait_cycles.
 __device__ bool grid_sync(const WideJob& job)
 {
-  return grid_sync(job.bar, job.size + (job.stall_waits ? 1u : 0u), job.wait_cycles);
+  return grid_barrier(job.bar, job.size + (job.stall_waits ? 1u : 0u), job.wait_cycles);
 }
 
 #define WSYNC()                 \
