@@ -81,22 +81,33 @@ __device__ bool wait_bounded(uint64_t* mbar, uint32_t parity, long long limit = 
   return true;
 }
 
-// BF16 planes (rows_pad x kpad, row-major) of X(i, p) = X[i*rs + p*cs],
-// i < rows, p < K, zero elsewhere.
-__global__ void split_planes_kernel(const float* __restrict__ X, int64_t rs, int64_t cs, int rows,
-                                    int K, int rows_pad, int kpad, __nv_bfloat16* hi,
-                                    __nv_bfloat16* lo)
+// One operand's planes: hi and lo (may be null), rows_pad x kpad row-major,
+// of X(i, p) = X[i*rs + p*cs] (of max(X, 0) with relu) for i < rows, p < K,
+// zero elsewhere.
+struct PlaneArgs
 {
-  const int64_t total = static_cast<int64_t>(rows_pad) * kpad;
+  const float* X;
+  int64_t rs, cs;
+  int rows, rows_pad, relu;
+  __nv_bfloat16 *hi, *lo;
+};
+
+// Both operands' planes in one launch (blockIdx.y picks the operand).
+__global__ void split_planes_kernel(PlaneArgs a, PlaneArgs b, int K, int kpad)
+{
+  const PlaneArgs& o = blockIdx.y == 0 ? a : b;
+  const int64_t total = static_cast<int64_t>(o.rows_pad) * kpad;
   for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total;
        t += static_cast<int64_t>(gridDim.x) * blockDim.x)
   {
     const int i = static_cast<int>(t / kpad), p = static_cast<int>(t % kpad);
-    const float x = (i < rows && p < K) ? X[i * rs + p * cs] : 0.f;
+    float x = (i < o.rows && p < K) ? o.X[i * o.rs + p * o.cs] : 0.f;
+    if (o.relu)
+      x = fmaxf(x, 0.f);
     const __nv_bfloat16 h = __float2bfloat16_rn(x);
-    hi[t] = h;
-    if (lo)
-      lo[t] = __float2bfloat16_rn(x - __bfloat162float(h));
+    o.hi[t] = h;
+    if (o.lo)
+      o.lo[t] = __float2bfloat16_rn(x - __bfloat162float(h));
   }
 }
 
@@ -327,8 +338,23 @@ bool make_plane_map(CUtensorMap* map, void* base, int rows, int kpad, int box_ro
             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Tile and plane sizes of an M x N x K product with BN-wide tiles.
+struct PlaneSizes
+{
+  int mt, nt, mpad, npad, kpad;
+  size_t bytes;
+  PlaneSizes(int M, int N, int K, int BN, bool three)
+    : mt((M + kBM - 1) / kBM), nt((N + BN - 1) / BN), mpad(mt * kBM), npad(nt * BN),
+      kpad(((K + kBK - 1) / kBK) * kBK),
+      bytes((static_cast<size_t>(mpad) + npad) * kpad * (three ? 2 : 1) * sizeof(__nv_bfloat16))
+  {
+  }
+};
+
+int bn_of(int N) { return N > 64 ? 128 : (N > 32 ? 64 : 32); }
+
 template <int BN>
-cudaError_t launch_bn(const TcGemmArgs& g, cudaStream_t st)
+cudaError_t launch_bn(const TcGemmArgs& g, bool relu_a, void* own_ws, cudaStream_t st)
 {
   static std::once_flag once[64];
   int dev = 0;
@@ -340,38 +366,43 @@ cudaError_t launch_bn(const TcGemmArgs& g, cudaStream_t st)
   });
   if (attr != cudaSuccess)
     return attr;
-  const int mt = (g.M + kBM - 1) / kBM, nt = (g.N + BN - 1) / BN;
-  const int mpad = mt * kBM, npad = nt * BN;
-  const int kpad = ((g.K + kBK - 1) / kBK) * kBK;
-  const int nk = kpad / kBK;
   const bool three = g.splits == 3;
+  const PlaneSizes z(g.M, g.N, g.K, BN, three);
+  const int mt = z.mt, nt = z.nt, mpad = z.mpad, npad = z.npad, kpad = z.kpad;
+  const int nk = kpad / kBK;
   CUtensorMap mAh{}, mAl{}, mBh{}, mBl{};
   __nv_bfloat16* ws = nullptr;
   if (nk > 0)
   {
-    // Stream-ordered workspace: calls on other streams get their own.
+    // The caller's workspace, else a stream-ordered one (calls on other
+    // streams get their own; it costs an allocation per call once the
+    // stream was waited for, since the pool gives its memory back then).
     const size_t a_elems = static_cast<size_t>(mpad) * kpad, b_elems = static_cast<size_t>(npad) * kpad;
-    const size_t bytes = (a_elems + b_elems) * (three ? 2 : 1) * sizeof(__nv_bfloat16);
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&ws), bytes, st);
-    if (e != cudaSuccess)
-      return e;
+    if (own_ws)
+      ws = static_cast<__nv_bfloat16*>(own_ws);
+    else
+    {
+      cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&ws), z.bytes, st);
+      if (e != cudaSuccess)
+        return e;
+    }
     __nv_bfloat16* ah = ws;
     __nv_bfloat16* bh = ah + a_elems;
     __nv_bfloat16* al = three ? bh + b_elems : nullptr;
     __nv_bfloat16* bl = three ? al + a_elems : nullptr;
     const int threads = 256;
-    const int blocks_a = static_cast<int>(std::min<size_t>((a_elems + threads - 1) / threads, 4096));
-    const int blocks_b = static_cast<int>(std::min<size_t>((b_elems + threads - 1) / threads, 4096));
-    split_planes_kernel<<<blocks_a, threads, 0, st>>>(g.A, g.a_rs, g.a_cs, g.M, g.K, mpad, kpad,
-                                                      ah, al);
+    const size_t most = std::max(a_elems, b_elems);
+    const int blocks = static_cast<int>(std::min<size_t>((most + threads - 1) / threads, 4096));
     // B^T (N x K): element (j, p) = B(p, j) = B[p*b_rs + j*b_cs].
-    split_planes_kernel<<<blocks_b, threads, 0, st>>>(g.B, g.b_cs, g.b_rs, g.N, g.K, npad, kpad,
-                                                      bh, bl);
+    split_planes_kernel<<<dim3(blocks, 2), threads, 0, st>>>(
+      PlaneArgs{g.A, g.a_rs, g.a_cs, g.M, mpad, relu_a ? 1 : 0, ah, al},
+      PlaneArgs{g.B, g.b_cs, g.b_rs, g.N, npad, 0, bh, bl}, g.K, kpad);
     if (!make_plane_map(&mAh, ah, mpad, kpad, kBM) || !make_plane_map(&mBh, bh, npad, kpad, BN) ||
         (three && (!make_plane_map(&mAl, al, mpad, kpad, kBM) ||
                    !make_plane_map(&mBl, bl, npad, kpad, BN))))
     {
-      cudaFreeAsync(ws, st);
+      if (!own_ws)
+        cudaFreeAsync(ws, st);
       return cudaErrorInvalidValue;
     }
     if (!three)
@@ -383,7 +414,7 @@ cudaError_t launch_bn(const TcGemmArgs& g, cudaStream_t st)
   dim3 grid(mt, nt);
   tc_gemm_tma_kernel<BN><<<grid, kTcThreads, tc_smem_bytes<BN>(), st>>>(mAh, mAl, mBh, mBl, g, nk);
   cudaError_t e = cudaGetLastError();
-  if (ws)
+  if (ws && !own_ws)
     cudaFreeAsync(ws, st);
   return e;
 }
@@ -406,7 +437,8 @@ int* error_flag()
 
 cudaError_t tc_gemm_f32(cudaStream_t st, int M, int N, int K, const float* A, int64_t a_rs,
                         int64_t a_cs, const float* B, int64_t b_rs, int64_t b_cs, float* C,
-                        int64_t ldc, const float* bias, bool relu, bool accumulate, int splits)
+                        int64_t ldc, const float* bias, bool relu, bool accumulate, int splits,
+                        bool relu_a, void* ws)
 {
   if (M <= 0 || N <= 0)
     return cudaSuccess;
@@ -417,11 +449,20 @@ cudaError_t tc_gemm_f32(cudaStream_t st, int M, int N, int K, const float* A, in
   TcGemmArgs g{M, N, K, A, a_rs, a_cs, B, b_rs, b_cs, C, ldc, bias,
                relu ? 1 : 0, accumulate ? 1 : 0, splits, err,
                (stall && stall[0] == '1') ? 1 : 0};
-  if (N > 64)
-    return launch_bn<128>(g, st);
-  if (N > 32)
-    return launch_bn<64>(g, st);
-  return launch_bn<32>(g, st);
+  switch (bn_of(N))
+  {
+    case 128:
+      return launch_bn<128>(g, relu_a, ws, st);
+    case 64:
+      return launch_bn<64>(g, relu_a, ws, st);
+    default:
+      return launch_bn<32>(g, relu_a, ws, st);
+  }
+}
+
+size_t tc_gemm_ws_bytes(int M, int N, int K, int splits)
+{
+  return PlaneSizes(M, N, K, bn_of(N), splits == 3).bytes;
 }
 
 // Reads and clears the timeout flag of the current device (synchronises st).

@@ -36,3 +36,30 @@ def test_mlp_training_reduces_loss(ttg):
     hist = m.train(x, t, epochs=40, lr=3e-3, batch=2048)
     assert hist[-1] < 0.1 * hist[0]
     assert m.kernel_launches() > 0
+
+
+@pytest.mark.parametrize("F,H,rows", [(10, 128, 4096), (1, 128, 1), (32, 128, 33), (7, 31, 31),
+                                      (10, 97, 6000), (33, 128, 64), (10, 160, 200)])
+def test_mlp_gradients_at_the_edges_of_the_fused_backward(ttg, F, H, rows):
+    # Rows not a multiple of 32 or more than the CTAs hold at once, widths and
+    # feature counts at and past the kernel's limits (the wider models run
+    # their GEMMs).  Small weights under biases of +-1 keep every
+    # pre-activation away from zero, so no ReLU mask hangs on a rounding: what
+    # is left is the products' 2^-16 per term, within the tolerance of the
+    # test above.
+    from tensor_train_gb300.mlp import RankModel
+    m = RankModel(F, H, seed=5)
+    rng = np.random.default_rng(F * H + rows)
+    w = rng.uniform(-1, 1, m.num_params).astype(np.float32) / (16 * H)
+    sign = np.where(np.arange(H) % 3 == 1, -1.0, 1.0)
+    w[F * H:F * H + H] = sign
+    w[F * H + H + H * H:F * H + 2 * H + H * H] = np.roll(sign, 1)
+    w[F * H + 2 * H + H * H:-1] = rng.uniform(-1, 1, H)
+    m.set_params(w)
+    x = rng.standard_normal((rows, F)).astype(np.float32)
+    t = rng.standard_normal(rows).astype(np.float32)
+    p = m.params()
+    g, loss = m.gradients(x, t)
+    lr, gr = mlp_ref.loss_and_grad(p, x, t, F, H)
+    assert abs(loss - lr) <= 1e-4 * (1 + lr)
+    assert np.linalg.norm(g - gr) <= 1e-4 * np.linalg.norm(gr)
