@@ -18,10 +18,11 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"]
 
 SOURCES = ["ttg_kernels.cu", "ttg_wide.cu", "ttg_api.cpp", "ttg_host.cpp", "ttg_noalloc.cu",
-           "ttg_mlp.cu", "ttg_tc_gemm.cu", "ttg_shard.cpp", "ttg_inner.cu"]
+           "ttg_mlp.cu", "ttg_tc_gemm.cu", "ttg_shard.cpp", "ttg_inner.cu",
+           "ttg_eval.cu"]
 HEADERS = ["ttg_device.cuh", "ttg_device_df.cuh", "ttg_df64.cuh", "ttg_job.h", "ttg_kernels.h",
            "ttg_tc.cuh", "ttg_sweep_common.cuh", "ttg_ozaki.cuh", "ttg_wy_df.cuh", "ttg_gemm_live.h",
-           "ttg_gridbar.cuh", "ttg_gemm_grid.cuh", "ttg_mlp_back.cuh"]
+           "ttg_gridbar.cuh", "ttg_gemm_grid.cuh", "ttg_mlp_back.cuh", "ttg_eval.h"]
 
 
 def _nvcc() -> str:

@@ -22,6 +22,7 @@
 
 #include "../../include/ttg.h"
 #include "ttg_job.h"
+#include "ttg_eval.h"
 #include "ttg_kernels.h"
 
 using namespace ttg;
@@ -298,7 +299,10 @@ struct ttg_plan
   const int32_t* eval_idx = nullptr;
   int64_t M = 0;
   int rcap = 0;
-  size_t off_idx = 0, off_out = 0, off_bad = 0;
+  size_t off_idx = 0, off_out = 0, off_bad = 0, off_segs = 0, off_modes = 0, off_tables = 0;
+  EvalLayout eval_layout;
+  std::vector<EvalSeg> eval_segs;
+  std::vector<EvalMerge> eval_merges;
   int64_t h2d = 0, d2h = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, evk0 = nullptr, evk1 = nullptr;
   bool kernel_timed = false;
@@ -851,15 +855,13 @@ int32_t plan_run(ttg_plan& P, cudaStream_t st)
   {
     TTG_CUDA(cudaMemsetAsync(d + P.off_bad, 0, sizeof(int), st));
     const Shape& s = P.shapes[0];
-    const int sms = std::max(device().sms, 1);
-    const int64_t warps_needed = (P.M + 7) / 8;
-    const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(warps_needed, 8LL * sms)));
-    launch_eval(reinterpret_cast<double*>(d + P.off_arena),
-                reinterpret_cast<CoreSlot*>(d + P.off_slots), s.d,
+    launch_eval(P.eval_merges, reinterpret_cast<const EvalSeg*>(d + P.off_segs),
+                P.eval_layout.left, static_cast<int>(P.eval_segs.size()),
+                reinterpret_cast<const int*>(d + P.off_modes), s.d,
                 reinterpret_cast<const int*>(d + P.off_idx), P.M,
-                reinterpret_cast<double*>(d + P.off_out), P.rcap,
-                reinterpret_cast<int*>(d + P.off_bad), grid, st);
-    g_launches += 1;
+                reinterpret_cast<double*>(d + P.off_out), *std::max_element(s.r.begin(), s.r.end()),
+                P.rcap, reinterpret_cast<int*>(d + P.off_bad), std::max(device().sms, 1), st);
+    g_launches += 1 + static_cast<int64_t>(P.eval_merges.size());
     TTG_CUDA(cudaGetLastError());
     return TTG_OK;
   }
@@ -2480,7 +2482,40 @@ int32_t ttg_plan_create_matvec_round(const ttg_tensor* a, const ttg_tensor* x,
 // ---------------------------------------------------------------------------
 // eval_batch, inner, norm.
 // ---------------------------------------------------------------------------
-static int32_t build_eval_plan(ttg_plan& P, const ttg_tensor* a, const int32_t* idx, int32_t M)
+// Whether products of neighbouring cores stay inside FP64's range wherever
+// the products with a row vector do: every partial sum of the cores' exponents
+// (of the largest entry, plus half the rank's for the sum over it) within 2^800
+// of every other, and no infinity or NaN.  The index-by-index products of such
+// a train neither overflow nor lose anything above 2^-1000 of its scale, and a
+// table spans at most 14 sites, 4 bits each.
+static bool eval_products_safe(const Shape& s)
+{
+  double sum = 0.0, lo = 0.0, hi = 0.0;
+  for (int k = 0; k < s.d; ++k)
+  {
+    const double* x = s.data + s.src_off[k];
+    uint64_t top = 0;
+    for (int64_t i = 0; i < s.size[k]; ++i)
+    {
+      uint64_t u;
+      std::memcpy(&u, x + i, sizeof(u));
+      u &= 0x7ff0000000000000ull;
+      top = u > top ? u : top;
+    }
+    const int e = static_cast<int>(top >> 52);
+    if (e == 0x7ff)
+      return false;
+    if (e == 0)
+      continue;  // a zero core: every product with it is zero
+    sum += e - 1023 + 0.5 * std::log2(static_cast<double>(s.r[k + 1]));
+    lo = std::min(lo, sum);
+    hi = std::max(hi, sum);
+  }
+  return hi - lo <= 800.0;
+}
+
+static int32_t build_eval_plan(ttg_plan& P, const ttg_tensor* a, const int32_t* idx, int32_t M,
+                               int32_t M_all)
 {
   Shape s;
   if (int32_t st = describe(a, "eval_batch", s))
@@ -2505,15 +2540,22 @@ static int32_t build_eval_plan(ttg_plan& P, const ttg_tensor* a, const int32_t* 
   P.rcap = (rmax + 31) / 32 * 32;
   if (P.rcap > 1536)
     return fail(TTG_ERR_NO_SPACE, "eval_batch: ranks above 1536 are not served");
-  TTG_CUDA(eval_smem_optin(P.rcap));
-  // layout: [arena | slots | tts | idx] prefix, then [out | bad].
+  std::vector<int> modes(static_cast<size_t>(s.d));
+  for (int k = 0; k < s.d; ++k)
+    modes[k] = s.mode(k);
+  P.eval_layout = plan_eval(s.r.data(), modes.data(), s.d, M_all);
+  if (P.eval_layout.tables && !eval_products_safe(s))
+    plain_eval(P.eval_layout, modes.data(), s.d);
+  const int nseg = static_cast<int>(P.eval_layout.cut.size()) - 1;
+  TTG_CUDA(eval_smem_optin(nseg, s.d, rmax, P.rcap));
+  // layout: [arena | segments | modes | idx] prefix, then [out | bad | tables].
   size_t o = 0;
   P.off_arena = o;
   o = align256(o + sizeof(double) * static_cast<size_t>(P.arena_doubles));
-  P.off_slots = o;
-  o = align256(o + sizeof(CoreSlot) * P.slots.size());
-  P.off_tts = o;
-  o = align256(o + sizeof(TTInfo) * P.tts.size());
+  P.off_segs = o;
+  o = align256(o + sizeof(EvalSeg) * static_cast<size_t>(nseg));
+  P.off_modes = o;
+  o = align256(o + sizeof(int32_t) * static_cast<size_t>(s.d));
   P.off_order = o;
   const size_t table_end = o;
   P.off_idx = o;
@@ -2523,17 +2565,26 @@ static int32_t build_eval_plan(ttg_plan& P, const ttg_tensor* a, const int32_t* 
   o = align256(o + sizeof(double) * static_cast<size_t>(std::max<int64_t>(M, 1)));
   P.off_bad = o;
   o = align256(o + 256);
+  P.off_tables = o;
+  o = align256(o + sizeof(double) * static_cast<size_t>(P.eval_layout.table_doubles));
   P.total_bytes = o;
   TTG_CUDA(P.dev.ensure(P.total_bytes));
   TTG_CUDA(P.host.ensure(table_end));
   char* h = static_cast<char*>(P.host.p);
-  std::memset(h, 0, table_end);
+  char* dv = static_cast<char*>(P.dev.p);
+  std::vector<int64_t> off(static_cast<size_t>(s.d));
   double* arena = reinterpret_cast<double*>(h + P.off_arena);
   for (int k = 0; k < s.d; ++k)
-    std::memcpy(arena + P.slots[k].off, s.data + s.src_off[k],
+  {
+    off[k] = P.slots[k].off;
+    std::memcpy(arena + off[k], s.data + s.src_off[k],
                 sizeof(double) * static_cast<size_t>(s.size[k]));
-  std::memcpy(h + P.off_slots, P.slots.data(), sizeof(CoreSlot) * P.slots.size());
-  std::memcpy(h + P.off_tts, P.tts.data(), sizeof(TTInfo) * P.tts.size());
+  }
+  lay_out_eval(P.eval_layout, s.r.data(), modes.data(), off.data(), s.d,
+               reinterpret_cast<const double*>(dv + P.off_arena),
+               reinterpret_cast<double*>(dv + P.off_tables), P.eval_segs, P.eval_merges);
+  std::memcpy(h + P.off_segs, P.eval_segs.data(), sizeof(EvalSeg) * P.eval_segs.size());
+  std::memcpy(h + P.off_modes, modes.data(), sizeof(int32_t) * modes.size());
   P.h2d = static_cast<int64_t>(table_end + sizeof(int32_t) * static_cast<size_t>(M) * s.d);
   P.d2h = static_cast<int64_t>(sizeof(double) * M + sizeof(int));
   return TTG_OK;
@@ -2558,7 +2609,7 @@ int32_t ttg_plan_create_eval(const ttg_tensor* a, const int32_t* idx, int32_t M,
   if (int32_t st = need_device())
     return st;
   auto* P = new ttg_plan;
-  if (int32_t st = build_eval_plan(*P, a, idx, M))
+  if (int32_t st = build_eval_plan(*P, a, idx, M, M))
   {
     delete P;
     return st;
@@ -2569,23 +2620,7 @@ int32_t ttg_plan_create_eval(const ttg_tensor* a, const int32_t* idx, int32_t M,
 
 int32_t ttg_eval_batch(const ttg_tensor* a, const int32_t* idx, int32_t M, double* out)
 {
-  g_err.clear();
-  if (!out && M > 0)
-    return fail(TTG_ERR_ARG, "eval_batch: null output");
-  if (int32_t st = need_device())
-    return st;
-  std::lock_guard<std::mutex> lk(dev_state().mu);
-  ttg_plan P;
-  if (int32_t st = build_eval_plan(P, a, idx, M))
-    return st;
-  if (M == 0)
-    return TTG_OK;
-  cudaStream_t st = lib_stream();
-  if (int32_t e = eval_upload(P, st))
-    return e;
-  if (int32_t e = plan_run(P, st))
-    return e;
-  return ttg_plan_download(&P, st, nullptr, out, nullptr);
+  return ttg::eval_batch_part(a, idx, M, M, out);
 }
 
 int32_t ttg_inner(const ttg_tensor* a, const ttg_tensor* b, double* out)
@@ -2671,3 +2706,25 @@ int32_t ttg_norm(const ttg_tensor* a, double* out)
 }
 
 }  // extern "C"
+
+int32_t ttg::eval_batch_part(const ttg_tensor* a, const int32_t* idx, int32_t M, int32_t M_all,
+                             double* out)
+{
+  g_err.clear();
+  if (!out && M > 0)
+    return fail(TTG_ERR_ARG, "eval_batch: null output");
+  if (int32_t st = need_device())
+    return st;
+  std::lock_guard<std::mutex> lk(dev_state().mu);
+  ttg_plan P;
+  if (int32_t st = build_eval_plan(P, a, idx, M, M_all))
+    return st;
+  if (M == 0)
+    return TTG_OK;
+  cudaStream_t st = lib_stream();
+  if (int32_t e = eval_upload(P, st))
+    return e;
+  if (int32_t e = plan_run(P, st))
+    return e;
+  return ttg_plan_download(&P, st, nullptr, out, nullptr);
+}

@@ -12,7 +12,6 @@
 //   build_streaming_matvec/matmat    detail/streaming_apply.hpp:39-202
 //   fused_matvec/matmat_core         detail/fused_apply_core.hpp:33-272
 //   matvec_core / matmat_core        apply/tt_matrix_apply.hpp:40-224
-//   eval_at / eval_batch             algebra/tt_eval.hpp:32-112
 #include <cuda_runtime.h>
 
 #include "ttg_device.cuh"
@@ -1533,72 +1532,6 @@ __global__ void apply_core_kernel(const double* __restrict__ Ac, const double* _
   }
 }
 
-// eval_batch: one warp per multi-index; the running row vector lives in
-// shared memory (two buffers per warp of `rcap` doubles).
-__global__ void __launch_bounds__(kThreads) eval_kernel(const double* __restrict__ ar,
-                                                        const CoreSlot* __restrict__ S, int d,
-                                                        const int* __restrict__ idx, int64_t M,
-                                                        double* __restrict__ out, int rcap,
-                                                        int* __restrict__ bad)
-{
-  extern __shared__ double evbuf[];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  double* v = evbuf + static_cast<int64_t>(w) * 2 * rcap;
-  double* vn = v + rcap;
-  const int64_t warps_total = static_cast<int64_t>(gridDim.x) * kWarps;
-  for (int64_t smp = blockIdx.x * static_cast<int64_t>(kWarps) + w; smp < M; smp += warps_total)
-  {
-    const int* ix = idx + smp * d;
-    int i0 = ix[0];
-    bool ok = (i0 >= 0 && i0 < S[0].n);
-    for (int k = 1; k < d; ++k)
-    {
-      const int ik = ix[k];
-      ok = ok && (ik >= 0 && ik < S[k].n);
-    }
-    if (!ok)
-    {
-      if (lane == 0)
-      {
-        out[smp] = __longlong_as_double(0x7ff8000000000000ll);
-        atomicExch(bad, 1);
-      }
-      continue;
-    }
-    {
-      const int r1 = S[0].rp;
-      const double* c0 = ar + S[0].off + static_cast<int64_t>(i0) * r1;
-      for (int b = lane; b < r1; b += 32)
-        v[b] = c0[b];
-    }
-    __syncwarp();
-    for (int k = 1; k < d; ++k)
-    {
-      const int r = S[k].r, n = S[k].n, rp = S[k].rp;
-      const int ik = ix[k];
-      const double* ck = ar + S[k].off + static_cast<int64_t>(ik) * rp;
-      const int64_t stride = static_cast<int64_t>(n) * rp;
-      for (int b0 = 0; b0 < rp; b0 += 32)
-      {
-        const int b = b0 + lane;
-        double acc = 0.0;
-        if (b < rp)
-          for (int a = 0; a < r; ++a)
-            acc = fma(v[a], ck[a * stride + b], acc);
-        if (b < rp)
-          vn[b] = acc;
-      }
-      __syncwarp();
-      double* t = v;
-      v = vn;
-      vn = t;
-    }
-    if (lane == 0)
-      out[smp] = v[0];
-    __syncwarp();
-  }
-}
-
 void launch_round(const RoundJob& job, int grid, int ctas_per_sm, cudaStream_t stream)
 {
   const size_t smem = sizeof(double) * static_cast<size_t>(job.smem_doubles);
@@ -1635,13 +1568,6 @@ void launch_apply_core(const double* A, const double* X, double* Y, int r, int m
                                                                   sp);
 }
 
-void launch_eval(const double* ar, const CoreSlot* S, int d, const int* idx, int64_t M,
-                 double* out, int rcap, int* bad, int grid, cudaStream_t stream)
-{
-  const size_t smem = static_cast<size_t>(kWarps) * 2 * rcap * sizeof(double);
-  eval_kernel<<<grid, kThreads, smem, stream>>>(ar, S, d, idx, M, out, rcap, bad);
-}
-
 // Eight independent DFMA chains per thread (operands from kernel
 // parameters); one store per thread into out[grid*block].
 __global__ void fp64_peak_kernel(double* out, int iters, double a, double b)
@@ -1664,13 +1590,6 @@ __global__ void fp64_peak_kernel(double* out, int iters, double a, double b)
 void launch_fp64_peak(double* out, int iters, int grid, int block, cudaStream_t stream)
 {
   fp64_peak_kernel<<<grid, block, 0, stream>>>(out, iters, 0.999, 0.001);
-}
-
-cudaError_t eval_smem_optin(int rcap)
-{
-  const size_t smem = static_cast<size_t>(kWarps) * 2 * rcap * sizeof(double);
-  return cudaFuncSetAttribute(eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              static_cast<int>(smem));
 }
 
 }  // namespace ttg

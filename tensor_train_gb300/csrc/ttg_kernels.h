@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include "../../include/ttg.h"
 #include "ttg_job.h"
 
 namespace ttg
@@ -18,8 +19,6 @@ cudaError_t launch_wide_round(const WideJob& job, int grid, cudaStream_t stream)
 cudaError_t wide_round_setup(int smem_doubles, int* max_grid);
 void launch_apply_core(const double* A, const double* X, double* Y, int r, int m, int p, int rp,
                        int s, int nout, int sp, cudaStream_t stream);
-void launch_eval(const double* ar, const CoreSlot* S, int d, const int* idx, int64_t M,
-                 double* out, int rcap, int* bad, int grid, cudaStream_t stream);
 // Partial environments of the inner-product chain (ttg_inner.cu).
 constexpr int kInnerSlices = 4;
 // <a, b> of two TTs in `ar` into *out (cooperative).  tiles: the most 16 x 16
@@ -28,7 +27,6 @@ constexpr int kInnerSlices = 4;
 cudaError_t launch_inner(const double* ar, const CoreSlot* SA, const CoreSlot* SB, int d, int tiles,
                          int sms, double* scratch, int64_t env_cap, GridBar* bar, double* out,
                          cudaStream_t stream);
-cudaError_t eval_smem_optin(int rcap);
 cudaError_t round_smem_optin(int smem_doubles);
 void launch_fp64_peak(double* out, int iters, int grid, int block, cudaStream_t stream);
 // tcgen05 split-BF16 GEMM (ttg_tc_gemm.cu): C = A B (+ bias) (relu) (+ C),
@@ -41,6 +39,10 @@ cudaError_t tc_gemm_f32(cudaStream_t st, int M, int N, int K, const float* A, in
 size_t tc_gemm_ws_bytes(int M, int N, int K, int splits);
 // Reads and clears the tensor-core GEMM timeout flag (synchronises st).
 bool tc_gemm_timed_out(cudaStream_t st);
+// ttg_eval_batch of M multi-indices that are part of a call with M_all: cut as
+// for M_all, so that a split call's values do not depend on the split.
+int32_t eval_batch_part(const ttg_tensor* a, const int32_t* idx, int32_t M, int32_t M_all,
+                        double* out);
 // Sets the message returned by ttg_last_error() on this thread.
 void set_last_error(const std::string& msg);
 

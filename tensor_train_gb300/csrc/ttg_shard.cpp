@@ -266,7 +266,7 @@ int32_t ttg_eval_batch_devices(const ttg_tensor* a, const int32_t* idx, int32_t 
       errs[p] = std::string("eval_batch_devices: cudaSetDevice: ") + cudaGetErrorString(e);
       return;
     }
-    st[p] = ttg_eval_batch(a, idx + lo * d, static_cast<int32_t>(hi - lo), out + lo);
+    st[p] = ttg::eval_batch_part(a, idx + lo * d, static_cast<int32_t>(hi - lo), M, out + lo);
     if (st[p] != TTG_OK)
       errs[p] = ttg_last_error();
   };
