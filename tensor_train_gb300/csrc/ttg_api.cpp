@@ -518,13 +518,17 @@ int32_t setup_wide(ttg_plan& P)
   const size_t cm = sizeof(double) * static_cast<size_t>(core_max);
   const size_t oW = take(cm), oU = take(cm), oP = take(cm), oA = take(cm), oR = take(cc),
                oV = take(cc), oF = take(cc), oT1 = take(cc), oT2 = take(cc),
-               opart = take(8 * static_cast<size_t>(grid) + 8), oumax = take(8),
+               opart = take(16 * static_cast<size_t>(grid) + 16), oumax = take(8),
+               oTw = take(8 * kWidePb * kWidePb * static_cast<size_t>((c_max + kWidePb - 1) / kWidePb)),
                otau = take(8 * c_max), osig = take(8 * c_max),
                osorted = take(8 * c_max), oord = take(4 * c_max), ocn = take(8 * (cols_max + 1)),
                oival = take(64), orot = take(4 * ms), orel = take(4 * ms),
                oS1 = take(stream ? 8 * static_cast<size_t>(s_max) : 8),
                oS2 = take(stream ? 8 * static_cast<size_t>(s_max) : 8),
                oFs = take(stream ? 8 * static_cast<size_t>(f_max) : 8);
+  // The exchange packets come last, so that one strided fill zeroes every
+  // team's.
+  const size_t opk = take(sizeof(uint4) * static_cast<size_t>(wide_packets(c_max)));
   // One such block per team, then the teams' barrier words.
   const size_t team_bytes = o;
   const size_t obar = team_bytes * static_cast<size_t>(teams_max);
@@ -554,6 +558,9 @@ int32_t setup_wide(ttg_plan& P)
   j.T1 = reinterpret_cast<double*>(b + oT1);
   j.T2 = reinterpret_cast<double*>(b + oT2);
   j.part = reinterpret_cast<double*>(b + opart);
+  j.Tw = reinterpret_cast<double*>(b + oTw);
+  j.packets = reinterpret_cast<uint4*>(b + opk);
+  j.c_max = c_max;
   j.umax = reinterpret_cast<unsigned long long*>(b + oumax);
   j.mixed = P.opts.precision == TTG_PREC_MIXED ? 1 : 0;
   // Sliced-BF16 tensor-core contractions (mixed path only): measured slower
@@ -882,6 +889,9 @@ int32_t plan_run(ttg_plan& P, cudaStream_t st)
     if (P.wide)
     {
       TTG_CUDA(cudaMemsetAsync(P.wjob.bar, 0, sizeof(GridBar) * P.wide_teams, st));
+      TTG_CUDA(cudaMemset2DAsync(P.wjob.packets, static_cast<size_t>(P.wjob.team_bytes), 0,
+                                 sizeof(uint4) * static_cast<size_t>(wide_packets(P.wjob.c_max)),
+                                 static_cast<size_t>(P.wide_teams), st));
       WideJob j = P.wjob;
       j.teams = P.wide_teams;
       const int tsize = P.wide_grid / P.wide_teams;

@@ -8,6 +8,8 @@
 
 #include <cstdint>
 
+#include <vector_types.h>
+
 #if defined(__CUDACC__)
 #define TTG_HD __host__ __device__
 #else
@@ -132,6 +134,17 @@ struct GridBar
   int err;
 };
 
+// Blocked QR of the whole-GPU kernel (ttg_wide_qr.cuh): reflectors per block,
+// most row slabs of a panel and of a block's application, and the exchange
+// packets (16 bytes each) of one team for ranks up to c_max.
+constexpr int kWidePb = 16;
+constexpr int kWidePanelSlabs = 32;
+constexpr int kWideTrailSlabs = 16;
+inline int64_t wide_packets(int64_t c_max)
+{
+  return 2 * (kWidePanelSlabs + 1) * kWidePb + 2 * kWideTrailSlabs * c_max * kWidePb;
+}
+
 // Whole-GPU rounding of a few large TTs (wide_round_kernel): the arena,
 // slots and TT records as in RoundJob, plus grid-shared work buffers sized
 // for the largest core (core_max doubles) and rank (c_max).
@@ -176,7 +189,10 @@ struct WideJob
   int* ord;            // c_max
   double* cn;          // sum of ranks: balancing column norms
   int* ival;           // [0] = truncation rank of the current bond
-  double* part;        // one partial sum per CTA
+  double* part;        // two partial sums per CTA
+  double* Tw;          // kWidePb^2 per block of reflectors
+  uint4* packets;      // wide_packets(c_max): zeroed before each launch
+  int64_t c_max;
   unsigned long long* umax;  // grid-wide max of |x| bit patterns
   unsigned int* sweep_rot;  // max_sweeps
   unsigned int* sweep_rel;  // max_sweeps

@@ -4,19 +4,18 @@
 // and meet at a grid barrier between dependent phases.  Same algorithm and
 // branch structure as round_tt (detail::round, round/tt_round.hpp:36-134),
 // each step spread over the grid:
-//   * Householder QR (qr_thin, types/tt_eigen_bridge.hpp:42-60): column l
-//     belongs to CTA l mod P.  The owner of column j forms reflector j and
-//     publishes it; after one barrier every CTA applies it to its own
-//     columns.  Owned columns stay in shared memory when they fit.
-//   * Q and Q [Uc; 0]: each CTA forms its own columns from the published
-//     reflectors -- no barriers.
+//   * Householder QR (qr_thin, types/tt_eigen_bridge.hpp:42-60), Q and
+//     Q [Uc; 0] in blocks of 16 reflectors (ttg_wide_qr.cuh).  Matrices too
+//     tall for its shared-memory tiles go column by column: column l belongs
+//     to CTA l mod P, the owner of column j forms reflector j and publishes
+//     it, and after one barrier every CTA applies it to its own columns.
 //   * One-sided Jacobi SVD: block-pair rounds.  Columns are cut into blocks
 //     of b; in each round of the round-robin tournament over blocks a CTA
 //     loads a block pair into shared memory, runs one local sweep over all
 //     pairs of its 2b columns (cta_jacobi) and writes them back; a barrier
 //     ends the round.  Outer sweeps stop when a sweep rotates nothing or its
 //     largest relative rotation is below kJacobiStopRel.
-//   * Contractions: 64x64 FP64 output tiles spread over the CTAs.
+//   * Contractions: 32x32 or 16x16 FP64 output tiles spread over the CTAs.
 // QR, contractions and balancing are FP64.  The SVD is FP64 Jacobi on the
 // plain path; on the mixed path FP32 sweeps do the bulk of the rotating and
 // df64 sweeps (FP32 pipes) polish to FP64-level accuracy, as in the
@@ -32,11 +31,13 @@
 
 #include "ttg_device.cuh"
 #include "ttg_device_df.cuh"
+#include "ttg_gemm_grid.cuh"
 #include "ttg_gridbar.cuh"
 #include "ttg_job.h"
 #include "ttg_kernels.h"
 #include "ttg_ozaki.cuh"
 #include "ttg_sweep_common.cuh"
+#include "ttg_wide_qr.cuh"
 
 namespace ttg
 {
@@ -61,6 +62,8 @@ struct WideSmem
   double* p;
   int64_t cap;  // doubles
   OzState* oz;  // TMEM accumulator and MMA barrier of this CTA (null: FP64 tiles only)
+  uint32_t* seq;  // next exchange tag, the same on every thread of the team
+  bool* blocked;  // whether W holds the last QR in the blocked form
 };
 
 // dst[0..n) = src[0..n), spread over the grid.
@@ -73,7 +76,10 @@ __device__ void wide_copy(const WideJob& job, double* dst, const double* src, in
 
 // C = A B over the grid, tile t on CTA t mod P: 128x64 sliced-BF16 tiles
 // on the tensor cores (FP64-accurate, oz_tile) when the job allows them and
-// K <= 512, else 64x64 FP64 tiles.  Returns false if a tensor-core wait
+// K <= 512, else FP64 tiles of 32x32, or of 16x16 where the larger ones would
+// leave the fullest CTA with more work (the FP64 pipe bounds both).  64x64
+// tiles left 165 tiles of the d = 40, rank-257 sweep's products to 152 CTAs:
+// two rounds for the work of one.  Returns false if a tensor-core wait
 // timed out (the grid error word is set).
 // fp64_only: FP64 tiles even when the sliced tensor-core tiles are on
 // (products whose error bound is stated for FP64).
@@ -93,18 +99,35 @@ __device__ bool wide_gemm(const WideJob& job, int M, int N, int K, View A, View 
       atomicExch(&job.bar->err, 1);
     return ok;
   }
-  const int tm = (M + 63) / 64, tn = (N + 63) / 64;
-  for (int t = job.rank; t < tm * tn; t += job.size)
-    cta_gemm_tile((t / tn) * 64, (t % tn) * 64, M, N, K, A, B, C, c_rs, c_cs, sh, kTriNone);
+  auto rounds = [&](int T) {
+    const int64_t tiles = static_cast<int64_t>((M + T - 1) / T) * ((N + T - 1) / T);
+    return (tiles + job.size - 1) / job.size;
+  };
+  auto at = [&](const View& v) { return [v](int64_t i, int64_t j) { return v(i, j); }; };
+  auto put = [&](int i, int j, double v) { C[i * c_rs + j * c_cs] = v; };
+  const bool ak = A.rs != 1, bk = B.cs != 1;  // load along the contiguous direction
+  double* tile = sm.p;  // the dynamic shared memory is free between steps
+  if (rounds(32) * 4 <= rounds(16))
+  {
+    const int tm = (M + 31) / 32, tn = (N + 31) / 32;
+    for (int t = job.rank; t < tm * tn; t += job.size)
+      grid_tile<2>((t / tn) * 32, (t % tn) * 32, M, N, 0, K, at(A), at(B), put, tile, ak, bk);
+  }
+  else
+  {
+    const int tm = (M + 15) / 16, tn = (N + 15) / 16;
+    for (int t = job.rank; t < tm * tn; t += job.size)
+      grid_tile<1>((t / tn) * 16, (t % tn) * 16, M, N, 0, K, at(A), at(B), put, tile, ak, bk);
+  }
   __syncthreads();
   return true;
 }
 
-// Householder QR of X (h x c), column-distributed.  Reflector tails go to
+// Householder QR of X (h x c), column by column.  Reflector tails go to
 // job.W (column-major, ld h), scales to job.tau, R (k x c, column-major,
 // ld k) to job.R.  Returns k = min(h, c); false in *ok on a barrier failure.
-__device__ int wide_qr(const WideJob& job, View X, int h, int c, WideSmem sm, CtaShared& sh,
-                       bool* ok)
+__device__ __noinline__ int wide_qr_columns(const WideJob& job, View X, int h, int c, WideSmem sm,
+                                            CtaShared& sh, bool* ok)
 {
   const int P = job.size, me = job.rank;
   const int k = h < c ? h : c;
@@ -209,13 +232,75 @@ __device__ int wide_qr(const WideJob& job, View X, int h, int c, WideSmem sm, Ct
   return k;
 }
 
-// Column l (l mod P == this CTA) of H_0 ... H_{kref-1} [B(:, l); 0] into
-// out(i, l) = out[i*o_rs + l*o_cs], for l < ncols; B column-major (nb x
-// ncols, ld nb), nb <= h.  y is a length-h work column.
-__device__ void wide_apply_q(const WideJob& job, int h, int kref, const double* B, int nb,
+// Householder QR of X (h x c): reflectors in job.W, R (k x c, column-major,
+// ld k) in job.R.  Returns k = min(h, c); false in *ok on a barrier failure.
+__device__ int wide_qr(const WideJob& job, View X, int h, int c, WideSmem sm, CtaShared& sh,
+                       bool* ok)
+{
+  const int P = job.size, me = job.rank;
+  *sm.blocked = wide_blocked_fits(h, c, P, sm.cap);
+  if (!*sm.blocked)
+    return wide_qr_columns(job, X, h, c, sm, sh, ok);
+  const int k = h < c ? h : c;
+  const int64_t stride = static_cast<int64_t>(P) * blockDim.x;
+  const int64_t first = me * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  for (int64_t e = first; e < static_cast<int64_t>(h) * c; e += stride)
+    job.W[e] = X(e % h, e / h);
+  for (int64_t e = first; e < static_cast<int64_t>(k) * c; e += stride)
+    job.R[e] = 0.0;
+  *ok = grid_sync(job);
+  for (int j0 = 0; j0 < k && *ok; j0 += kPb)
+  {
+    const int nb = k - j0 < kPb ? k - j0 : kPb;
+    const int rows = panel_rows(h - j0, P);
+    const int S = (h - j0 + rows - 1) / rows;
+    uint32_t& seq = *sm.seq;
+    if (me < S)
+      *ok = wide_panel(job, h, k, j0, nb, S, rows, seq, sm.p);
+    // The panel columns' final entries above it, by the idle CTAs.
+    const int idle = P > S ? P - S : P, who = P > S ? me - S : me;
+    if (who >= 0)
+      for (int e = who * kThreads + threadIdx.x; e < j0 * nb; e += idle * kThreads)
+      {
+        const int i = e % j0;
+        const int64_t l = j0 + e / j0;
+        job.R[i + l * k] = job.W[l * h + i];
+      }
+    seq += kPb;
+    *ok = grid_sync(job) && *ok;
+    if (*ok && j0 + nb < c)
+    {
+      *ok = wide_trail(job, h, c, j0, nb, seq, sm.p, sm.cap);
+      *ok = grid_sync(job) && *ok;
+    }
+    seq += 1;
+  }
+  if (*ok && c > k)
+  {
+    for (int64_t e = first; e < static_cast<int64_t>(k) * (c - k); e += stride)
+    {
+      const int64_t i = e % k, l = k + e / k;
+      job.R[i + l * k] = job.W[l * h + i];
+    }
+    *ok = grid_sync(job);
+  }
+  return k;
+}
+
+// out(i, l) = out[i*o_rs + l*o_cs] = (H_0 ... H_{kref-1} [B; 0])(i, l) for
+// l < ncols; B column-major (nb x ncols, ld nb), nb <= h, or the identity
+// (eye).  Column by column when the QR was (column l on CTA l mod P; y is a
+// length-h work column).  Returns false on a failed wait.
+__device__ bool wide_apply_q(const WideJob& job, int h, int kref, const double* B, int nb,
                              int ncols, double* out, int64_t o_rs, int64_t o_cs, bool eye,
                              WideSmem sm, CtaShared& sh)
 {
+  if (*sm.blocked)
+  {
+    const uint32_t seq = *sm.seq;
+    *sm.seq += static_cast<uint32_t>((kref + kPb - 1) / kPb);
+    return wide_q(job, h, kref, B, nb, ncols, out, o_rs, o_cs, eye, seq, sm.p, sm.cap);
+  }
   const int P = job.size, me = job.rank;
   for (int l = me; l < ncols; l += P)
   {
@@ -245,6 +330,7 @@ __device__ void wide_apply_q(const WideJob& job, int h, int kref, const double* 
       out[i * o_rs + static_cast<int64_t>(l) * o_cs] = y[i];
     __syncthreads();
   }
+  return true;
 }
 
 // One-sided Jacobi of A (p x q, column-major, lda; element type E = float,
@@ -631,7 +717,8 @@ __device__ bool wide_right_orth(const WideJob& job, CoreSlot* S, int d, WideSmem
       return false;
     // core_k <- Q^T (Q column-major w x kk is the core's row-major layout);
     // prev (hp x kk) = left_unfold(prev) R^T.
-    wide_apply_q(job, w, kk, nullptr, 0, kk, cs, 1, w, true, sm, sh);
+    if (!wide_apply_q(job, w, kk, nullptr, 0, kk, cs, 1, w, true, sm, sh))
+      return false;
     if (!wide_gemm(job, hp, kk, r, View{ps, r, 1}, View{job.R, kk, 1}, job.Pb, kk, 1, sm, sh))
       return false;
     WSYNC();
@@ -643,6 +730,93 @@ __device__ bool wide_right_orth(const WideJob& job, CoreSlot* S, int d, WideSmem
     }
     WSYNC();
   }
+  return true;
+}
+
+// No-truncation certificate of the bond matrix X (h x c) from its QR's R in
+// job.R.  First by the inverse: the columns z_j of R^-1 are independent back
+// substitutions, a warp each, with no barrier among them (27 us for c = 257,
+// where one CTA's elimination of the Gram matrix is bound by that SM's FP64
+// rate: 0.7 ms).  The computed Z has R Z = I - E, |E| <= gamma_c |R| |Z|
+// (Higham, thm. 8.5), so
+//   sigma_min(R) >= (1 - g) / ||Z||_F,   g = gamma ||R||_F ||Z||_F.
+// Where that bound clears the elimination's own test with the elimination's
+// error to spare (tau of certify_tau, its error term twice), the elimination
+// would have met only positive pivots: the bond is certified.  Otherwise the
+// elimination decides, as it does alone in the per-TT sweep.
+__device__ bool wide_certify(const WideJob& job, int c, int h, double delta, WideSmem sm,
+                             CtaShared& sh, bool* certified)
+{
+  const int P = job.size, me = job.rank;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  constexpr double u = CertOps<double>::u;
+  double zz = 0.0, rr = 0.0;
+  bool tried = static_cast<int64_t>(kWarps + 1) * c <= sm.cap;
+  if (tried)
+  {
+    double* dinv = sm.p;
+    double* x = sm.p + static_cast<int64_t>(w + 1) * c;
+    for (int i = threadIdx.x; i < c; i += blockDim.x)
+      dinv[i] = 1.0 / job.R[i + static_cast<int64_t>(i) * c];
+    __syncthreads();
+    for (int j = me + P * w; j < c; j += P * kWarps)
+    {
+      for (int i = lane; i <= j; i += 32)
+      {
+        const double r = job.R[i + static_cast<int64_t>(j) * c];
+        rr = fma(r, r, rr);
+        x[i] = i == j ? 1.0 : 0.0;
+      }
+      __syncwarp();
+      for (int i = j; i >= 0; --i)
+      {
+        const double z = x[i] * dinv[i];
+        const double* col = job.R + static_cast<int64_t>(i) * c;
+        for (int q = lane; q < i; q += 32)
+          x[q] = fma(-z, col[q], x[q]);
+        if (lane == 0)
+          zz = fma(z, z, zz);
+        __syncwarp();
+      }
+    }
+  }
+  zz = cta_sum(zz, sh);
+  rr = cta_sum(rr, sh);
+  if (threadIdx.x == 0)
+  {
+    job.part[2 * me] = zz;
+    job.part[2 * me + 1] = rr;
+  }
+  WSYNC();
+  zz = rr = 0.0;
+  for (int i = threadIdx.x; i < P; i += blockDim.x)
+  {
+    zz += __ldcg(job.part + 2 * i);
+    rr += __ldcg(job.part + 2 * i + 1);
+  }
+  zz = sqrt(cta_sum(zz, sh));
+  rr = sqrt(cta_sum(rr, sh));
+  const double g = 1.1 * (c + 4) * u * rr * zz;
+  const double low = (1.0 - g) / zz;
+  const double eR = static_cast<double>(c) * h * u * rr;
+  const double tau = (1.0 + 4.0 * u) * (delta + eR) * (delta + eR) + 8.0 * (c + 1.0) * u * rr * rr;
+  // A NaN or an overflow anywhere fails one of the comparisons.
+  *certified = tried && g < 0.5 && low * low > tau;
+  if (*certified)
+    return true;
+  // G = R^T R (FP64) over the grid into job.A, then one CTA eliminates it
+  // and the decision reaches every CTA through job.ival[1].
+  if (!wide_gemm(job, c, c, c, View{job.R, c, 1}, View{job.R, 1, c}, job.A, 1, c, sm, sh, true))
+    return false;
+  WSYNC();
+  if (me == 0)
+  {
+    const bool yes = cta_certify_from_gram(job.A, job.R, c, h, delta, sh, u);
+    if (threadIdx.x == 0)
+      job.ival[1] = yes ? 1 : 0;
+  }
+  WSYNC();
+  *certified = *reinterpret_cast<volatile const int*>(job.ival + 1) != 0;
   return true;
 }
 
@@ -672,37 +846,19 @@ __device__ bool wide_left_svd(const WideJob& job, View X, int h, int c, double d
     bool certified = false;
     if (certify)
     {
-      // G = R^T R (FP64) over the grid into job.A, then one CTA eliminates
-      // it (FP64) and proves sigma_min(R) > delta; the decision reaches every
-      // CTA through job.ival[1].  The QR here is FP64 on both paths.
-      if (!wide_gemm(job, c, c, c, View{job.R, c, 1}, View{job.R, 1, c}, job.A, 1, c, sm, sh,
-                     true))
+      if (!wide_certify(job, c, h, delta, sm, sh, &certified))
         return false;
-      WSYNC();
-      if (me == 0)
-      {
-        const bool yes =
-          cta_certify_from_gram(job.A, job.R, c, h, delta, sh, CertOps<double>::u);
-        if (threadIdx.x == 0)
-          job.ival[1] = yes ? 1 : 0;
-      }
-      WSYNC();
-      certified = *reinterpret_cast<volatile const int*>(job.ival + 1) != 0;
     }
     if (certified)
     {
-      // Every singular value is kept: U = Q (Uc = I in V), F = R.
+      // Every singular value is kept: U = Q, F = R.
       r_new = c;
       const int64_t cc = static_cast<int64_t>(c) * c;
       for (int64_t e = job.rank * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < cc;
            e += static_cast<int64_t>(job.size) * blockDim.x)
-      {
-        const int64_t i = e % c, j = e / c;
-        job.V[e] = i == j ? 1.0 : 0.0;
-        job.F[i * c + j] = job.R[e];
-      }
-      WSYNC();
-      wide_apply_q(job, h, c, job.V, c, r_new, job.Ub, 1, h, false, sm, sh);
+        job.F[(e % c) * c + e / c] = job.R[e];
+      if (!wide_apply_q(job, h, c, nullptr, 0, c, job.Ub, 1, h, true, sm, sh))
+        return false;
       WSYNC();
     }
     else
@@ -734,7 +890,8 @@ __device__ bool wide_left_svd(const WideJob& job, View X, int h, int c, double d
       if (!wide_gemm(job, r_new, c, c, View{job.V, c, 1}, View{job.R, 1, c}, job.F, c, 1, sm,
                      sh))
         return false;
-      wide_apply_q(job, h, c, job.V, c, r_new, job.Ub, 1, h, false, sm, sh);
+      if (!wide_apply_q(job, h, c, job.V, c, r_new, job.Ub, 1, h, false, sm, sh))
+        return false;
       WSYNC();
     }
   }
@@ -922,7 +1079,8 @@ __device__ bool wide_round_right_tt(const WideJob& job, int tti, WideSmem sm, Ct
       return false;
     // core_k <- Q (h x kk, row-major); next (kk x wn) = R right_unfold(next),
     // R (kk x rp) column-major in job.R.
-    wide_apply_q(job, h, kk, nullptr, 0, kk, cs, kk, 1, true, sm, sh);
+    if (!wide_apply_q(job, h, kk, nullptr, 0, kk, cs, kk, 1, true, sm, sh))
+      return false;
     if (!wide_gemm(job, kk, wn, rp, View{job.R, 1, kk}, View{ns, wn, 1}, job.Pb, wn, 1, sm, sh))
       return false;
     WSYNC();
@@ -1086,7 +1244,7 @@ __device__ bool wide_stream_tt(const WideJob& job, int item, WideSmem sm, CtaSha
   return true;
 }
 
-__global__ void __launch_bounds__(kThreads) wide_round_kernel(WideJob job)
+__global__ void __launch_bounds__(kThreads, 1) wide_round_kernel(WideJob job)
 {
   extern __shared__ double dyn_smem[];
   __shared__ CtaShared sh;
@@ -1105,7 +1263,9 @@ __global__ void __launch_bounds__(kThreads) wide_round_kernel(WideJob job)
     tc::fence_after_sync();
     oz.tmem = tmem_base;
   }
-  const WideSmem sm{dyn_smem, job.smem_doubles, job.tc ? &oz : nullptr};
+  uint32_t seq = 1;
+  bool blocked = false;
+  const WideSmem sm{dyn_smem, job.smem_doubles, job.tc ? &oz : nullptr, &seq, &blocked};
   // Teams: the grid splits into `teams` groups of equal size; group g owns
   // its own work buffers (one block of team_bytes each) and barrier word, and
   // rounds items g, g + teams, ... (the order is longest first).
@@ -1137,6 +1297,8 @@ __global__ void __launch_bounds__(kThreads) wide_round_kernel(WideJob job)
     tj.cn = sh_ptr(job.cn);
     tj.ival = sh_ptr(job.ival);
     tj.part = sh_ptr(job.part);
+    tj.Tw = sh_ptr(job.Tw);
+    tj.packets = sh_ptr(job.packets);
     tj.umax = sh_ptr(job.umax);
     tj.sweep_rot = sh_ptr(job.sweep_rot);
     tj.sweep_rel = sh_ptr(job.sweep_rel);

@@ -1,0 +1,590 @@
+// Blocked Householder QR and its Q over the CTAs of a team, FP64.
+//
+// The unblocked form met at a grid barrier per column (~10 us each: barrier,
+// norm, update of the CTA's columns one CTA-wide reduction at a time), and Q
+// cost a chain of as many CTA-wide reductions: 8.2 ms per step of the d = 40,
+// rank-257 sweep against a floor of 0.7 ms at the chip's FP64 rate.  Here
+// kPb columns are factored by a few CTAs and applied as one block
+// I - V T V^T (compact WY; LAPACK dlarft, Schreiber & Van Loan 1989):
+//
+//   * wide_panel: the panel's rows are cut into slabs of >= 64, one per CTA,
+//     in shared memory.  Per column one exchange: each CTA publishes its
+//     share of the products of the column with all kPb panel columns (its
+//     norm, the next columns' dots and the entries of V^T V for T at once),
+//     and every CTA adds the slabs' shares in the same order.
+//   * wide_trail / wide_form_q: the trailing matrix (or Q) is cut into slabs
+//     of rows times groups of columns, one CTA each, so that every SM's FP64
+//     pipe has the same share; W = V^T B is exchanged between the slabs of a
+//     column group only.  Q's tiles stay in shared memory over all blocks.
+//
+// An exchange is one 16-byte packet per value, {low word, tag, high word,
+// tag}: each 8-byte half says by its tag that it has arrived (8-byte accesses
+// are single), so a reader needs no fence and no flag, only a poll of the
+// packet itself.  Tags never repeat within a launch, and the packets are
+// zeroed before it.  Packet buffers alternate by the tag's parity: a CTA two
+// exchanges ahead has all packets of the one between, whose senders have read
+// the first.  Every poll is bounded like the grid barrier's.
+//
+// Reflector convention as cta_householder_qr (Eigen's makeHouseholder).
+#pragma once
+
+#include <cfloat>
+#include <cstdint>
+#include <cuda_runtime.h>
+
+#include "ttg_device.cuh"
+#include "ttg_job.h"
+
+namespace ttg
+{
+namespace
+{
+
+constexpr int kPb = kWidePb;
+
+// -- packets ------------------------------------------------------------------
+__device__ __forceinline__ void packet_put(uint4* p, double v, uint32_t tag)
+{
+  const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(v));
+  asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(p),
+               "r"(static_cast<uint32_t>(u)), "r"(tag), "r"(static_cast<uint32_t>(u >> 32))
+               : "memory");
+}
+
+// Waits for a packet; 0.0 and *fail = true when the wait gave up.
+__device__ __forceinline__ double packet_get(const WideJob& job, const uint4* p, uint32_t tag,
+                                             bool* fail)
+{
+  uint32_t lo, t0, hi, t1;
+  int polls = 0;
+  long long start = 0;
+  for (;;)
+  {
+    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(lo), "=r"(t0), "=r"(hi), "=r"(t1)
+                 : "l"(p)
+                 : "memory");
+    if (t0 == tag && t1 == tag)
+      return __longlong_as_double(
+        static_cast<long long>((static_cast<unsigned long long>(hi) << 32) | lo));
+    if ((++polls & 255) == 0)
+    {
+      if (start == 0)
+        start = clock64();
+      const bool late = clock64() - start > job.wait_cycles;
+      if (late)
+        atomicExch(&job.bar->err, 1);
+      if (late || *reinterpret_cast<volatile int*>(&job.bar->err))
+      {
+        *fail = true;
+        return 0.0;
+      }
+    }
+  }
+}
+
+// Slots: panel products (slab, column), the panel row's own entries, and the
+// trailing products (slab, column, reflector).
+__device__ __forceinline__ uint4* panel_slot(const WideJob& job, uint32_t tag, int slab, int l)
+{
+  return job.packets + ((tag & 1u) * (kWidePanelSlabs + 1) + slab) * kPb + l;
+}
+__device__ __forceinline__ uint4* trail_slot(const WideJob& job, uint32_t tag, int slab, int col, int i)
+{
+  return job.packets + 2 * (kWidePanelSlabs + 1) * kPb +
+         ((static_cast<int64_t>(tag & 1u) * kWideTrailSlabs + slab) * job.c_max + col) * kPb + i;
+}
+
+// -- panel --------------------------------------------------------------------
+struct PanelShared
+{
+  double d[kPb];       // the column's products with the panel's columns
+  double row[kPb];     // the panel columns' entries in the column's row
+  double w[kPb];       // what the row loses per column
+  double G[kPb * kPb]; // V^T V above the diagonal
+  double T[kPb * kPb]; // column-major, upper triangular
+  double inv[kPb], tau[kPb];
+};
+
+// Column i of T = -tau_i T(0:i, 0:i) G(0:i, i), T(i, i) = tau_i, by the 32
+// lanes of a warp.
+__device__ __forceinline__ void panel_t_column(PanelShared& ps, int i)
+{
+  const int l = threadIdx.x & 31;
+  const double nt = -ps.tau[i];
+  double acc = 0.0;
+  if (l < i)
+    for (int q = l; q < i; ++q)
+      acc = fma(ps.T[l + q * kPb], nt * ps.G[q + i * kPb], acc);
+  __syncwarp();
+  if (l < kPb)
+    ps.T[l + i * kPb] = l < i ? acc : (l == i ? -nt : 0.0);
+  __syncwarp();
+}
+
+// Factors columns j0 .. j0 + nb of W (h rows) on the first S CTAs of the
+// team, `rows` rows from j0 on each.  On return W holds the explicit V (from
+// row j0 on), R its entries, job.Tw the block's T.  Tags seq .. seq + nb.
+__device__ __noinline__ bool wide_panel(const WideJob& job, int h, int k, int j0, int nb, int S,
+                                        int rows, uint32_t seq, double* sm)
+{
+  const int me = job.rank, t = threadIdx.x;
+  const int r0 = j0 + me * rows;  // this slab's first row
+  const int nr = h - r0 < rows ? h - r0 : rows;
+  const int ld = rows | 1;
+  PanelShared& ps = *reinterpret_cast<PanelShared*>(sm);
+  double* P = sm + sizeof(PanelShared) / sizeof(double);
+  const int lane = t & 31, w = t >> 5;
+  for (int i = w; i < nb; i += kWarps)
+    for (int r = lane; r < nr; r += 32)
+      P[i * ld + r] = job.W[static_cast<int64_t>(j0 + i) * h + r0 + r];
+  __syncthreads();
+  bool fail = false;
+  for (int i = 0; i < nb; ++i)
+  {
+    const uint32_t tag = seq + i;
+    const int j = j0 + i;           // the column, and its diagonal row
+    const int lo = j + 1 > r0 ? j + 1 - r0 : 0;  // first slab row below the diagonal
+    const bool owner = j >= r0 && j < r0 + nr;
+    const double* x = P + i * ld;
+    // Products of x below row j: 8 lanes per panel column on four warps (one
+    // per FP64 pipe: more lanes per column only add reduction steps).
+    if (t < 8 * kPb)
+    {
+      const int l = t >> 3, g = t & 7;
+      double a0 = 0.0, a1 = 0.0;
+      if (l < nb)
+      {
+        const double* y = P + l * ld;
+        int r = lo + g;
+        for (; r + 8 < nr; r += 16)
+        {
+          a0 = fma(x[r], y[r], a0);
+          a1 = fma(x[r + 8], y[r + 8], a1);
+        }
+        if (r < nr)
+          a0 = fma(x[r], y[r], a0);
+      }
+      a0 += a1;
+      a0 += __shfl_xor_sync(0xffffffffu, a0, 4);
+      a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
+      a0 += __shfl_xor_sync(0xffffffffu, a0, 1);
+      if (g == 0 && l < nb)
+      {
+        if (S > 1)
+          packet_put(panel_slot(job, tag, me, l), a0, tag);
+        else
+          ps.d[l] = a0;
+      }
+    }
+    else if (owner && t < 8 * kPb + nb)
+    {
+      const int l = t - 8 * kPb;
+      if (S > 1)
+        packet_put(panel_slot(job, tag, kWidePanelSlabs, l), P[l * ld + j - r0], tag);
+      else
+        ps.row[l] = P[l * ld + j - r0];
+    }
+    // T's previous column while the packets travel (the first CTA's T is used).
+    if (me == 0 && w == 6 && i > 0)
+      panel_t_column(ps, i - 1);
+    if (S > 1 && t < 8 * kPb)
+    {
+      const int l = t >> 3, g = t & 7;
+      double v = 0.0;
+      if (l < nb)
+        for (int s = g; s < S; s += 8)
+          v += packet_get(job, panel_slot(job, tag, s, l), tag, &fail);
+      __syncwarp();
+      v += __shfl_xor_sync(0xffffffffu, v, 4);
+      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      if (g == 0)
+        ps.d[l] = v;
+    }
+    else if (S > 1 && t < 8 * kPb + nb)
+      ps.row[t - 8 * kPb] = packet_get(job, panel_slot(job, tag, kWidePanelSlabs, t - 8 * kPb), tag,
+                                       &fail);
+    if (__syncthreads_or(fail))
+      return false;
+    // The reflector, and what it takes from each later column.
+    if (w == 0)
+    {
+      const double tail2 = ps.d[i], x0 = ps.row[i];
+      double beta = x0, tau = 0.0, inv = 0.0;
+      if (!(tail2 <= DBL_MIN))
+      {
+        const double s = fma(x0, x0, tail2);
+        const double rs = rsqrt(s);
+        double n = s * rs;  // |x|, one Newton step from the reciprocal root
+        n = fma(fma(-n, n, s), 0.5 * rs, n);
+        const double ax = fabs(x0);
+        inv = 1.0 / (ax + n);
+        inv = x0 >= 0.0 ? inv : -inv;
+        beta = x0 >= 0.0 ? -n : n;
+        tau = (n + ax) / n;
+      }
+      if (lane < nb)
+      {
+        if (lane > i)
+        {
+          const double dot = tau * fma(inv, ps.d[lane], ps.row[lane]);
+          ps.w[lane] = dot * inv;
+          if (owner)
+            P[lane * ld + j - r0] = ps.row[lane] - dot;
+        }
+        else if (lane < i)  // v_l . v_i, v_l = inv_l x_l
+          ps.G[lane + i * kPb] = ps.inv[lane] * fma(inv, ps.d[lane], ps.row[lane]);
+      }
+      __syncwarp();
+      if (lane == 0)
+      {
+        ps.inv[i] = inv;
+        ps.tau[i] = tau;
+        if (owner)
+          P[i * ld + j - r0] = beta;
+      }
+    }
+    __syncthreads();
+    for (int l = i + 1 + w; l < nb; l += kWarps)
+    {
+      const double f = -ps.w[l];
+      double* y = P + l * ld;
+      for (int r = lo + lane; r < nr; r += 32)
+        y[r] = fma(f, x[r], y[r]);
+    }
+    __syncthreads();
+  }
+  if (me == 0 && w == 6)
+    panel_t_column(ps, nb - 1);
+  // R's entries and the explicit V.
+  for (int i = w; i < nb; i += kWarps)
+  {
+    const int j = j0 + i;
+    const double inv = ps.inv[i];
+    for (int r = lane; r < nr; r += 32)
+    {
+      const int gr = r0 + r;
+      const double x = P[i * ld + r];
+      if (gr <= j)
+        job.R[gr + static_cast<int64_t>(j) * k] = x;
+      job.W[static_cast<int64_t>(j) * h + gr] = gr < j ? 0.0 : (gr == j ? 1.0 : inv * x);
+    }
+  }
+  __syncthreads();
+  if (me == 0)
+    for (int e = t; e < kPb * kPb; e += kThreads)
+      job.Tw[static_cast<int64_t>(j0 / kPb) * kPb * kPb + e] =
+        (e / kPb < nb && e % kPb < nb) ? ps.T[e] : 0.0;
+  __syncthreads();
+  return true;
+}
+
+// -- block application ---------------------------------------------------------
+// How a matrix of `hp` rows and m columns is cut for a block's application:
+// St slabs of `rows` rows times Gt groups of at most nc columns.  The cost is
+// the FP64 clocks of the fullest CTA: 2 kPb FMAs per element at 2 per clock,
+// the slabs' sums, and an exchange's latency.
+struct TrailCut
+{
+  int St, Gt, rows, nc;
+};
+
+// Lane s - 1 of every warp weighs s slabs; all lanes of the CTA get the cut.
+__device__ TrailCut trail_cut(int hp, int m, int P, int64_t cap)
+{
+  const int s = (threadIdx.x & 31) + 1;
+  const int most = P < kWideTrailSlabs ? P : kWideTrailSlabs;
+  auto cut_of = [&](int slabs) {
+    TrailCut k;
+    k.rows = (hp + slabs - 1) / slabs;
+    k.St = (hp + k.rows - 1) / k.rows;
+    k.Gt = P / k.St < m ? P / k.St : m;
+    k.nc = (m + k.Gt - 1) / k.Gt;
+    return k;
+  };
+  unsigned long long best = ~0ull;
+  if (s <= most)
+  {
+    const TrailCut k = cut_of(s);
+    const int64_t need =
+      static_cast<int64_t>(kPb + k.nc) * (k.rows | 1) + 2 * kPb * k.nc + kPb * kPb;
+    if (need <= cap)
+      best = (static_cast<unsigned long long>(kPb) * k.nc * k.rows + 8ull * k.nc * k.St +
+              (k.St > 1 ? 2500 : 0))
+               << 5 |
+             static_cast<unsigned>(s - 1);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+  {
+    const unsigned long long x = __shfl_xor_sync(0xffffffffu, best, o);
+    best = x < best ? x : best;
+  }
+  if (best == ~0ull)
+    return TrailCut{0, 0, 0, 0};
+  return cut_of(static_cast<int>(best & 31) + 1);
+}
+
+// Sums of 16 values over the G lanes of a group by halving: lane gl ends with
+// value(s) i0 .. i0 + max(16 / G, 1) in acc[0..].
+template <int G>
+__device__ __forceinline__ void halving_sum(double (&acc)[kPb], int gl)
+{
+  int o = G / 2;
+#pragma unroll
+  for (int n = kPb / 2; n >= 1; n >>= 1)
+  {
+    if (o == 0)
+      break;
+    const bool up = (gl & o) != 0;
+#pragma unroll
+    for (int i = 0; i < kPb / 2; ++i)
+      if (i < n)
+      {
+        const double keep = up ? acc[i + n] : acc[i];
+        const double send = up ? acc[i] : acc[i + n];
+        acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    o >>= 1;
+  }
+  if (G == 32)
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+}
+
+// The tile B (nr x nc in shared memory, column-major, ldb) <- its rows of
+// (I - V T' V^T) B, T' = T^T (kTrans) or T: V's rows of this slab in Vs
+// (kPb columns, ldv), B's other slabs on the other CTAs of the group, whose
+// shares of V^T B are exchanged under `tag` (St > 1).  col(q): the column's
+// index in the exchange.  Ws, Zs: kPb nc doubles each.
+template <int G, bool kTrans, class FCol>
+__device__ __forceinline__ bool block_apply_g(const WideJob& job, const double* Vs, int ldv, double* Bs,
+                                              int ldb, int nr, int nc, const double* Ts, double* Ws,
+                                              double* Zs, int St, int slab, uint32_t tag, FCol col)
+{
+  const int t = threadIdx.x, gl = t & (G - 1), q0 = t / G;
+  constexpr int kCols = kThreads / G;
+  const int i0 = G == 32 ? gl >> 1 : gl * (kPb / G > 0 ? kPb / G : 1);
+  for (int qb = 0; qb < nc; qb += kCols)
+  {
+    const int q = qb + q0;
+    double acc[kPb];
+#pragma unroll
+    for (int i = 0; i < kPb; ++i)
+      acc[i] = 0.0;
+    if (q < nc)
+    {
+      const double* y = Bs + q * ldb;
+      for (int r = gl; r < nr; r += G)
+      {
+        const double b = y[r];
+#pragma unroll
+        for (int i = 0; i < kPb; ++i)
+          acc[i] = fma(Vs[i * ldv + r], b, acc[i]);
+      }
+    }
+    halving_sum<G>(acc, gl);
+    if (q < nc)
+    {
+      constexpr int kEach = kPb / G > 0 ? kPb / G : 1;
+#pragma unroll
+      for (int e = 0; e < kEach; ++e)
+        if (G < 32 || (gl & 1) == 0)
+        {
+          if (St > 1)
+            packet_put(trail_slot(job, tag, slab, col(q), i0 + e), acc[e], tag);
+          else
+            Ws[q * kPb + i0 + e] = acc[e];
+        }
+    }
+  }
+  bool fail = false;
+  if (St > 1)
+    for (int e = t; e < nc * kPb; e += kThreads)
+    {
+      const int c = col(e / kPb);
+      double v = 0.0;
+      for (int s = 0; s < St; ++s)
+        v += packet_get(job, trail_slot(job, tag, s, c, e % kPb), tag, &fail);
+      Ws[e] = v;
+    }
+  if (__syncthreads_or(fail))
+    return false;
+  for (int e = t; e < nc * kPb; e += kThreads)
+  {
+    const int i = e % kPb;
+    const double* wq = Ws + (e - i);
+    double z = 0.0;
+#pragma unroll
+    for (int l = 0; l < kPb; ++l)
+      z = fma(kTrans ? Ts[l + i * kPb] : Ts[i + l * kPb], wq[l], z);
+    Zs[e] = z;
+  }
+  __syncthreads();
+  for (int qb = 0; qb < nc; qb += kCols)
+  {
+    const int q = qb + q0;
+    if (q >= nc)
+      break;
+    double z[kPb];
+#pragma unroll
+    for (int i = 0; i < kPb; ++i)
+      z[i] = -Zs[q * kPb + i];
+    double* y = Bs + q * ldb;
+    for (int r = gl; r < nr; r += G)
+    {
+      double b = y[r];
+#pragma unroll
+      for (int i = 0; i < kPb; ++i)
+        b = fma(z[i], Vs[i * ldv + r], b);
+      y[r] = b;
+    }
+  }
+  __syncthreads();
+  return true;
+}
+
+template <bool kTrans, class FCol>
+__device__ bool block_apply(const WideJob& job, const double* Vs, int ldv, double* Bs, int ldb, int nr,
+                            int nc, const double* Ts, double* Ws, double* Zs, int St, int slab,
+                            uint32_t tag, FCol col)
+{
+  // Lanes per column: as few as keep all 256 threads at work.
+  if (nc > 16)
+    return block_apply_g<8, kTrans>(job, Vs, ldv, Bs, ldb, nr, nc, Ts, Ws, Zs, St, slab, tag, col);
+  if (nc > 8)
+    return block_apply_g<16, kTrans>(job, Vs, ldv, Bs, ldb, nr, nc, Ts, Ws, Zs, St, slab, tag, col);
+  return block_apply_g<32, kTrans>(job, Vs, ldv, Bs, ldb, nr, nc, Ts, Ws, Zs, St, slab, tag, col);
+}
+
+// V's rows [r0, r0 + nr) of the block at j0 (zero above row j0 and past nb),
+// and the block's T, into shared memory.
+__device__ __forceinline__ void load_block(const WideJob& job, int h, int j0, int nb, int r0, int nr,
+                                           double* Vs, int ldv, double* Ts)
+{
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int i = w; i < kPb; i += kWarps)
+    for (int r = lane; r < nr; r += 32)
+      Vs[i * ldv + r] = (i < nb && r0 + r >= j0) ? job.W[static_cast<int64_t>(j0 + i) * h + r0 + r] : 0.0;
+  for (int e = threadIdx.x; e < kPb * kPb; e += kThreads)
+    Ts[e] = job.Tw[static_cast<int64_t>(j0 / kPb) * kPb * kPb + e];
+}
+
+// W's columns from j0 + nb on <- (I - V T^T V^T) W, V the block at j0.
+__device__ __noinline__ bool wide_trail(const WideJob& job, int h, int c, int j0, int nb, uint32_t tag,
+                                        double* sm, int64_t cap)
+{
+  const int c0 = j0 + nb, m = c - c0, hp = h - j0;
+  const TrailCut cut = trail_cut(hp, m, job.size, cap);
+  const int slab = job.rank % cut.St, g = job.rank / cut.St;
+  if (g >= cut.Gt)
+    return true;
+  const int r0 = j0 + slab * cut.rows;
+  const int nr = h - r0 < cut.rows ? h - r0 : cut.rows;
+  const int q0 = g * cut.nc;
+  const int nc = m - q0 < cut.nc ? m - q0 : cut.nc;
+  if (nc <= 0)
+    return true;
+  const int ld = cut.rows | 1;
+  double* Vs = sm;
+  double* Bs = Vs + kPb * ld;
+  double* Ws = Bs + cut.nc * ld;
+  double* Zs = Ws + kPb * cut.nc;
+  double* Ts = Zs + kPb * cut.nc;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  load_block(job, h, j0, nb, r0, nr, Vs, ld, Ts);
+  double* B = job.W + static_cast<int64_t>(c0 + q0) * h + r0;
+  for (int q = w; q < nc; q += kWarps)
+    for (int r = lane; r < nr; r += 32)
+      Bs[q * ld + r] = B[static_cast<int64_t>(q) * h + r];
+  __syncthreads();
+  if (!block_apply<true>(job, Vs, ld, Bs, ld, nr, nc, Ts, Ws, Zs, cut.St, slab, tag,
+                         [&](int q) { return q0 + q; }))
+    return false;
+  for (int q = w; q < nc; q += kWarps)
+    for (int r = lane; r < nr; r += 32)
+      B[static_cast<int64_t>(q) * h + r] = Bs[q * ld + r];
+  __syncthreads();
+  return true;
+}
+
+// out(i, l) = (H_0 ... H_{kref-1} [B; 0])(i, l), l < ncols, from the blocks in
+// W; B column-major (nb_rows x ncols) or, with eye, the identity.  No grid
+// barrier inside; the tags used are seq .. seq + number of blocks.
+__device__ __noinline__ bool wide_q(const WideJob& job, int h, int kref, const double* B, int nb_rows,
+                                    int ncols, double* out, int64_t o_rs, int64_t o_cs, bool eye,
+                                    uint32_t seq, double* sm, int64_t cap)
+{
+  const TrailCut cut = trail_cut(h, ncols, job.size, cap);
+  const int slab = job.rank % cut.St, g = job.rank / cut.St;
+  if (g >= cut.Gt)
+    return true;
+  const int r0 = slab * cut.rows;
+  const int nr = h - r0 < cut.rows ? h - r0 : cut.rows;
+  // Columns g, g + Gt, ...: with the identity start a block touches columns
+  // from its own first on, so every group gets some of each.
+  const int nc = (ncols - g + cut.Gt - 1) / cut.Gt;
+  const int ld = cut.rows | 1;
+  double* Vs = sm;
+  double* Bs = Vs + kPb * ld;
+  double* Ws = Bs + cut.nc * ld;
+  double* Zs = Ws + kPb * cut.nc;
+  double* Ts = Zs + kPb * cut.nc;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int q = w; q < nc; q += kWarps)
+  {
+    const int l = g + cut.Gt * q;
+    for (int r = lane; r < nr; r += 32)
+    {
+      const int gr = r0 + r;
+      Bs[q * ld + r] = eye ? (gr == l ? 1.0 : 0.0)
+                           : (gr < nb_rows ? B[gr + static_cast<int64_t>(l) * nb_rows] : 0.0);
+    }
+  }
+  const int blocks = (kref + kPb - 1) / kPb;
+  for (int b = blocks - 1; b >= 0; --b)
+  {
+    const int j0 = b * kPb;
+    const int nb = kref - j0 < kPb ? kref - j0 : kPb;
+    int qa = 0;  // first column that the block touches
+    if (eye && j0 > g)
+      qa = (j0 - g + cut.Gt - 1) / cut.Gt;
+    if (qa >= nc)
+      continue;
+    load_block(job, h, j0, nb, r0, nr, Vs, ld, Ts);
+    __syncthreads();
+    if (!block_apply<false>(job, Vs, ld, Bs + qa * ld, ld, nr, nc - qa, Ts, Ws, Zs, cut.St, slab,
+                            seq + static_cast<uint32_t>(blocks - 1 - b),
+                            [&](int q) { return g + cut.Gt * (qa + q); }))
+      return false;
+  }
+  __syncthreads();
+  for (int q = w; q < nc; q += kWarps)
+  {
+    const int64_t l = g + cut.Gt * q;
+    for (int r = lane; r < nr; r += 32)
+      out[(r0 + r) * o_rs + l * o_cs] = Bs[q * ld + r];
+  }
+  __syncthreads();
+  return true;
+}
+
+// Rows per panel slab and slabs for hp rows.
+__device__ __forceinline__ int panel_rows(int hp, int P)
+{
+  const int most = P < kWidePanelSlabs ? P : kWidePanelSlabs;
+  const int rows = (hp + most - 1) / most;
+  return rows < 64 ? 64 : rows;
+}
+
+// Whether the blocked routines' tiles fit: the panel's slab, and some cut of
+// the trailing matrix and of Q.
+__device__ bool wide_blocked_fits(int h, int c, int P, int64_t cap)
+{
+  const int64_t panel = static_cast<int64_t>(kPb) * (panel_rows(h, P) | 1) +
+                        static_cast<int64_t>(sizeof(PanelShared) / sizeof(double));
+  return panel <= cap && trail_cut(h, c, P, cap).St > 0;
+}
+
+}  // namespace
+}  // namespace ttg
