@@ -1,0 +1,75 @@
+// FP64 pieces shared by the blocked Householder routines (ttg_wide_qr.cuh,
+// ttg_wy.cuh): the scalars of a reflector and the reduction of a block's 16
+// products.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace ttg
+{
+namespace
+{
+
+// The scalars of a reflector from s = x0^2 + |tail|^2 and ax = |x0|:
+// n = |x|, rs = 1 / n, inv = 1 / (ax + n).  One third-order step
+// (Householder's iteration: the error of the start cubed) from the hardware's
+// approximations of the reciprocal root and the reciprocal, which hold at
+// least 20 bits: 2^-60 before the last rounding.  What counts is the number
+// of FP64 instructions (64 clocks each) that every other thread waits for:
+// with the library's root and two divisions the step took 1.39 us per column,
+// with these 0.6 us.
+__device__ __forceinline__ void reflector_scalars(double s, double ax, double* n, double* rs,
+                                                  double* inv)
+{
+  double y, r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+  const double t = s * y;  // ~n
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(ax + t));
+  const double e = fma(-t, y, 1.0);  // n = t (1 - e)^(-1/2), rs = y (1 - e)^(-1/2)
+  const double q = e * fma(0.375, e, 0.5);
+  *n = fma(t, q, t);
+  *rs = fma(y, q, y);
+  const double f = fma(-*n, r, fma(-ax, r, 1.0));  // 1 / (ax + n) = r (1 + f + f^2 + ...)
+  *inv = fma(r, fma(f, f, f), r);
+}
+
+// Sign and magnitude tests on the bit patterns: a comparison of doubles is an
+// instruction of the FP64 pipe too.
+__device__ __forceinline__ bool not_negative(double x)  // -0.0 counts as 0
+{
+  const long long b = __double_as_longlong(x);
+  return b >= 0 || (b << 1) == 0;
+}
+__device__ __forceinline__ double copy_sign(double mag, bool positive)
+{
+  return __longlong_as_double(__double_as_longlong(mag) ^ (positive ? 0ll : (1ll << 63)));
+}
+
+// Sums of 16 values over the G lanes of a group by halving: lane gl ends with
+// value(s) i0 .. i0 + max(16 / G, 1) in acc[0..].
+template <int G>
+__device__ __forceinline__ void halving_sum(double (&acc)[16], int gl)
+{
+  int o = G / 2;
+#pragma unroll
+  for (int n = 8; n >= 1; n >>= 1)
+  {
+    if (o == 0)
+      break;
+    const bool up = (gl & o) != 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i < n)
+      {
+        const double keep = up ? acc[i + n] : acc[i];
+        const double send = up ? acc[i] : acc[i + n];
+        acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    o >>= 1;
+  }
+  if (G == 32)
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+}
+
+}  // namespace
+}  // namespace ttg

@@ -82,10 +82,11 @@ __device__ void wide_copy(const WideJob& job, double* dst, const double* src, in
 // two rounds for the work of one.  Returns false if a tensor-core wait
 // timed out (the grid error word is set).
 // fp64_only: FP64 tiles even when the sliced tensor-core tiles are on
-// (products whose error bound is stated for FP64).
+// (products whose error bound is stated for FP64).  tri: the zero triangle of
+// an R factor (GemmTri), whose part of K a tile skips.
 __device__ bool wide_gemm(const WideJob& job, int M, int N, int K, View A, View B, double* C,
                           int64_t c_rs, int64_t c_cs, WideSmem sm, CtaShared& sh,
-                          bool fp64_only = false)
+                          bool fp64_only = false, int tri = kTriNone)
 {
   if (!fp64_only && job.tc && sm.oz && K <= 512 &&
       static_cast<int64_t>(kOzSmemBytes) <= sm.cap * 8)
@@ -107,17 +108,24 @@ __device__ bool wide_gemm(const WideJob& job, int M, int N, int K, View A, View 
   auto put = [&](int i, int j, double v) { C[i * c_rs + j * c_cs] = v; };
   const bool ak = A.rs != 1, bk = B.cs != 1;  // load along the contiguous direction
   double* tile = sm.p;  // the dynamic shared memory is free between steps
+  auto k0 = [&](int i0, int j0) { return tri == kTriUpperA ? i0 : (tri == kTriLowerB ? j0 : 0); };
   if (rounds(32) * 4 <= rounds(16))
   {
     const int tm = (M + 31) / 32, tn = (N + 31) / 32;
     for (int t = job.rank; t < tm * tn; t += job.size)
-      grid_tile<2>((t / tn) * 32, (t % tn) * 32, M, N, 0, K, at(A), at(B), put, tile, ak, bk);
+    {
+      const int i0 = (t / tn) * 32, j0 = (t % tn) * 32;
+      grid_tile<2>(i0, j0, M, N, k0(i0, j0), K, at(A), at(B), put, tile, ak, bk);
+    }
   }
   else
   {
     const int tm = (M + 15) / 16, tn = (N + 15) / 16;
     for (int t = job.rank; t < tm * tn; t += job.size)
-      grid_tile<1>((t / tn) * 16, (t % tn) * 16, M, N, 0, K, at(A), at(B), put, tile, ak, bk);
+    {
+      const int i0 = (t / tn) * 16, j0 = (t % tn) * 16;
+      grid_tile<1>(i0, j0, M, N, k0(i0, j0), K, at(A), at(B), put, tile, ak, bk);
+    }
   }
   __syncthreads();
   return true;
@@ -719,7 +727,8 @@ __device__ bool wide_right_orth(const WideJob& job, CoreSlot* S, int d, WideSmem
     // prev (hp x kk) = left_unfold(prev) R^T.
     if (!wide_apply_q(job, w, kk, nullptr, 0, kk, cs, 1, w, true, sm, sh))
       return false;
-    if (!wide_gemm(job, hp, kk, r, View{ps, r, 1}, View{job.R, kk, 1}, job.Pb, kk, 1, sm, sh))
+    if (!wide_gemm(job, hp, kk, r, View{ps, r, 1}, View{job.R, kk, 1}, job.Pb, kk, 1, sm, sh, false,
+                   kTriLowerB))
       return false;
     WSYNC();
     wide_copy(job, ps, job.Pb, static_cast<int64_t>(hp) * kk);
@@ -733,52 +742,102 @@ __device__ bool wide_right_orth(const WideJob& job, CoreSlot* S, int d, WideSmem
   return true;
 }
 
+// Columns me + P w (+ multiples of 8 P) of R^-1 (R: c x c upper triangular,
+// column-major, c <= 32 E), one per warp, the vector in registers (row
+// lane + 32 e in x[e]).  With R = D Rt, Rt of unit diagonal, Rt z = D^-1 e_j: a
+// step is a broadcast of z_i and one FMA.  R passes through shared memory 32
+// columns at a time, the next 32 in flight.  Adds this lane's shares of
+// ||R^-1||_F^2 and ||R||_F^2.
+template <int E>
+__device__ __noinline__ void inverse_columns(const WideJob& job, int c, double* sm, double* zz,
+                                             double* rr)
+{
+  constexpr int kLd = 32 * E + 1;
+  const int P = job.size, me = job.rank;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double* dinv = sm;
+  double* stage = sm + 32 * E;
+  for (int i = threadIdx.x; i < c; i += blockDim.x)
+    dinv[i] = 1.0 / job.R[i + static_cast<int64_t>(i) * c];
+  // Columns [32 e, 32 e + 32) down to row 32 e + 31 into buffer e & 1.
+  auto load = [&](int e) {
+    double* buf = stage + (e & 1) * 32 * kLd;
+    const int rows = c < 32 * e + 32 ? c : 32 * e + 32;
+    for (int i = w; i < 32 && 32 * e + i < c; i += kWarps)
+      for (int r = lane; r < rows; r += 32)
+        copy_async(buf + i * kLd + r, job.R + r + static_cast<int64_t>(32 * e + i) * c, true);
+  };
+  for (int j0 = me; j0 < c; j0 += P * kWarps)
+  {
+    const int j = j0 + P * w;
+    int last = j0;  // the CTA's largest column
+    while (last + P < c && last + P < j0 + P * kWarps)
+      last += P;
+    __syncthreads();
+    double x[E], d[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+    {
+      const int i = lane + 32 * e;
+      const double r = j < c && i <= j ? job.R[i + static_cast<int64_t>(j) * c] : 0.0;
+      *rr = fma(r, r, *rr);
+      d[e] = i < c ? dinv[i] : 0.0;
+      x[e] = i == j ? d[e] : 0.0;
+    }
+    load(last / 32);
+#pragma unroll
+    for (int e = E - 1; e >= 0; --e)
+    {
+      if (32 * e > last)
+        continue;
+      copies_wait();
+      __syncthreads();
+      if (e > 0)
+        load(e - 1);
+      const double* buf = stage + (e & 1) * 32 * kLd;
+      if (j < c)
+        for (int i = j < 32 * e + 31 ? j : 32 * e + 31; i >= 32 * e; --i)
+        {
+          const double z = __shfl_sync(0xffffffffu, x[e], i & 31);
+          const double* col = buf + (i - 32 * e) * kLd + lane;
+#pragma unroll
+          for (int q = 0; q <= e; ++q)
+          {
+            const double rt = lane + 32 * q < i ? col[32 * q] * d[q] : 0.0;
+            x[q] = fma(-z, rt, x[q]);
+          }
+          if (lane == 0)
+            *zz = fma(z, z, *zz);
+        }
+      __syncthreads();  // buffer e & 1 is filled again two blocks on
+    }
+  }
+}
+
 // No-truncation certificate of the bond matrix X (h x c) from its QR's R in
 // job.R.  First by the inverse: the columns z_j of R^-1 are independent back
-// substitutions, a warp each, with no barrier among them (27 us for c = 257,
-// where one CTA's elimination of the Gram matrix is bound by that SM's FP64
-// rate: 0.7 ms).  The computed Z has R Z = I - E, |E| <= gamma_c |R| |Z|
-// (Higham, thm. 8.5), so
+// substitutions, a warp each, with no barrier among them, where one CTA's
+// elimination of the Gram matrix is bound by that SM's FP64 rate (0.7 ms at
+// c = 257).  The computed Z has R Z = I - E, |E| <= gamma_(c+2) |R| |Z|
+// (Higham, thm. 8.5, with two more roundings in the scaled columns), so
 //   sigma_min(R) >= (1 - g) / ||Z||_F,   g = gamma ||R||_F ||Z||_F.
 // Where that bound clears the elimination's own test with the elimination's
 // error to spare (tau of certify_tau, its error term twice), the elimination
-// would have met only positive pivots: the bond is certified.  Otherwise the
-// elimination decides, as it does alone in the per-TT sweep.
-__device__ bool wide_certify(const WideJob& job, int c, int h, double delta, WideSmem sm,
-                             CtaShared& sh, bool* certified)
+// would have met only positive pivots: the bond is certified.  Otherwise, and
+// for c > 288, the elimination decides, as it does alone in the per-TT sweep.
+__device__ __noinline__ bool wide_certify(const WideJob& job, int c, int h, double delta,
+                                          WideSmem sm, CtaShared& sh, bool* certified)
 {
   const int P = job.size, me = job.rank;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   constexpr double u = CertOps<double>::u;
   double zz = 0.0, rr = 0.0;
-  bool tried = static_cast<int64_t>(kWarps + 1) * c <= sm.cap;
+  const bool tried = c <= 288 && (2 * 32 * 289 + 288) <= sm.cap;
   if (tried)
   {
-    double* dinv = sm.p;
-    double* x = sm.p + static_cast<int64_t>(w + 1) * c;
-    for (int i = threadIdx.x; i < c; i += blockDim.x)
-      dinv[i] = 1.0 / job.R[i + static_cast<int64_t>(i) * c];
-    __syncthreads();
-    for (int j = me + P * w; j < c; j += P * kWarps)
-    {
-      for (int i = lane; i <= j; i += 32)
-      {
-        const double r = job.R[i + static_cast<int64_t>(j) * c];
-        rr = fma(r, r, rr);
-        x[i] = i == j ? 1.0 : 0.0;
-      }
-      __syncwarp();
-      for (int i = j; i >= 0; --i)
-      {
-        const double z = x[i] * dinv[i];
-        const double* col = job.R + static_cast<int64_t>(i) * c;
-        for (int q = lane; q < i; q += 32)
-          x[q] = fma(-z, col[q], x[q]);
-        if (lane == 0)
-          zz = fma(z, z, zz);
-        __syncwarp();
-      }
-    }
+    if (c <= 96)
+      inverse_columns<3>(job, c, sm.p, &zz, &rr);
+    else
+      inverse_columns<9>(job, c, sm.p, &zz, &rr);
   }
   zz = cta_sum(zz, sh);
   rr = cta_sum(rr, sh);
@@ -796,7 +855,7 @@ __device__ bool wide_certify(const WideJob& job, int c, int h, double delta, Wid
   }
   zz = sqrt(cta_sum(zz, sh));
   rr = sqrt(cta_sum(rr, sh));
-  const double g = 1.1 * (c + 4) * u * rr * zz;
+  const double g = 1.1 * (c + 6) * u * rr * zz;
   const double low = (1.0 - g) / zz;
   const double eR = static_cast<double>(c) * h * u * rr;
   const double tau = (1.0 + 4.0 * u) * (delta + eR) * (delta + eR) + 8.0 * (c + 1.0) * u * rr * rr;
@@ -823,11 +882,14 @@ __device__ bool wide_certify(const WideJob& job, int c, int h, double delta, Wid
 // Truncated SVD of X (h x c) over the grid, as left_svd of the per-TT
 // kernel (detail/truncate.hpp:61-99 branches): *r_new_out, U in job.Ub
 // (column-major, h x r_new), diag(s) V^T rows in job.F (row-major, r_new x
-// c).  X must not alias the work buffers (A, W, R, V, F, Ub, Pb, T1, T2).
+// c); *f_upper: F is the upper triangular R.  X must not alias the work buffers (A, W, R, V, F, Ub, Pb, T1, T2).
 __device__ bool wide_left_svd(const WideJob& job, View X, int h, int c, double delta, TTInfo& T,
-                              BondStat* bs, WideSmem sm, CtaShared& sh, int* r_new_out)
+                              BondStat* bs, WideSmem sm, CtaShared& sh, int* r_new_out,
+                              bool* f_upper = nullptr)
 {
   const int me = job.rank;
+  if (f_upper)
+    *f_upper = false;
   const bool lead = (me == 0 && threadIdx.x == 0);
   const int nsv = h < c ? h : c;
   const double floor2 = 1e-6 * delta * delta / static_cast<double>(nsv > 1 ? nsv : 1);
@@ -853,6 +915,8 @@ __device__ bool wide_left_svd(const WideJob& job, View X, int h, int c, double d
     {
       // Every singular value is kept: U = Q, F = R.
       r_new = c;
+      if (f_upper)
+        *f_upper = true;
       const int64_t cc = static_cast<int64_t>(c) * c;
       for (int64_t e = job.rank * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < cc;
            e += static_cast<int64_t>(job.size) * blockDim.x)
@@ -1022,10 +1086,12 @@ __device__ bool wide_round_tt(const WideJob& job, int tti, WideSmem sm, CtaShare
     double* ns = ar + S[k + 1].off;
     BondStat* bs = job.bond_stats ? job.bond_stats + T.first + k : nullptr;
     int r_new = 1;
-    if (!wide_left_svd(job, View{cs, c, 1}, h, c, delta, T, bs, sm, sh, &r_new))
+    bool upper = false;
+    if (!wide_left_svd(job, View{cs, c, 1}, h, c, delta, T, bs, sm, sh, &r_new, &upper))
       return false;
     // next (r_new x wn) = F right_unfold(next); core_k <- U (row-major).
-    if (!wide_gemm(job, r_new, wn, c, View{job.F, c, 1}, View{ns, wn, 1}, job.Pb, wn, 1, sm, sh))
+    if (!wide_gemm(job, r_new, wn, c, View{job.F, c, 1}, View{ns, wn, 1}, job.Pb, wn, 1, sm, sh, false,
+                   upper ? kTriUpperA : kTriNone))
       return false;
     WSYNC();
     wide_copy(job, ns, job.Pb, static_cast<int64_t>(r_new) * wn);
@@ -1081,7 +1147,8 @@ __device__ bool wide_round_right_tt(const WideJob& job, int tti, WideSmem sm, Ct
     // R (kk x rp) column-major in job.R.
     if (!wide_apply_q(job, h, kk, nullptr, 0, kk, cs, kk, 1, true, sm, sh))
       return false;
-    if (!wide_gemm(job, kk, wn, rp, View{job.R, 1, kk}, View{ns, wn, 1}, job.Pb, wn, 1, sm, sh))
+    if (!wide_gemm(job, kk, wn, rp, View{job.R, 1, kk}, View{ns, wn, 1}, job.Pb, wn, 1, sm, sh, false,
+                   kTriUpperA))
       return false;
     WSYNC();
     wide_copy(job, ns, job.Pb, static_cast<int64_t>(kk) * wn);
@@ -1105,11 +1172,13 @@ __device__ bool wide_round_right_tt(const WideJob& job, int tti, WideSmem sm, Ct
     double* cs = ar + S[k].off;
     double* ps = ar + S[k - 1].off;
     int r_new = 1;
-    if (!wide_left_svd(job, View{cs, 1, w}, w, r, delta, T, nullptr, sm, sh, &r_new))
+    bool upper = false;
+    if (!wide_left_svd(job, View{cs, 1, w}, w, r, delta, T, nullptr, sm, sh, &r_new, &upper))
       return false;
     // prev (hp x r_new) = left_unfold(prev) F^T, F (r_new x r) row-major in
     // job.F; core_k <- U^T, whose row-major layout is U's column-major one.
-    if (!wide_gemm(job, hp, r_new, r, View{ps, r, 1}, View{job.F, 1, r}, job.Pb, r_new, 1, sm, sh))
+    if (!wide_gemm(job, hp, r_new, r, View{ps, r, 1}, View{job.F, 1, r}, job.Pb, r_new, 1, sm, sh,
+                   false, upper ? kTriLowerB : kTriNone))
       return false;
     WSYNC();
     wide_copy(job, ps, job.Pb, static_cast<int64_t>(hp) * r_new);

@@ -34,6 +34,7 @@
 
 #include "ttg_device.cuh"
 #include "ttg_job.h"
+#include "ttg_reflector.cuh"
 
 namespace ttg
 {
@@ -51,22 +52,50 @@ __device__ __forceinline__ void packet_put(uint4* p, double v, uint32_t tag)
                : "memory");
 }
 
-// Waits for a packet; 0.0 and *fail = true when the wait gave up.
-__device__ __forceinline__ double packet_get(const WideJob& job, const uint4* p, uint32_t tag,
-                                             bool* fail)
+// A packet as it is now; true when it has arrived.
+__device__ __forceinline__ bool packet_try(const uint4* p, uint32_t tag, double* v)
 {
   uint32_t lo, t0, hi, t1;
+  asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(lo), "=r"(t0), "=r"(hi), "=r"(t1)
+               : "l"(p)
+               : "memory");
+  *v = __longlong_as_double(
+    static_cast<long long>((static_cast<unsigned long long>(hi) << 32) | lo));
+  return t0 == tag && t1 == tag;
+}
+
+// Waits for the packets p[0], p[stride], ... of which n <= N are wanted, all
+// polled together (one L2 round trip per attempt for the set, not one per
+// packet), and returns their sum in a fixed order; *fail = true when the wait
+// gave up.
+template <int N>
+__device__ __forceinline__ double packets_sum(const WideJob& job, const uint4* p, int64_t stride, int n,
+                                              uint32_t tag, bool* fail)
+{
+  double v[N];
   int polls = 0;
   long long start = 0;
   for (;;)
   {
-    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(lo), "=r"(t0), "=r"(hi), "=r"(t1)
-                 : "l"(p)
-                 : "memory");
-    if (t0 == tag && t1 == tag)
-      return __longlong_as_double(
-        static_cast<long long>((static_cast<unsigned long long>(hi) << 32) | lo));
+    uint32_t lo[N], t0[N], hi[N], t1[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+      asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(lo[e]), "=r"(t0[e]), "=r"(hi[e]), "=r"(t1[e])
+                   : "l"(p + (e < n ? e : 0) * stride)
+                   : "memory");
+    bool all = true;
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+    {
+      all = all && t0[e] == tag && t1[e] == tag;
+      v[e] = e < n ? __longlong_as_double(static_cast<long long>(
+                       (static_cast<unsigned long long>(hi[e]) << 32) | lo[e]))
+                   : 0.0;
+    }
+    if (all)
+      break;
     if ((++polls & 255) == 0)
     {
       if (start == 0)
@@ -81,6 +110,13 @@ __device__ __forceinline__ double packet_get(const WideJob& job, const uint4* p,
       }
     }
   }
+#pragma unroll
+  for (int w = N / 2; w > 0; w >>= 1)
+#pragma unroll
+    for (int e = 0; e < N / 2; ++e)
+      if (e < w && e + w < n)
+        v[e] += v[e + w];
+  return v[0];
 }
 
 // Slots: panel products (slab, column), the panel row's own entries, and the
@@ -147,25 +183,20 @@ __device__ __noinline__ bool wide_panel(const WideJob& job, int h, int k, int j0
     const int lo = j + 1 > r0 ? j + 1 - r0 : 0;  // first slab row below the diagonal
     const bool owner = j >= r0 && j < r0 + nr;
     const double* x = P + i * ld;
-    // Products of x below row j: 8 lanes per panel column on four warps (one
-    // per FP64 pipe: more lanes per column only add reduction steps).
+    // Products of x below row j: 8 lanes per panel column on four warps, one
+    // per FP64 pipe.  A warp's FP64 instruction holds its pipe for 64 clocks,
+    // which is also its latency: what counts is their number, so one chain
+    // per lane and no more lanes than this.
     if (t < 8 * kPb)
     {
       const int l = t >> 3, g = t & 7;
-      double a0 = 0.0, a1 = 0.0;
+      double a0 = 0.0;
       if (l < nb)
       {
         const double* y = P + l * ld;
-        int r = lo + g;
-        for (; r + 8 < nr; r += 16)
-        {
-          a0 = fma(x[r], y[r], a0);
-          a1 = fma(x[r + 8], y[r + 8], a1);
-        }
-        if (r < nr)
+        for (int r = lo + g; r < nr; r += 8)
           a0 = fma(x[r], y[r], a0);
       }
-      a0 += a1;
       a0 += __shfl_xor_sync(0xffffffffu, a0, 4);
       a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
       a0 += __shfl_xor_sync(0xffffffffu, a0, 1);
@@ -191,10 +222,15 @@ __device__ __noinline__ bool wide_panel(const WideJob& job, int h, int k, int j0
     if (S > 1 && t < 8 * kPb)
     {
       const int l = t >> 3, g = t & 7;
+      static_assert(kWidePanelSlabs == 32, "up to four packets per lane");
       double v = 0.0;
-      if (l < nb)
-        for (int s = g; s < S; s += 8)
-          v += packet_get(job, panel_slot(job, tag, s, l), tag, &fail);
+      if (l < nb && g < S)
+      {
+        const int n = (S - g + 7) / 8;
+        const uint4* p = panel_slot(job, tag, g, l);
+        v = S <= 8 ? packets_sum<1>(job, p, 8 * kPb, n, tag, &fail)
+                   : packets_sum<4>(job, p, 8 * kPb, n, tag, &fail);
+      }
       __syncwarp();
       v += __shfl_xor_sync(0xffffffffu, v, 4);
       v += __shfl_xor_sync(0xffffffffu, v, 2);
@@ -203,46 +239,52 @@ __device__ __noinline__ bool wide_panel(const WideJob& job, int h, int k, int j0
         ps.d[l] = v;
     }
     else if (S > 1 && t < 8 * kPb + nb)
-      ps.row[t - 8 * kPb] = packet_get(job, panel_slot(job, tag, kWidePanelSlabs, t - 8 * kPb), tag,
-                                       &fail);
+      ps.row[t - 8 * kPb] =
+        packets_sum<1>(job, panel_slot(job, tag, kWidePanelSlabs, t - 8 * kPb), 0, 1, tag, &fail);
     if (__syncthreads_or(fail))
       return false;
-    // The reflector, and what it takes from each later column.
-    if (w == 0)
+    // The reflector, and what it takes from each later column.  tau inv =
+    // +-1 / n: warp 0 forms what the update below waits for, warps 1 and 2 (on
+    // other pipes, the same scalars again) the rest.
+    if (w < 3)
     {
       const double tail2 = ps.d[i], x0 = ps.row[i];
-      double beta = x0, tau = 0.0, inv = 0.0;
-      if (!(tail2 <= DBL_MIN))
+      const bool up = not_negative(x0);
+      double beta = x0, tau = 0.0, inv = 0.0, wi = 0.0;
+      if (__double_as_longlong(tail2) > __double_as_longlong(DBL_MIN))  // tail2 >= 0, or a NaN
       {
-        const double s = fma(x0, x0, tail2);
-        const double rs = rsqrt(s);
-        double n = s * rs;  // |x|, one Newton step from the reciprocal root
-        n = fma(fma(-n, n, s), 0.5 * rs, n);
+        double n, rs;
         const double ax = fabs(x0);
-        inv = 1.0 / (ax + n);
-        inv = x0 >= 0.0 ? inv : -inv;
-        beta = x0 >= 0.0 ? -n : n;
-        tau = (n + ax) / n;
+        reflector_scalars(fma(x0, x0, tail2), ax, &n, &rs, &inv);
+        inv = copy_sign(inv, up);
+        wi = copy_sign(rs, up);
+        beta = copy_sign(n, !up);
+        tau = fma(ax, rs, 1.0);  // (n + |x0|) / n
       }
-      if (lane < nb)
+      const int l = lane < nb ? lane : 0;
+      const double dot = fma(inv, ps.d[l], ps.row[l]);
+      if (w == 0)
       {
-        if (lane > i)
-        {
-          const double dot = tau * fma(inv, ps.d[lane], ps.row[lane]);
-          ps.w[lane] = dot * inv;
-          if (owner)
-            P[lane * ld + j - r0] = ps.row[lane] - dot;
-        }
-        else if (lane < i)  // v_l . v_i, v_l = inv_l x_l
-          ps.G[lane + i * kPb] = ps.inv[lane] * fma(inv, ps.d[lane], ps.row[lane]);
+        if (lane > i && lane < nb)
+          ps.w[lane] = dot * wi;
       }
-      __syncwarp();
-      if (lane == 0)
+      else if (w == 1)
       {
-        ps.inv[i] = inv;
-        ps.tau[i] = tau;
-        if (owner)
+        if (owner && lane > i && lane < nb)
+          P[lane * ld + j - r0] = fma(-tau, dot, ps.row[lane]);
+        if (owner && lane == i)
           P[i * ld + j - r0] = beta;
+      }
+      else
+      {
+        // G(l, i) = v_l . v_i, v_l = inv_l x_l.
+        if (lane < i)
+          ps.G[lane + i * kPb] = ps.inv[lane] * dot;
+        if (lane == i)
+        {
+          ps.inv[i] = inv;
+          ps.tau[i] = tau;
+        }
       }
     }
     __syncthreads();
@@ -284,14 +326,15 @@ __device__ __noinline__ bool wide_panel(const WideJob& job, int h, int k, int j0
 // How a matrix of `hp` rows and m columns is cut for a block's application:
 // St slabs of `rows` rows times Gt groups of at most nc columns.  The cost is
 // the FP64 clocks of the fullest CTA: 2 kPb FMAs per element at 2 per clock,
-// the slabs' sums, and an exchange's latency.
+// the slabs' sums, and an exchange's latency (~1.8 us measured).
 struct TrailCut
 {
   int St, Gt, rows, nc;
 };
 
 // Lane s - 1 of every warp weighs s slabs; all lanes of the CTA get the cut.
-__device__ TrailCut trail_cut(int hp, int m, int P, int64_t cap)
+// nv: V slabs held at once (wide_q loads the next block's beside this one's).
+__device__ TrailCut trail_cut(int hp, int m, int P, int64_t cap, int nv)
 {
   const int s = (threadIdx.x & 31) + 1;
   const int most = P < kWideTrailSlabs ? P : kWideTrailSlabs;
@@ -308,10 +351,22 @@ __device__ TrailCut trail_cut(int hp, int m, int P, int64_t cap)
   {
     const TrailCut k = cut_of(s);
     const int64_t need =
-      static_cast<int64_t>(kPb + k.nc) * (k.rows | 1) + 2 * kPb * k.nc + kPb * kPb;
+      static_cast<int64_t>(nv * kPb + k.nc) * (k.rows | 1) + 2 * kPb * k.nc + nv * kPb * kPb;
+    // Columns and rows as the lanes of block_apply cover them, on the busiest
+    // of the four FP64 pipes; wide_q starts with few of its columns and ends
+    // with all, so it is weighed at four points between.
+    auto clocks = [&](int nc) {
+      const int w = nc <= 8 ? 4 : (nc <= 16 ? 8 : 16), G = nc <= 8 ? 32 : (nc <= 16 ? 16 : 8);
+      return static_cast<unsigned long long>(kPb) * ((nc + w - 1) / w * w) *
+             ((k.rows + G - 1) / G * G);
+    };
+    const unsigned long long work =
+      nv == 1 ? clocks(k.nc)
+              : (clocks((k.nc + 3) / 4) + clocks((k.nc + 1) / 2) + clocks((3 * k.nc + 3) / 4) +
+                 clocks(k.nc)) /
+                  4;
     if (need <= cap)
-      best = (static_cast<unsigned long long>(kPb) * k.nc * k.rows + 8ull * k.nc * k.St +
-              (k.St > 1 ? 2500 : 0))
+      best = (work + 8ull * k.nc * k.St + (k.St > 1 ? 3500 : 0))
                << 5 |
              static_cast<unsigned>(s - 1);
   }
@@ -324,32 +379,6 @@ __device__ TrailCut trail_cut(int hp, int m, int P, int64_t cap)
   if (best == ~0ull)
     return TrailCut{0, 0, 0, 0};
   return cut_of(static_cast<int>(best & 31) + 1);
-}
-
-// Sums of 16 values over the G lanes of a group by halving: lane gl ends with
-// value(s) i0 .. i0 + max(16 / G, 1) in acc[0..].
-template <int G>
-__device__ __forceinline__ void halving_sum(double (&acc)[kPb], int gl)
-{
-  int o = G / 2;
-#pragma unroll
-  for (int n = kPb / 2; n >= 1; n >>= 1)
-  {
-    if (o == 0)
-      break;
-    const bool up = (gl & o) != 0;
-#pragma unroll
-    for (int i = 0; i < kPb / 2; ++i)
-      if (i < n)
-      {
-        const double keep = up ? acc[i + n] : acc[i];
-        const double send = up ? acc[i] : acc[i + n];
-        acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-      }
-    o >>= 1;
-  }
-  if (G == 32)
-    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
 }
 
 // The tile B (nr x nc in shared memory, column-major, ldb) <- its rows of
@@ -402,10 +431,11 @@ __device__ __forceinline__ bool block_apply_g(const WideJob& job, const double* 
   if (St > 1)
     for (int e = t; e < nc * kPb; e += kThreads)
     {
-      const int c = col(e / kPb);
-      double v = 0.0;
-      for (int s = 0; s < St; ++s)
-        v += packet_get(job, trail_slot(job, tag, s, c, e % kPb), tag, &fail);
+      const uint4* p = trail_slot(job, tag, 0, col(e / kPb), e % kPb);
+      const int64_t stride = job.c_max * kPb;
+      double v = packets_sum<8>(job, p, stride, St < 8 ? St : 8, tag, &fail);
+      if (St > 8)
+        v += packets_sum<8>(job, p + 8 * stride, stride, St - 8, tag, &fail);
       Ws[e] = v;
     }
   if (__syncthreads_or(fail))
@@ -431,7 +461,20 @@ __device__ __forceinline__ bool block_apply_g(const WideJob& job, const double* 
     for (int i = 0; i < kPb; ++i)
       z[i] = -Zs[q * kPb + i];
     double* y = Bs + q * ldb;
-    for (int r = gl; r < nr; r += G)
+    int r = gl;
+    for (; r + G < nr; r += 2 * G)  // two rows at a time: independent chains
+    {
+      double b = y[r], b2 = y[r + G];
+#pragma unroll
+      for (int i = 0; i < kPb; ++i)
+      {
+        b = fma(z[i], Vs[i * ldv + r], b);
+        b2 = fma(z[i], Vs[i * ldv + r + G], b2);
+      }
+      y[r] = b;
+      y[r + G] = b2;
+    }
+    if (r < nr)
     {
       double b = y[r];
 #pragma unroll
@@ -457,17 +500,34 @@ __device__ bool block_apply(const WideJob& job, const double* Vs, int ldv, doubl
   return block_apply_g<32, kTrans>(job, Vs, ldv, Bs, ldb, nr, nc, Ts, Ws, Zs, St, slab, tag, col);
 }
 
-// V's rows [r0, r0 + nr) of the block at j0 (zero above row j0 and past nb),
-// and the block's T, into shared memory.
+// 8 bytes from global to shared memory, in flight until copies_wait; zeros
+// where !in (src is not read).
+__device__ __forceinline__ void copy_async(double* dst, const double* src, bool in)
+{
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(in ? 8 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void copies_wait()
+{
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// Starts the copies of V's rows [r0, r0 + nr) of the block at j0 (zero above
+// row j0 and past nb) and of the block's T into shared memory.
 __device__ __forceinline__ void load_block(const WideJob& job, int h, int j0, int nb, int r0, int nr,
                                            double* Vs, int ldv, double* Ts)
 {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int i = w; i < kPb; i += kWarps)
+  {
+    const double* col = job.W + static_cast<int64_t>(i < nb ? j0 + i : j0) * h + r0;
     for (int r = lane; r < nr; r += 32)
-      Vs[i * ldv + r] = (i < nb && r0 + r >= j0) ? job.W[static_cast<int64_t>(j0 + i) * h + r0 + r] : 0.0;
+      copy_async(Vs + i * ldv + r, col + r, i < nb && r0 + r >= j0);
+  }
   for (int e = threadIdx.x; e < kPb * kPb; e += kThreads)
-    Ts[e] = job.Tw[static_cast<int64_t>(j0 / kPb) * kPb * kPb + e];
+    copy_async(Ts + e, job.Tw + static_cast<int64_t>(j0 / kPb) * kPb * kPb + e, true);
 }
 
 // W's columns from j0 + nb on <- (I - V T^T V^T) W, V the block at j0.
@@ -475,7 +535,7 @@ __device__ __noinline__ bool wide_trail(const WideJob& job, int h, int c, int j0
                                         double* sm, int64_t cap)
 {
   const int c0 = j0 + nb, m = c - c0, hp = h - j0;
-  const TrailCut cut = trail_cut(hp, m, job.size, cap);
+  const TrailCut cut = trail_cut(hp, m, job.size, cap, 1);
   const int slab = job.rank % cut.St, g = job.rank / cut.St;
   if (g >= cut.Gt)
     return true;
@@ -496,7 +556,8 @@ __device__ __noinline__ bool wide_trail(const WideJob& job, int h, int c, int j0
   double* B = job.W + static_cast<int64_t>(c0 + q0) * h + r0;
   for (int q = w; q < nc; q += kWarps)
     for (int r = lane; r < nr; r += 32)
-      Bs[q * ld + r] = B[static_cast<int64_t>(q) * h + r];
+      copy_async(Bs + q * ld + r, B + static_cast<int64_t>(q) * h + r, true);
+  copies_wait();
   __syncthreads();
   if (!block_apply<true>(job, Vs, ld, Bs, ld, nr, nc, Ts, Ws, Zs, cut.St, slab, tag,
                          [&](int q) { return q0 + q; }))
@@ -515,7 +576,7 @@ __device__ __noinline__ bool wide_q(const WideJob& job, int h, int kref, const d
                                     int ncols, double* out, int64_t o_rs, int64_t o_cs, bool eye,
                                     uint32_t seq, double* sm, int64_t cap)
 {
-  const TrailCut cut = trail_cut(h, ncols, job.size, cap);
+  const TrailCut cut = trail_cut(h, ncols, job.size, cap, 2);
   const int slab = job.rank % cut.St, g = job.rank / cut.St;
   if (g >= cut.Gt)
     return true;
@@ -525,11 +586,11 @@ __device__ __noinline__ bool wide_q(const WideJob& job, int h, int kref, const d
   // from its own first on, so every group gets some of each.
   const int nc = (ncols - g + cut.Gt - 1) / cut.Gt;
   const int ld = cut.rows | 1;
-  double* Vs = sm;
-  double* Bs = Vs + kPb * ld;
+  double* Vs = sm;  // two slabs
+  double* Bs = Vs + 2 * kPb * ld;
   double* Ws = Bs + cut.nc * ld;
   double* Zs = Ws + kPb * cut.nc;
-  double* Ts = Zs + kPb * cut.nc;
+  double* Ts = Zs + kPb * cut.nc;  // two blocks' T
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int q = w; q < nc; q += kWarps)
   {
@@ -542,18 +603,29 @@ __device__ __noinline__ bool wide_q(const WideJob& job, int h, int kref, const d
     }
   }
   const int blocks = (kref + kPb - 1) / kPb;
-  for (int b = blocks - 1; b >= 0; --b)
-  {
+  // First of this group's columns that block b touches.
+  auto first_col = [&](int b) {
+    return eye && b * kPb > g ? (b * kPb - g + cut.Gt - 1) / cut.Gt : 0;
+  };
+  auto load = [&](int b, int buf) {
     const int j0 = b * kPb;
-    const int nb = kref - j0 < kPb ? kref - j0 : kPb;
-    int qa = 0;  // first column that the block touches
-    if (eye && j0 > g)
-      qa = (j0 - g + cut.Gt - 1) / cut.Gt;
-    if (qa >= nc)
-      continue;
-    load_block(job, h, j0, nb, r0, nr, Vs, ld, Ts);
+    load_block(job, h, j0, kref - j0 < kPb ? kref - j0 : kPb, r0, nr, Vs + buf * kPb * ld, ld,
+               Ts + buf * kPb * kPb);
+  };
+  int b = blocks - 1;
+  while (b >= 0 && first_col(b) >= nc)
+    --b;
+  if (b >= 0)
+    load(b, 0);
+  for (int buf = 0; b >= 0; --b, buf ^= 1)
+  {
+    copies_wait();
     __syncthreads();
-    if (!block_apply<false>(job, Vs, ld, Bs + qa * ld, ld, nr, nc - qa, Ts, Ws, Zs, cut.St, slab,
+    if (b > 0)
+      load(b - 1, buf ^ 1);  // in flight while this block is applied
+    const int qa = first_col(b);
+    if (!block_apply<false>(job, Vs + buf * kPb * ld, ld, Bs + qa * ld, ld, nr, nc - qa,
+                            Ts + buf * kPb * kPb, Ws, Zs, cut.St, slab,
                             seq + static_cast<uint32_t>(blocks - 1 - b),
                             [&](int q) { return g + cut.Gt * (qa + q); }))
       return false;
@@ -583,7 +655,7 @@ __device__ bool wide_blocked_fits(int h, int c, int P, int64_t cap)
 {
   const int64_t panel = static_cast<int64_t>(kPb) * (panel_rows(h, P) | 1) +
                         static_cast<int64_t>(sizeof(PanelShared) / sizeof(double));
-  return panel <= cap && trail_cut(h, c, P, cap).St > 0;
+  return panel <= cap && trail_cut(h, c, P, cap, 2).St > 0;
 }
 
 }  // namespace
