@@ -128,8 +128,13 @@ typedef struct ttg_tensor {
   int32_t* cols;    /* d: n_k of a TT-matrix; NULL for a TT */
   int64_t* offsets; /* d+1: core k = data[offsets[k] .. offsets[k+1]) */
   double* data;
-  int32_t owned;    /* set by the library on outputs */
+  int32_t owned;    /* set by the library on outputs; inputs: see below */
 } ttg_tensor;
+
+/* Value of `owned` of an input whose cores do not follow one another in one
+ * buffer: core k starts at data[offsets[k]] (its size is that of its shape),
+ * offsets[d] is not read.  Cores need not be copied together to be passed. */
+#define TTG_CORES_APART 0x5ca7a
 
 /* ---- library ---------------------------------------------------------- */
 const char* ttg_version(void);

@@ -216,26 +216,40 @@ def kernel_launches() -> int:
 
 
 # -- marshalling ---------------------------------------------------------------
+_CORES_APART = 0x5ca7a  # TTG_CORES_APART
+
+
 class _In:
-    """Keeps the numpy buffers of an input tensor alive for one call."""
+    """An input tensor for one call: the cores where they lie (offsets from
+    the first), or copied together when one of them is not contiguous float64
+    at a multiple of 8 bytes from it."""
 
     def __init__(self, cores):
         cores = [np.ascontiguousarray(c, dtype=np.float64) for c in cores]
         self.d = len(cores)
         self.matrix = self.d > 0 and cores[0].ndim == 4
+        owned = 0
         if self.d:
             self.ranks = np.array([cores[0].shape[0]] + [c.shape[-1] for c in cores], np.int32)
             self.rows = np.array([c.shape[1] for c in cores], np.int32)
             self.cols = np.array([c.shape[2] for c in cores], np.int32) if self.matrix else None
-            sizes = [c.size for c in cores]
-            self.offsets = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
-            self.data = np.concatenate([c.ravel() for c in cores])
+            at = [c.__array_interface__["data"][0] for c in cores]
+            if all((a - at[0]) % 8 == 0 for a in at) and at[0] % 8 == 0:
+                self.data = cores
+                self.offsets = np.array([(a - at[0]) // 8 for a in at] + [0], np.int64)
+                owned, data = _CORES_APART, at[0]
+            else:
+                sizes = [c.size for c in cores]
+                self.offsets = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+                self.data = np.concatenate([c.ravel() for c in cores])
+                data = self.data.ctypes.data
         else:
             self.ranks = np.ones(1, np.int32)
             self.rows = np.zeros(1, np.int32)
             self.cols = None
             self.offsets = np.zeros(1, np.int64)
             self.data = np.zeros(1, np.float64)
+            data = self.data.ctypes.data
         t = _Tensor()
         t.d = self.d
         t.ranks = self.ranks.ctypes.data_as(C.POINTER(C.c_int32))
@@ -243,24 +257,39 @@ class _In:
         t.cols = (self.cols.ctypes.data_as(C.POINTER(C.c_int32)) if self.cols is not None
                   else C.POINTER(C.c_int32)())
         t.offsets = self.offsets.ctypes.data_as(C.POINTER(C.c_int64))
-        t.data = self.data.ctypes.data_as(C.POINTER(C.c_double))
-        t.owned = 0
+        t.data = C.cast(C.c_void_p(data), C.POINTER(C.c_double))
+        t.owned = owned
         self.t = t
 
 
-def _out_to_cores(t: _Tensor):
+class _Owned:
+    """The buffer of an output tensor, freed with the last array on it."""
+
+    def __init__(self, t, size):
+        self.t = _Tensor.from_buffer_copy(t)
+        self.free = lib().ttg_free
+        self.__array_interface__ = {
+            "shape": (size,), "typestr": "<f8", "version": 3,
+            "data": (C.cast(t.data, C.c_void_p).value, False)}
+
+    def __del__(self):
+        self.free(C.byref(self.t))
+
+
+def _take(t: _Tensor):
+    """The cores of an output tensor: arrays on its buffer, which they own."""
     d = t.d
-    matrix = bool(t.cols)
+    if d == 0:
+        lib().ttg_free(C.byref(t))
+        return []
+    ranks, rows, offsets = t.ranks[:d + 1], t.rows[:d], t.offsets[:d + 1]
+    cols = t.cols[:d] if t.cols else None
+    buf = np.asarray(_Owned(t, max(offsets[d], 1)))
     cores = []
     for k in range(d):
-        r, rp = t.ranks[k], t.ranks[k + 1]
-        n = t.rows[k]
-        shape = (r, n, t.cols[k], rp) if matrix else (r, n, rp)
-        size = int(np.prod(shape))
-        off = t.offsets[k]
-        buf = np.ctypeslib.as_array(t.data, shape=(t.offsets[d],)) if t.offsets[d] else None
-        cores.append(np.array(buf[off:off + size]).reshape(shape) if size else
-                     np.zeros(shape))
+        shape = ((ranks[k], rows[k], ranks[k + 1]) if cols is None
+                 else (ranks[k], rows[k], cols[k], ranks[k + 1]))
+        cores.append(buf[offsets[k]:offsets[k + 1]].reshape(shape))
     return cores
 
 
@@ -287,13 +316,6 @@ def _opts(o: RoundOptions | None) -> _Opts:
 def _result(r: _Result) -> RoundResult:
     return RoundResult(r.iters_run, bool(r.converged), r.final_resid, r.norm, r.delta,
                        r.device_ms, r.status, r.jacobi_sweeps, r.sketch_state, r.sketch_rel_err)
-
-
-def _take(out: _Tensor):
-    try:
-        return _out_to_cores(out)
-    finally:
-        lib().ttg_free(C.byref(out))
 
 
 # -- public operations -----------------------------------------------------------

@@ -133,7 +133,7 @@ int32_t describe(const ttg_tensor* t, const char* op, Shape& s)
       return fail(TTG_ERR_SHAPE, std::string(op) + ": core size exceeds INT_MAX");
     s.size.push_back(sz);
     const int64_t o = t->offsets ? t->offsets[k] : off;
-    if (t->offsets && t->offsets[k + 1] - t->offsets[k] != sz)
+    if (t->offsets && t->owned != TTG_CORES_APART && t->offsets[k + 1] - t->offsets[k] != sz)
       return fail(TTG_ERR_SHAPE, std::string(op) + ": offsets do not match core " +
                                      std::to_string(k) + " size");
     s.src_off.push_back(o);
@@ -195,14 +195,21 @@ struct HostPinned
 
 size_t align256(size_t b) { return (b + 255) & ~static_cast<size_t>(255); }
 
-// fn(i) for i in [0, n) on up to 16 host threads (packing and unpacking of
+// Threads for moving `bytes` of host memory: one per 4 MB, up to 16 (starting
+// one costs about what copying 0.2 MB does).
+int64_t host_threads(size_t bytes)
+{
+  return std::min<int64_t>(16, 1 + static_cast<int64_t>(bytes >> 22));
+}
+
+// fn(i) for i in [0, n) on up to `most` host threads (packing and unpacking of
 // many tensors is memcpy-bound; one thread would take longer than the
 // sweep).  Returns the first non-OK status.
 template <class Fn>
-int32_t parallel_for(int64_t n, Fn fn)
+int32_t parallel_for(int64_t n, int64_t most, Fn fn)
 {
   const int64_t hw = std::max<int64_t>(1, std::thread::hardware_concurrency());
-  const int64_t nt = std::min<int64_t>({16, hw, n});
+  const int64_t nt = std::min<int64_t>({most, hw, n});
   if (nt <= 1)
   {
     for (int64_t i = 0; i < n; ++i)
@@ -295,6 +302,10 @@ struct ttg_plan
          total_bytes = 0;
   DevMem dev;
   HostPinned host;
+  // One-shot calls upload a few large cores straight from the caller's memory
+  // (direct, set in layout_and_alloc) instead of through the pinned image.
+  bool one_shot = false;
+  bool direct = false;
   // eval plans
   const int32_t* eval_idx = nullptr;
   int64_t M = 0;
@@ -670,6 +681,13 @@ int32_t layout_and_alloc(ttg_plan& P)
                        static_cast<size_t>(std::max(P.grid, P.scratch_ctas)));
   P.total_bytes = o;
   TTG_CUDA(P.dev.ensure(P.total_bytes));
+  // Uploads from the caller's pageable memory run at the rate of pinned ones
+  // here (160-190 GB/s from 16 MB on), so where there are few copies to issue
+  // staging is a pass of host memory for nothing.  (Downloads are staged: into
+  // fresh memory they took 60 ms for 134 MB, 12 ms through the pinned image.)
+  const size_t arena_bytes = sizeof(double) * static_cast<size_t>(P.arena_doubles);
+  P.direct = P.one_shot && P.slots.size() <= 512 && arena_bytes >= (size_t{16} << 20) &&
+             arena_bytes / std::max<size_t>(P.slots.size(), 1) >= (size_t{256} << 10);
   TTG_CUDA(P.host.ensure(P.prefix_bytes));
   TTG_CUDA(cudaEventCreate(&P.ev0));
   TTG_CUDA(cudaEventCreate(&P.ev1));
@@ -680,14 +698,16 @@ int32_t layout_and_alloc(ttg_plan& P)
   char* h = static_cast<char*>(P.host.p);
   std::memset(h + P.off_slots, 0, P.prefix_bytes - P.off_slots);
   double* arena = reinterpret_cast<double*>(h + P.off_arena);
-  parallel_for(static_cast<int64_t>(P.shapes.size()), [&](int64_t t) -> int32_t {
-    const Shape& s = P.shapes[static_cast<size_t>(t)];
-    const TTInfo& ti = P.tts[static_cast<size_t>(t)];
-    for (int k = 0; k < s.d; ++k)
-      std::memcpy(arena + P.slots[ti.first + k].off, s.data + s.src_off[k],
-                  sizeof(double) * static_cast<size_t>(s.size[k]));
-    return TTG_OK;
-  });
+  if (!P.direct)
+    parallel_for(static_cast<int64_t>(P.shapes.size()), host_threads(arena_bytes),
+                 [&](int64_t t) -> int32_t {
+                   const Shape& s = P.shapes[static_cast<size_t>(t)];
+                   const TTInfo& ti = P.tts[static_cast<size_t>(t)];
+                   for (int k = 0; k < s.d; ++k)
+                     std::memcpy(arena + P.slots[ti.first + k].off, s.data + s.src_off[k],
+                                 sizeof(double) * static_cast<size_t>(s.size[k]));
+                   return TTG_OK;
+                 });
   std::memcpy(h + P.off_slots, P.slots.data(), sizeof(CoreSlot) * P.slots.size());
   std::memcpy(h + P.off_tts, P.tts.data(), sizeof(TTInfo) * P.tts.size());
   std::memcpy(h + P.off_order, P.order.data(), sizeof(int32_t) * P.order.size());
@@ -840,8 +860,24 @@ int32_t build_round_plan(ttg_plan& P, int32_t count, const ttg_tensor* ins,
 int32_t plan_upload(ttg_plan& P, cudaStream_t st)
 {
   char* d = static_cast<char*>(P.dev.p);
-  TTG_CUDA(cudaMemcpyAsync(d + P.off_pristine, P.host.p, P.prefix_bytes, cudaMemcpyHostToDevice,
-                           st));
+  if (!P.direct)
+  {
+    TTG_CUDA(cudaMemcpyAsync(d + P.off_pristine, P.host.p, P.prefix_bytes, cudaMemcpyHostToDevice,
+                             st));
+    return TTG_OK;
+  }
+  TTG_CUDA(cudaMemcpyAsync(d + P.off_pristine + P.off_slots,
+                           static_cast<char*>(P.host.p) + P.off_slots, P.prefix_bytes - P.off_slots,
+                           cudaMemcpyHostToDevice, st));
+  double* arena = reinterpret_cast<double*>(d + P.off_pristine + P.off_arena);
+  for (size_t t = 0; t < P.shapes.size(); ++t)
+  {
+    const Shape& s = P.shapes[t];
+    for (int k = 0; k < s.d; ++k)
+      TTG_CUDA(cudaMemcpyAsync(arena + P.slots[P.tts[t].first + k].off, s.data + s.src_off[k],
+                               sizeof(double) * static_cast<size_t>(s.size[k]),
+                               cudaMemcpyHostToDevice, st));
+  }
   return TTG_OK;
 }
 
@@ -945,9 +981,10 @@ int32_t plan_download_raw(ttg_plan& P, cudaStream_t st)
   return TTG_OK;
 }
 
-// Builds an output tensor from TT `t` of the downloaded host image.
+// Builds an output tensor from TT `t` of the downloaded host image.  alone:
+// the call's only output.
 int32_t emit_tensor(ttg_plan& P, int t, bool matrix, const std::vector<int>& mrow,
-                    const std::vector<int>& ncol, ttg_tensor* out)
+                    const std::vector<int>& ncol, ttg_tensor* out, bool alone = true)
 {
   const char* h = static_cast<const char*>(P.host.p);
   const CoreSlot* S = reinterpret_cast<const CoreSlot*>(h + P.off_slots);
@@ -981,13 +1018,16 @@ int32_t emit_tensor(ttg_plan& P, int t, bool matrix, const std::vector<int>& mro
   out->data = static_cast<double*>(std::malloc(sizeof(double) * std::max<int64_t>(total, 1)));
   if (!out->data)
     return fail(TTG_ERR_OOM, "host allocation failed");
-  for (int k = 0; k < d; ++k)
-  {
-    const CoreSlot& c = S[ti.first + k];
-    std::memcpy(out->data + out->offsets[k], arena + c.off,
-                sizeof(double) * static_cast<size_t>(static_cast<int64_t>(c.r) * c.n * c.rp));
-  }
-  return TTG_OK;
+  // The only tensor of a call is copied by several threads, core by core; of
+  // many, each by one of the caller's.
+  return parallel_for(d, alone ? host_threads(sizeof(double) * static_cast<size_t>(total)) : 1,
+                      [&](int64_t k) -> int32_t {
+                        const CoreSlot& c = S[ti.first + k];
+                        std::memcpy(out->data + out->offsets[k], arena + c.off,
+                                    sizeof(double) * static_cast<size_t>(
+                                                       static_cast<int64_t>(c.r) * c.n * c.rp));
+                        return TTG_OK;
+                      });
 }
 
 void fill_result(const TTInfo& ti, float ms, ttg_round_result* r)
@@ -1029,7 +1069,7 @@ struct DeviceState
   std::once_flag stream_once, stream2_once;
   cudaStream_t stream = nullptr;
   cudaStream_t stream2 = nullptr;  // the second chunk of a pipelined batch
-  DevMem dev_pool, dev_pool2;
+  DevMem dev_pool, dev_pool2, wide_pool;
   HostPinned host_pool, host_pool2;
 };
 
@@ -1063,23 +1103,28 @@ cudaStream_t lib_stream2()
 struct PoolLease
 {
   ttg_plan& P;
+  DeviceState& D;
   DevMem& dev;
   HostPinned& host;
+  const bool wide;  // slot 0 also lends the whole-GPU work buffers
   explicit PoolLease(ttg_plan& p, int slot = 0)
-    : P(p), dev(slot ? dev_state().dev_pool2 : dev_state().dev_pool),
-      host(slot ? dev_state().host_pool2 : dev_state().host_pool)
+    : P(p), D(dev_state()), dev(slot ? D.dev_pool2 : D.dev_pool),
+      host(slot ? D.host_pool2 : D.host_pool), wide(slot == 0)
   {
-    std::swap(P.dev.p, dev.p);
-    std::swap(P.dev.bytes, dev.bytes);
-    std::swap(P.host.p, host.p);
-    std::swap(P.host.bytes, host.bytes);
+    swap();
   }
-  ~PoolLease()
+  ~PoolLease() { swap(); }
+  void swap()
   {
     std::swap(P.dev.p, dev.p);
     std::swap(P.dev.bytes, dev.bytes);
     std::swap(P.host.p, host.p);
     std::swap(P.host.bytes, host.bytes);
+    if (wide)
+    {
+      std::swap(P.wdev.p, D.wide_pool.p);
+      std::swap(P.wdev.bytes, D.wide_pool.bytes);
+    }
   }
 };
 
@@ -1433,24 +1478,25 @@ int32_t ttg_plan_download(ttg_plan* P, void* stream, ttg_tensor* outs, double* v
     return e;
   const char* h = static_cast<const char*>(P->host.p);
   const TTInfo* T = reinterpret_cast<const TTInfo*>(h + P->off_tts);
-  for (size_t i = 0; i < P->out_tts.size(); ++i)
-  {
-    const int t = P->out_tts[i];
-    const Shape& s = P->shapes[P->kind == kPlanRound ? t : 0];
-    bool matrix = s.matrix;
-    std::vector<int> mrow = s.m, ncol = s.n;
-    if (P->kind != kPlanRound)
-    {
+  const int32_t emitted = parallel_for(
+    static_cast<int64_t>(P->out_tts.size()),
+    host_threads(sizeof(double) * static_cast<size_t>(P->arena_doubles)),
+    [&](int64_t ii) -> int32_t {
+      const size_t i = static_cast<size_t>(ii);
+      const int t = P->out_tts[i];
       // apply-round: rows from the operator, cols from the operand.
-      matrix = P->shapes[1].matrix;
-      mrow = P->shapes[0].m;
-      ncol = P->shapes[1].n;
-    }
-    if (outs)
-      if (int32_t e = emit_tensor(*P, t, matrix, mrow, ncol, &outs[i]))
-        return e;
-    fill_result(T[t], 0.0f, results ? &results[i] : nullptr);
-  }
+      const bool round = P->kind == kPlanRound;
+      const Shape& rows = P->shapes[round ? t : 0];
+      const Shape& cols = P->shapes[round ? t : 1];
+      if (outs)
+        if (int32_t e = emit_tensor(*P, t, cols.matrix, rows.m, cols.n, &outs[i],
+                                    P->out_tts.size() == 1))
+          return e;
+      fill_result(T[t], 0.0f, results ? &results[i] : nullptr);
+      return TTG_OK;
+    });
+  if (emitted)
+    return emitted;
   return first_bad_status(*P) ? fail(first_bad_status(*P), "sweep reported a device status")
                               : TTG_OK;
 }
@@ -1487,6 +1533,7 @@ struct TensorView
     t.cols = (s.matrix && !pack) ? cols.data() : nullptr;
     t.offsets = offsets.data();
     t.data = const_cast<double*>(s.data);
+    t.owned = TTG_CORES_APART;  // the source's cores may lie apart
   }
 };
 
@@ -1779,7 +1826,8 @@ static int32_t unpack_round(ttg_plan& P, const int32_t* orig, ttg_tensor* outs,
   const char* h = static_cast<const char*>(P.host.p);
   const TTInfo* T = reinterpret_cast<const TTInfo*>(h + P.off_tts);
   const int64_t n = static_cast<int64_t>(P.shapes.size());
-  return parallel_for(n, [&](int64_t ii) -> int32_t {
+  const int64_t most = host_threads(sizeof(double) * static_cast<size_t>(P.arena_doubles));
+  return parallel_for(n, most, [&](int64_t ii) -> int32_t {
     const int t = static_cast<int>(ii);
     const int i = orig ? orig[t] : t;
     const Shape& s = P.shapes[t];
@@ -1795,7 +1843,7 @@ static int32_t unpack_round(ttg_plan& P, const int32_t* orig, ttg_tensor* outs,
       }
       return TTG_OK;
     }
-    if (int32_t e = emit_tensor(P, t, s.matrix, s.m, s.n, &outs[i]))
+    if (int32_t e = emit_tensor(P, t, s.matrix, s.m, s.n, &outs[i], n == 1))
       return e;
     fill_result(T[t], ms, results ? &results[i] : nullptr);
     return TTG_OK;
@@ -1942,6 +1990,7 @@ static int32_t round_common(int32_t count, const ttg_tensor* ins, const ttg_roun
   CallTrace trace;
   ttg_plan P;
   PoolLease lease(P);
+  P.one_shot = true;
   if (int32_t st = build_round_plan(P, count, ins, opts, op))
     return st;
   trace.mark("plan+pack");
@@ -2001,6 +2050,8 @@ int32_t ttg_right_orthogonalize(const ttg_tensor* in, ttg_tensor* out)
   std::lock_guard<std::mutex> lk(dev_state().mu);
   ttg_round_options o{};
   ttg_plan P;
+  PoolLease lease(P);
+  P.one_shot = true;
   if (int32_t st = build_round_plan(P, 1, in, &o, "right_orthogonalize", kJobRightOrth))
     return st;
   if (P.shapes[0].d <= 1)
@@ -2028,6 +2079,8 @@ int32_t ttg_left_orthogonalize(const ttg_tensor* in, ttg_tensor* out)
   std::lock_guard<std::mutex> lk(dev_state().mu);
   ttg_round_options o{};
   ttg_plan P;
+  PoolLease lease(P);
+  P.one_shot = true;
   if (int32_t st = build_round_plan(P, 1, in, &o, "left_orthogonalize", kJobLeftOrth))
     return st;
   if (P.shapes[0].d <= 1)
@@ -2234,6 +2287,7 @@ static int32_t apply_round_common(const ttg_tensor* a, const ttg_tensor* x,
   std::lock_guard<std::mutex> lk(dev_state().mu);
   ttg_plan P;
   PoolLease lease(P);
+  P.one_shot = true;
   int32_t st = (mode == 2) ? build_stream_plan(P, A, X, opts)
                            : build_apply_plan(P, A, X, mode == 1, opts);
   if (st)
@@ -2658,6 +2712,7 @@ int32_t ttg_inner(const ttg_tensor* a, const ttg_tensor* b, double* out)
     return st;
   std::lock_guard<std::mutex> lk(dev_state().mu);
   ttg_plan P;
+  PoolLease lease(P);
   P.shapes = {A, B};
   add_tensor(P, A, true, nullptr);
   add_tensor(P, B, true, nullptr);
@@ -2727,6 +2782,7 @@ int32_t ttg::eval_batch_part(const ttg_tensor* a, const int32_t* idx, int32_t M,
     return st;
   std::lock_guard<std::mutex> lk(dev_state().mu);
   ttg_plan P;
+  PoolLease lease(P);
   if (int32_t st = build_eval_plan(P, a, idx, M, M_all))
     return st;
   if (M == 0)
