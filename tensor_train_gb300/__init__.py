@@ -20,6 +20,7 @@ from __future__ import annotations
 import ctypes as C
 import dataclasses
 import enum
+import math
 import os
 
 import numpy as np
@@ -222,7 +223,8 @@ _CORES_APART = 0x5ca7a  # TTG_CORES_APART
 class _In:
     """An input tensor for one call: the cores where they lie (offsets from
     the first), or copied together when one of them is not contiguous float64
-    at a multiple of 8 bytes from it."""
+    at a multiple of 8 bytes from it, or not of the size its ranks and modes
+    give (the offsets then say so to the library, which refuses it)."""
 
     def __init__(self, cores):
         cores = [np.ascontiguousarray(c, dtype=np.float64) for c in cores]
@@ -234,7 +236,10 @@ class _In:
             self.rows = np.array([c.shape[1] for c in cores], np.int32)
             self.cols = np.array([c.shape[2] for c in cores], np.int32) if self.matrix else None
             at = [c.__array_interface__["data"][0] for c in cores]
-            if all((a - at[0]) % 8 == 0 for a in at) and at[0] % 8 == 0:
+            left = [cores[0].shape[0]] + [c.shape[-1] for c in cores]
+            whole = all(c.size == r * math.prod(c.shape[1:3 if self.matrix else 2]) * q
+                        for c, r, q in zip(cores, left, left[1:]))
+            if whole and all((a - at[0]) % 8 == 0 for a in at) and at[0] % 8 == 0:
                 self.data = cores
                 self.offsets = np.array([(a - at[0]) // 8 for a in at] + [0], np.int64)
                 owned, data = _CORES_APART, at[0]
