@@ -741,6 +741,7 @@ RoundJob make_job(ttg_plan& P)
   j.max_rank = P.opts.max_rank;
   j.max_sweeps = P.opts.max_sweeps > 0 ? P.opts.max_sweeps : 40;
   j.smem_doubles = P.smem_doubles;
+  j.form_doubles = P.smem_doubles;
   j.mixed = P.opts.precision == TTG_PREC_MIXED ? 1 : 0;
   j.a_idx = reinterpret_cast<const int32_t*>(d + P.off_aidx);
   j.b_idx = reinterpret_cast<const int32_t*>(d + P.off_bidx);

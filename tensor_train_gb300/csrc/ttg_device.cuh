@@ -98,26 +98,30 @@ __device__ __forceinline__ void cta_fill(double* p, int64_t n, double v)
     p[i] = v;
 }
 
-// dst(i, j) = src(i, j) for an (m x n) block; dst column-major with ld.
-__device__ void cta_copy_to_colmajor(double* dst, int64_t ld, View src, int64_t m, int64_t n)
+// f(i, j) for i < m, j < n by groups of lanes along i (8, 16 or 32 by m):
+// neighbouring lanes get neighbouring i, and no index is divided (a 64-bit
+// division per element made the copies of a 64 x 16 step cost as much as its
+// contraction).
+template <class F>
+__device__ __forceinline__ void cta_each(int m, int n, F f)
 {
-  const int64_t total = m * n;
-  for (int64_t t = threadIdx.x; t < total; t += blockDim.x)
-  {
-    const int64_t i = t % m, j = t / m;
-    dst[i + j * ld] = src(i, j);
-  }
+  const int G = m > 16 ? 32 : (m > 8 ? 16 : 8);
+  const int gl = threadIdx.x & (G - 1);
+  for (int j = threadIdx.x / G; j < n; j += kThreads / G)
+    for (int i = gl; i < m; i += G)
+      f(i, j);
+}
+
+// dst(i, j) = src(i, j) for an (m x n) block; dst column-major with ld.
+__device__ void cta_copy_to_colmajor(double* dst, int64_t ld, View src, int m, int n)
+{
+  cta_each(m, n, [&](int i, int j) { dst[i + j * ld] = src(i, j); });
 }
 
 // dst row-major (m x n, ld) from a view.
-__device__ void cta_copy_to_rowmajor(double* dst, int64_t ld, View src, int64_t m, int64_t n)
+__device__ void cta_copy_to_rowmajor(double* dst, int64_t ld, View src, int m, int n)
 {
-  const int64_t total = m * n;
-  for (int64_t t = threadIdx.x; t < total; t += blockDim.x)
-  {
-    const int64_t i = t / n, j = t % n;
-    dst[i * ld + j] = src(i, j);
-  }
+  cta_each(n, m, [&](int j, int i) { dst[i * ld + j] = src(i, j); });
 }
 
 // Lanes per column in the column loops of the unblocked Householder
@@ -246,12 +250,9 @@ __device__ __noinline__ void cta_householder_qr(double* A, int m, int c, int64_t
 // column-major (k x c) buffer with leading dimension k.
 __device__ void cta_extract_r(double* R, const double* A, int k, int c, int64_t ld)
 {
-  const int64_t total = static_cast<int64_t>(k) * c;
-  for (int64_t t = threadIdx.x; t < total; t += blockDim.x)
-  {
-    const int i = static_cast<int>(t % k), j = static_cast<int>(t / k);
-    R[t] = (i <= j) ? A[i + j * ld] : 0.0;
-  }
+  cta_each(k, c, [&](int i, int j) {
+    R[i + static_cast<int64_t>(j) * k] = (i <= j) ? A[i + j * ld] : 0.0;
+  });
   __syncthreads();
 }
 
@@ -400,6 +401,27 @@ enum GemmTri : int
   kTriLowerB = 2,
 };
 
+// A thread's share of a 16-deep slab of both operands: loaded while the slab
+// before it is multiplied (loaded and staged in one go, each of its four
+// rounds waited for memory).
+struct GemmSlab
+{
+  static constexpr int kEach = 16 * 64 / kThreads;
+  double a[kEach], b[kEach];
+  __device__ __forceinline__ void load(const View& A, const View& B, int i0, int j0, int p0, int M,
+                                       int N, int K)
+  {
+#pragma unroll
+    for (int e = 0; e < kEach; ++e)
+    {
+      const int t = threadIdx.x + e * kThreads;
+      const int gi = i0 + t % 64, gp = p0 + t / 64, gj = j0 + t % 64;
+      a[e] = (gi < M && gp < K) ? A(gi, gp) : 0.0;
+      b[e] = (gp < K && gj < N) ? B(gp, gj) : 0.0;
+    }
+  }
+};
+
 // One 64 x 64 tile of C = A B (FP64): k slabs of 16 staged in shared
 // memory, 4 x 4 outputs per thread.  A thread multiplies only the rows and
 // columns of its block that are inside the matrix and, under tri, not in
@@ -415,17 +437,21 @@ __device__ void cta_gemm_tile(int i0, int j0, int M, int N, int K, View A, View 
     for (int b = 0; b < 4; ++b)
       acc[a][b] = 0.0;
   const int pstart = tri == kTriUpperA ? i0 : (tri == kTriLowerB ? j0 : 0);
+  GemmSlab slab;
+  slab.load(A, B, i0, j0, pstart, M, N, K);
   for (int p0 = pstart; p0 < K; p0 += 16)
   {
     __syncthreads();
-    for (int t = threadIdx.x; t < 16 * 64; t += blockDim.x)
+#pragma unroll
+    for (int e = 0; e < GemmSlab::kEach; ++e)
     {
-      const int kk = t / 64, ii = t % 64;
-      const int gi = i0 + ii, gp = p0 + kk, gj = j0 + ii;
-      sh.gemm_a[kk][ii] = (gi < M && gp < K) ? A(gi, gp) : 0.0;
-      sh.gemm_b[kk][ii] = (gp < K && gj < N) ? B(gp, gj) : 0.0;
+      const int t = threadIdx.x + e * kThreads;
+      sh.gemm_a[t / 64][t % 64] = slab.a[e];
+      sh.gemm_b[t / 64][t % 64] = slab.b[e];
     }
     __syncthreads();
+    if (p0 + 16 < K)
+      slab.load(A, B, i0, j0, p0 + 16, M, N, K);
     const int na = gemm_live(M - i0, ty, tri == kTriUpperA, p0 - i0);
     const int nb = gemm_live(N - j0, tx, tri == kTriLowerB, p0 - j0);
     const int kmax = K - p0 < 16 ? K - p0 : 16;

@@ -38,13 +38,16 @@ __device__ df64 cta_sum_df(df64 v, CtaShared& sh)
 __device__ double cta_pow2_of_max(View X, int64_t m, int64_t n, CtaShared& sh)
 {
   unsigned long long mx = 0ull;
-  const int64_t total = m * n;
-  for (int64_t t = threadIdx.x; t < total; t += blockDim.x)
-  {
+  auto take = [&](double x) {
     const unsigned long long b =
-      static_cast<unsigned long long>(__double_as_longlong(X(t % m, t / m))) & 0x7fffffffffffffffull;
+      static_cast<unsigned long long>(__double_as_longlong(x)) & 0x7fffffffffffffffull;
     mx = b > mx ? b : mx;
-  }
+  };
+  if ((X.rs == 1 && X.cs == m) || (X.cs == 1 && X.rs == n))  // one stretch of memory
+    for (int64_t t = threadIdx.x; t < m * n; t += blockDim.x)
+      take(X.p[t]);
+  else
+    cta_each(static_cast<int>(m), static_cast<int>(n), [&](int i, int j) { take(X(i, j)); });
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
   {
@@ -72,12 +75,8 @@ __device__ double cta_pow2_of_max(View X, int64_t m, int64_t n, CtaShared& sh)
 // W (df64, column-major m x n, ld) = split(X * 2^k).
 __device__ void cta_split_to_df(df64* W, int64_t ld, View X, int64_t m, int64_t n, int k)
 {
-  const int64_t total = m * n;
-  for (int64_t t = threadIdx.x; t < total; t += blockDim.x)
-  {
-    const int64_t i = t % m, j = t / m;
-    W[i + j * ld] = df_split_pow2(X(i, j), k);
-  }
+  cta_each(static_cast<int>(m), static_cast<int>(n),
+           [&](int i, int j) { W[i + j * ld] = df_split_pow2(X(i, j), k); });
 }
 
 // W[t] (FP64) = A[t] (df64) for t < n, in place when W and A alias
@@ -207,12 +206,9 @@ __device__ __noinline__ void cta_householder_qr_df(df64* A, int m, int c, int64_
 // R (k x c, column-major, FP64, ld k) = upper triangle of A, times 2^e.
 __device__ void cta_extract_r_df(double* R, const df64* A, int k, int c, int64_t ld, int e)
 {
-  const int64_t total = static_cast<int64_t>(k) * c;
-  for (int64_t t = threadIdx.x; t < total; t += blockDim.x)
-  {
-    const int i = static_cast<int>(t % k), j = static_cast<int>(t / k);
-    R[t] = (i <= j) ? df_join_pow2(A[i + j * ld], e) : 0.0;
-  }
+  cta_each(k, c, [&](int i, int j) {
+    R[i + static_cast<int64_t>(j) * k] = (i <= j) ? df_join_pow2(A[i + j * ld], e) : 0.0;
+  });
   __syncthreads();
 }
 
@@ -296,20 +292,52 @@ __device__ __noinline__ void cta_apply_q_df(const df64* A, int m, int kref, int6
   }
 }
 
+// The rotation that makes two columns orthogonal from their squared norms al,
+// be and product ga (Demmel & Veselic 1992, eq. 4.3): t, c = 1 / sqrt(1 +
+// t^2); *rel = |ga| / sqrt(al be).  False when |ga| <= tol sqrt(al be).
+template <class S>
+__device__ __forceinline__ bool jacobi_rotation(S al, S be, S ga, S tol, S* t, S* c, float* rel)
+{
+  if (ga == S(0) || fabs(ga) <= tol * sqrt(fmax(al, S(0)) * fmax(be, S(0))))
+    return false;
+  const S zeta = (be - al) / (S(2) * ga);
+  if (fabs(zeta) > S(1.0e18))
+    *t = S(0.5) / zeta;
+  else
+    *t = (zeta >= S(0) ? S(1) : S(-1)) / (fabs(zeta) + sqrt(S(1) + zeta * zeta));
+  *c = S(1) / sqrt(S(1) + *t * *t);
+  *rel = static_cast<float>(fabs(ga) / sqrt(fmax(al, S(0)) * fmax(be, S(0))));
+  return true;
+}
+
 // Element arithmetic of the one-sided Jacobi below, for FP32, FP64 and df64
-// matrices.  S is the type of the cached squared norms and the rotation
-// parameters (FP64 for df64), Acc the dot-product accumulator.
+// matrices.  S is the type of the thresholds, N of the cached squared norms,
+// Acc the dot-product accumulator.  rotation(): whether the pair is rotated,
+// and then the rotation, the new squared norms and |a_p . a_q| / (|a_p| |a_q|).
 template <class E>
 struct JOps;
 template <>
 struct JOps<float>
 {
   using S = float;
+  using N = float;
   using Acc = float;
   struct Rot
   {
     float c, s;
   };
+  static __device__ __forceinline__ bool above(N a, S floor2) { return a > floor2; }
+  static __device__ __forceinline__ bool rotation(N al, N be, Acc ga, S tol, Rot* r, N* na, N* nb,
+                                                  float* rel)
+  {
+    S t, c;
+    if (!jacobi_rotation<S>(al, be, ga, tol, &t, &c, rel))
+      return false;
+    *r = Rot{c, c * t};
+    *na = al - t * ga;
+    *nb = be + t * ga;
+    return true;
+  }
   static __device__ __forceinline__ Acc zero() { return 0.0f; }
   static __device__ __forceinline__ Acc fma(float a, float b, Acc c) { return fmaf(a, b, c); }
   static __device__ __forceinline__ Acc add(Acc a, Acc b) { return a + b; }
@@ -317,9 +345,8 @@ struct JOps<float>
   {
     return __shfl_xor_sync(0xffffffffu, v, o);
   }
-  static __device__ __forceinline__ S to_s(Acc v) { return v; }
+  static __device__ __forceinline__ N to_n(Acc v) { return v; }
   static __device__ __forceinline__ S eps() { return 4.0f * FLT_EPSILON; }
-  static __device__ __forceinline__ Rot rot(S c, S s) { return Rot{c, s}; }
   static __device__ __forceinline__ void apply(const Rot& r, float& x, float& y)
   {
     const float a = x, b = y;
@@ -331,11 +358,24 @@ template <>
 struct JOps<double>
 {
   using S = double;
+  using N = double;
   using Acc = double;
   struct Rot
   {
     double c, s;
   };
+  static __device__ __forceinline__ bool above(N a, S floor2) { return a > floor2; }
+  static __device__ __forceinline__ bool rotation(N al, N be, Acc ga, S tol, Rot* r, N* na, N* nb,
+                                                  float* rel)
+  {
+    S t, c;
+    if (!jacobi_rotation<S>(al, be, ga, tol, &t, &c, rel))
+      return false;
+    *r = Rot{c, c * t};
+    *na = al - t * ga;
+    *nb = be + t * ga;
+    return true;
+  }
   static __device__ __forceinline__ Acc zero() { return 0.0; }
   static __device__ __forceinline__ Acc fma(double a, double b, Acc c) { return ::fma(a, b, c); }
   static __device__ __forceinline__ Acc add(Acc a, Acc b) { return a + b; }
@@ -343,9 +383,8 @@ struct JOps<double>
   {
     return __shfl_xor_sync(0xffffffffu, v, o);
   }
-  static __device__ __forceinline__ S to_s(Acc v) { return v; }
+  static __device__ __forceinline__ N to_n(Acc v) { return v; }
   static __device__ __forceinline__ S eps() { return DBL_EPSILON; }
-  static __device__ __forceinline__ Rot rot(S c, S s) { return Rot{c, s}; }
   static __device__ __forceinline__ void apply(const Rot& r, double& x, double& y)
   {
     const double a = x, b = y;
@@ -353,26 +392,71 @@ struct JOps<double>
     y = r.s * a + r.c * b;
   }
 };
+// df64: nothing on the FP64 pipe (a warp's instruction holds it for 64 clocks;
+// the rotation in FP64, with its roots and divisions, was ~80 of them).  The
+// rank-96 update round: 22.7 -> 20.1 ms; 456 uneven trains: 115 -> 105 ms.  The
+// tangent is FP32's, then one Newton step on ga t^2 + (be - al) t - ga in
+// df64 (left at FP32's 1e-7 it leaves a pair of nearly equal columns short of
+// orthogonal by more than the sweeps' tolerance can see); the cosine is one
+// third-order step in df64 from the FP32 reciprocal root.
 template <>
 struct JOps<df64>
 {
   using S = double;
+  using N = df64;
   using Acc = df64;
   struct Rot
   {
     df64 c, s, ns;
   };
+  static __device__ __forceinline__ bool above(N a, S floor2)
+  {
+    return a.hi > static_cast<float>(floor2);
+  }
+  static __device__ __forceinline__ bool rotation(N al, N be, Acc ga, S tol, Rot* r, N* na, N* nb,
+                                                  float* rel)
+  {
+    const float size = sqrtf(fmaxf(al.hi, 0.0f)) * sqrtf(fmaxf(be.hi, 0.0f));
+    const float g = fabsf(ga.hi);
+    if (g == 0.0f || g <= static_cast<float>(tol) * size)
+      return false;
+    const df64 diff = df_sub(be, al);
+    const float z = diff.hi / (2.0f * ga.hi);
+    const float az = fabsf(z);
+    float t = az > 1.0e9f ? 0.5f / az : 1.0f / (az + sqrtf(fmaf(z, z, 1.0f)));
+    t = z >= 0.0f ? t : -t;
+    const float tt = t * t;
+    float te = fmaf(t, t, -tt);
+    const df64 f = df_fma(diff, df64{t, 0.0f},
+                          df_mul(ga, df_add(df64{tt, te}, df64{-1.0f, 0.0f})));
+    const float tl = -f.hi / fmaf(2.0f * ga.hi, t, diff.hi);
+    te = fmaf(2.0f * t, tl, te);  // (t + tl)^2 = tt + te
+    // e = 1 - (1 + (t + tl)^2) y^2 with y ~ c, from exact sums and products.
+    const float y = rsqrtf(1.0f + tt);
+    const float yy = y * y, ye = fmaf(y, y, -yy);
+    const float p = tt * yy, pe = fmaf(tt, yy, -p);
+    const df64 d1 = two_sum(1.0f, -yy), d = two_sum(d1.hi, -p);
+    const float lo = (d1.lo + d.lo) - ((pe + ye) + fmaf(tt, ye, te * yy));
+    // c = y (1 - e)^(-1/2) = y + y e / 2 + 3/8 y e^2, e = d.hi + lo.
+    const float e = d.hi + lo, h = 0.5f * d.hi;
+    const float yh = y * h, yhe = fmaf(y, h, -yh);
+    const df64 c1 = fast_two_sum(y, yh);
+    const df64 c = fast_two_sum(c1.hi, c1.lo + fmaf(y, fmaf(0.375f * e, e, 0.5f * lo), yhe));
+    const df64 tan = fast_two_sum(t, tl);
+    const df64 s = df_mul(c, tan);
+    *r = Rot{c, s, df_neg(s)};
+    *na = df_fma(df_neg(tan), ga, al);
+    *nb = df_fma(tan, ga, be);
+    *rel = g / size;
+    return true;
+  }
   static __device__ __forceinline__ Acc zero() { return df64{0.0f, 0.0f}; }
   static __device__ __forceinline__ Acc fma(df64 a, df64 b, Acc c) { return df_fma(a, b, c); }
   static __device__ __forceinline__ Acc add(Acc a, Acc b) { return df_add(a, b); }
   static __device__ __forceinline__ Acc shfl(Acc v, int o) { return df_shfl_xor(v, o); }
-  static __device__ __forceinline__ S to_s(Acc v) { return df_to(v); }
+  static __device__ __forceinline__ N to_n(Acc v) { return v; }
   // df64 carries 48 significand bits.
   static __device__ __forceinline__ S eps() { return 7.2e-15; }
-  static __device__ __forceinline__ Rot rot(S c, S s)
-  {
-    return Rot{df_from(c), df_from(s), df_from(-s)};
-  }
   static __device__ __forceinline__ void apply(const Rot& r, df64& x, df64& y)
   {
     const df64 a = x, b = y;
@@ -410,7 +494,7 @@ struct JOps<df64>
 // quadratically, so the next sweep's rotations would be ~stop_rel^2).
 template <class E>
 __device__ __noinline__ int cta_jacobi(E* A, int m, int n, int64_t lda, E* V, int64_t ldv, int max_sweeps,
-                          int* converged, typename JOps<E>::S* nrm, CtaShared& sh,
+                          int* converged, typename JOps<E>::N* nrm, CtaShared& sh,
                           typename JOps<E>::S floor2 = 0, typename JOps<E>::S stop_rel = 0,
                           float* maxrel_out = nullptr, int vrows = -1)
 {
@@ -460,7 +544,7 @@ __device__ __noinline__ int cta_jacobi(E* A, int m, int n, int64_t lda, E* V, in
       }
       acc = group_sum(acc);
       if (j < n && gl == 0)
-        nrm[j] = O::to_s(acc);
+        nrm[j] = O::to_n(acc);
     }
     __syncthreads();
     for (int r = 0; r < N - 1; ++r)
@@ -483,13 +567,12 @@ __device__ __noinline__ int cta_jacobi(E* A, int m, int n, int64_t lda, E* V, in
             q = tmp;
           }
         }
-        S al = 0, be = 0;
+        typename O::N al{}, be{};
         if (act)
         {
           al = nrm[p];
           be = nrm[q];
-          if (al <= floor2 || be <= floor2)
-            act = false;
+          act = O::above(al, floor2) && O::above(be, floor2);
         }
         E* ap = A + p * lda;
         E* aq = A + q * lda;
@@ -498,17 +581,11 @@ __device__ __noinline__ int cta_jacobi(E* A, int m, int n, int64_t lda, E* V, in
           for (int i = gl; i < m; i += G)
             acc = O::fma(ap[i], aq[i], acc);
         acc = group_sum(acc);
-        const S ga = O::to_s(acc);
-        if (!act || ga == S(0) || fabs(ga) <= tol * sqrt(fmax(al, S(0)) * fmax(be, S(0))))
+        typename O::Rot R;
+        typename O::N na, nb;
+        float rel;
+        if (!act || !O::rotation(al, be, acc, tol, &R, &na, &nb, &rel))
           continue;
-        const S zeta = (be - al) / (S(2) * ga);
-        S tt;
-        if (fabs(zeta) > S(1.0e18))
-          tt = S(0.5) / zeta;
-        else
-          tt = (zeta >= S(0) ? S(1) : S(-1)) / (fabs(zeta) + sqrt(S(1) + zeta * zeta));
-        const S c = S(1) / sqrt(S(1) + tt * tt);
-        const typename O::Rot R = O::rot(c, c * tt);
         for (int i = gl; i < m; i += G)
           O::apply(R, ap[i], aq[i]);
         if (V)
@@ -521,11 +598,9 @@ __device__ __noinline__ int cta_jacobi(E* A, int m, int n, int64_t lda, E* V, in
         }
         if (gl == 0)
         {
-          nrm[p] = al - tt * ga;
-          nrm[q] = be + tt * ga;
+          nrm[p] = na;
+          nrm[q] = nb;
           sh.flag = 1;
-          const float rel =
-            static_cast<float>(fabs(ga) / sqrt(fmax(al, S(0)) * fmax(be, S(0))));
           atomicMax(&sh.relbits, __float_as_uint(rel));
         }
       }
@@ -587,7 +662,16 @@ struct CertOps<double>
   static __device__ __forceinline__ double mul(double a, double b) { return a * b; }
   static __device__ __forceinline__ double neg(double a) { return -a; }
   static __device__ __forceinline__ double sub(double a, double b) { return a - b; }
-  static __device__ __forceinline__ double recip(double a) { return 1.0 / a; }
+  // One third-order step from the hardware's approximation: a rounding of the
+  // elimination like any other (the library's division is three times the
+  // instructions, on the path of every pivot).
+  static __device__ __forceinline__ double recip(double a)
+  {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
+    const double e = ::fma(-a, r, 1.0);
+    return ::fma(r, ::fma(e, e, e), r);
+  }
   static __device__ __forceinline__ bool positive(double a) { return a > 0.0; }
   static constexpr double u = 1.1102230246251565e-16;  // 2^-53
 };
@@ -872,8 +956,9 @@ __device__ __noinline__ int cta_jacobi_mixed(View src, int m, int n, double* A, 
     for (int64_t t = threadIdx.x; t < nn; t += blockDim.x)
       Vdd[t] = df_split_pow2(Vout[t], 0);
   __syncthreads();
-  const int sweeps = cta_jacobi<df64>(Ad, m, n, lda, Vdd, n, max_sweeps, converged, nrm, sh,
-                                      floor2 * isc * isc, kJacobiStopRel);
+  const int sweeps = cta_jacobi<df64>(Ad, m, n, lda, Vdd, n, max_sweeps, converged,
+                                      reinterpret_cast<df64*>(nrm), sh, floor2 * isc * isc,
+                                      kJacobiStopRel);
   for (int64_t t = threadIdx.x; t < mn; t += blockDim.x)
   {
     const int64_t e = (t % m) + (t / m) * lda;
@@ -912,8 +997,10 @@ __device__ __noinline__ void cta_gemm_df(int M, int N, int K, View A, View B, do
       for (int p0 = pstart; p0 < K; p0 += 16)
       {
         __syncthreads();
-        for (int t = threadIdx.x; t < 16 * 64; t += blockDim.x)
+#pragma unroll 2
+        for (int e = 0; e < 16 * 64 / kThreads; ++e)
         {
+          const int t = threadIdx.x + e * kThreads;
           const int kk = t / 64, ii = t % 64;
           const int gi = i0 + ii, gp = p0 + kk, gj = j0 + ii;
           as[kk][ii] = (gi < M && gp < K) ? df_split_pow2(A(gi, gp), -ea) : df64{0.0f, 0.0f};

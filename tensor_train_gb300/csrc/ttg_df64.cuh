@@ -70,17 +70,6 @@ struct df64
   float hi, lo;
 };
 
-__device__ __forceinline__ df64 df_from(double x)
-{
-  const float h = static_cast<float>(x);
-  return df64{h, static_cast<float>(x - static_cast<double>(h))};
-}
-
-__device__ __forceinline__ double df_to(df64 a)
-{
-  return static_cast<double>(a.hi) + static_cast<double>(a.lo);
-}
-
 // s + e = a + b exactly (TwoSum).
 __host__ __device__ __forceinline__ df64 two_sum(float a, float b)
 {
@@ -134,9 +123,9 @@ __host__ __device__ __forceinline__ df64 df_fma(df64 a, df64 b, df64 c)
 
 // ---------------------------------------------------------------------------
 // FP64 <-> df64 conversions with a power-of-two scale, from the IEEE bit
-// patterns on the integer and FP32 pipes.  df_from / df_to above take four
-// and three instructions of the FP64 pipe per element (conversions and an
-// add), and GB300's FP64 pipe retires 2 lanes per clock per SM against the
+// patterns on the integer and FP32 pipes.  Conversions by
+// casts would take four and three instructions of the FP64 pipe per element
+// (conversions and an add), and GB300's FP64 pipe retires 2 lanes per clock per SM against the
 // FP32 pipes' 128: in the mixed path those conversions, not the df64
 // arithmetic, would bound the step.
 // ---------------------------------------------------------------------------

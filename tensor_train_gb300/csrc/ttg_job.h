@@ -215,6 +215,7 @@ struct RoundJob
   int32_t max_rank;
   int32_t max_sweeps;
   int32_t smem_doubles;  // dynamic shared memory per CTA (doubles) for staging
+  int32_t form_doubles;  // size from which on df64 factorisations are blocked
   int32_t mixed;         // 1: FP32 Jacobi sweeps + FP64 refinement in the SVD steps
   // Streaming jobs: item i rounds the product of TT a_idx[i] (operator) and
   // b_idx[i] (operand) into output TT out_idx[i].  Row/col modes of the

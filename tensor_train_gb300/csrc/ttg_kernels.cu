@@ -16,6 +16,7 @@
 
 #include "ttg_device.cuh"
 #include "ttg_device_df.cuh"
+#include "ttg_wy.cuh"
 #include "ttg_wy_df.cuh"
 #include "ttg_job.h"
 #include "ttg_kernels.h"
@@ -50,6 +51,27 @@ __device__ void gemm_sel(bool mixed, int M, int N, int K, View A, View B, double
 // Dynamic shared memory of the CTA, used to stage the matrix a step works
 // on when it fits (cap doubles).
 
+// Where the blocked FP64 Householder routines keep their blocks' T and, for a
+// matrix in global memory, the panel they work on: in the `room` doubles of
+// shared memory at `free` (which for a matrix in shared memory start with
+// it); off when these do not fit.
+struct Wy
+{
+  bool on;
+  double* Ts;
+  double* stage;
+};
+__device__ __forceinline__ Wy wy_place(int h, int c, double* free, int64_t room)
+{
+  const int64_t hc = static_cast<int64_t>(h) * c, t = wy_t_need(h < c ? h : c);
+  if (hc + t <= room)
+    return Wy{true, free + hc, nullptr};
+  const int64_t panel = static_cast<int64_t>(h) * kWb;
+  if (hc > room && panel + t <= room)
+    return Wy{true, free + panel, free};
+  return Wy{false, nullptr, nullptr};
+}
+
 // QR of X (h x c).  Q -> *W (h x k, column-major, ld h), R -> R (k x c,
 // column-major, ld k), k = min(h, c).  The factorisation runs in shared
 // memory when h*c fits there, else in Wg; *W tells the caller where Q is.
@@ -58,10 +80,22 @@ __device__ void gemm_sel(bool mixed, int M, int N, int K, View A, View B, double
 __device__ __noinline__ int qr_factor(View X, int h, int c, double* Wg, double* tau, double* R, Smem sm,
                          double** Wout, bool mixed, CtaShared& sh, double* qdst = nullptr)
 {
-  double* W = (static_cast<int64_t>(h) * c <= sm.cap) ? sm.p : Wg;
+  const int64_t hc = static_cast<int64_t>(h) * c;
+  double* W = hc <= sm.cap ? sm.p : Wg;
   *Wout = W;
   if (mixed)
   {
+    // Blocks of kWyB reflectors for what is larger than sm.form, the panel
+    // staged behind W in shared memory, or in its place with W in global
+    // memory.
+    const int64_t need = wy_stage_need(h);
+    const bool wy = hc > sm.form && c > kWyB && need <= (sm.form < sm.cap ? sm.form : sm.cap);
+    int64_t behind = W == sm.p ? hc : 0;
+    if (wy && behind + need > sm.cap)
+    {
+      *Wout = W = Wg;
+      behind = 0;
+    }
     // df64 factorisation of X / 2^e; R scaled back exactly; Q rounded to FP64.
     df64* Wd = reinterpret_cast<df64*>(W);
     df64* td = reinterpret_cast<df64*>(tau);
@@ -69,18 +103,14 @@ __device__ __noinline__ int qr_factor(View X, int h, int c, double* Wg, double* 
     cta_split_to_df(Wd, h, X, h, c, -e);
     __syncthreads();
     const int k = h < c ? h : c;
-    // A panel in global memory is factored in blocks of kWyB reflectors
-    // with the shared region as staging (it holds nothing else here).
-    const bool wy = W != sm.p && c > kWyB && wy_stage_need(h) <= sm.cap;
-    df64* stage = reinterpret_cast<df64*>(sm.p);
-    df64* T = reinterpret_cast<df64*>(&sh.gemm_b[0][0]);
+    df64* stage = reinterpret_cast<df64*>(sm.p + behind);
     if (wy)
-      cta_householder_qr_df_wy(Wd, h, c, h, td, stage, T, sh);
+      cta_householder_qr_df_wy(Wd, h, c, h, td, stage, sh);
     else
       cta_householder_qr_df(Wd, h, c, h, td, sh);
     cta_extract_r_df(R, Wd, k, c, h, e);
     if (wy)
-      cta_form_q_df_wy(Wd, h, k, h, td, stage, T);
+      cta_form_q_df_wy(Wd, h, k, h, td, stage, sh);
     else
       cta_form_q_df(Wd, h, k, h, td);
     if (qdst)
@@ -88,10 +118,19 @@ __device__ __noinline__ int qr_factor(View X, int h, int c, double* Wg, double* 
     cta_join_from_df(qdst ? qdst : W, Wd, static_cast<int64_t>(h) * k);
     return k;
   }
+  const int k = h < c ? h : c;
+  const Wy wy = wy_place(h, c, sm.p, sm.cap);
+  if (wy.on && wy.stage)
+    *Wout = W = Wg;
   cta_copy_to_colmajor(W, h, X, h, c);
   __syncthreads();
+  if (wy.on)
+  {
+    cta_qr_wy(W, h, c, R, wy.Ts, wy.stage, sh);
+    cta_form_q_wy(W, h, k, wy.Ts, wy.stage, sh);
+    return k;
+  }
   cta_householder_qr(W, h, c, h, tau, sh);
-  const int k = h < c ? h : c;
   cta_extract_r(R, W, k, c, h);
   cta_form_q(W, h, k, h, tau);
   return k;
@@ -146,30 +185,39 @@ __device__ __noinline__ int left_svd(View X, int h, int c, double delta, int max
     // Shared-memory staging: the Jacobi matrix first (it is touched most),
     // then the Householder panel when both fit.
     const int64_t cc = static_cast<int64_t>(c) * c, hc = static_cast<int64_t>(h) * c;
+    // Mixed: blocked Householder, Q formation and Q application for what is
+    // larger than sm.form.
+    const int64_t wy_need = wy_stage_need(h);
+    const bool wy = mixed && hc + cc + c > sm.form && c > kWyB &&
+                    wy_need <= (sm.form < sm.cap ? sm.form : sm.cap);
     if (cc + c <= sm.cap)
     {
       A = sm.p;
       nrm = sm.p + cc;
-      if (hc + cc + c <= sm.cap)
+      if (hc + cc + c + (wy ? wy_need : 0) <= sm.cap)
         W = sm.p + cc + c;
     }
     const bool A_in_smem = (A == sm.p);
     df64* Wd = reinterpret_cast<df64*>(W);
     df64* td = reinterpret_cast<df64*>(tau);
     int eX = 0;  // mixed: the panel holds X / 2^eX
-    // Mixed, panel in global memory: blocked Householder, Q formation and
-    // Q application, staged in the shared region (free until the Jacobi /
+    // The blocked routines' panel lies behind the matrices in shared memory;
+    // with W in global memory in their place (free until the Jacobi /
     // certificate matrix A is written, and again once U is being formed).
-    const bool wy = mixed && W != sm.p + cc + c && c > kWyB && wy_stage_need(h) <= sm.cap;
-    df64* stage = reinterpret_cast<df64*>(sm.p);
-    df64* Twy = reinterpret_cast<df64*>(&sh.gemm_b[0][0]);
+    const int64_t wy_at = A_in_smem && W == sm.p + cc + c ? hc + cc + c : 0;
+    df64* stage = reinterpret_cast<df64*>(sm.p + wy_at);
+    // FP64: the blocked routines' T (and panel) lie behind A, which is
+    // written before they are last used.
+    const int64_t behind = A_in_smem ? cc + c : 0;
+    const Wy wy64 = mixed ? Wy{false, nullptr, nullptr}
+                          : wy_place(h, c, sm.p + behind, sm.cap - behind);
     if (mixed)
     {
       eX = pow2_exponent(cta_pow2_of_max(X, h, c, sh));
       cta_split_to_df(Wd, h, X, h, c, -eX);
       __syncthreads();
       if (wy)
-        cta_householder_qr_df_wy(Wd, h, c, h, td, stage, Twy, sh);
+        cta_householder_qr_df_wy(Wd, h, c, h, td, stage, sh);
       else
         cta_householder_qr_df(Wd, h, c, h, td, sh);
       cta_extract_r_df(R, Wd, c, c, h, eX);
@@ -178,8 +226,13 @@ __device__ __noinline__ int left_svd(View X, int h, int c, double delta, int max
     {
       cta_copy_to_colmajor(W, h, X, h, c);
       __syncthreads();
-      cta_householder_qr(W, h, c, h, tau, sh);
-      cta_extract_r(R, W, c, c, h);
+      if (wy64.on)
+        cta_qr_wy(W, h, c, R, wy64.Ts, wy64.stage, sh);
+      else
+      {
+        cta_householder_qr(W, h, c, h, tau, sh);
+        cta_extract_r(R, W, c, c, h);
+      }
     }
     const bool certified =
       certify && (mixed ? cta_certify_no_truncation_df(Wd, h, c, h, ldexp(delta, -eX),
@@ -240,11 +293,13 @@ __device__ __noinline__ int left_svd(View X, int h, int c, double delta, int max
       if (mixed)
       {
         if (wy)
-          cta_form_q_df_wy(Wd, h, c, h, td, stage, Twy);
+          cta_form_q_df_wy(Wd, h, c, h, td, stage, sh);
         else
           cta_form_q_df(Wd, h, c, h, td);
         cta_join_from_df(W, Wd, hc);
       }
+      else if (wy64.on)
+        cta_form_q_wy(W, h, c, wy64.Ts, wy64.stage, sh);
       else
         cta_form_q(W, h, c, h, tau);
       U = W;
@@ -259,7 +314,7 @@ __device__ __noinline__ int left_svd(View X, int h, int c, double delta, int max
       }
       __syncthreads();
       if (wy)
-        cta_apply_q_df_wy(Wd, h, c, h, td, Ud, r_new, h, stage, Twy);
+        cta_apply_q_df_wy(Wd, h, c, h, td, Ud, r_new, h, stage, sh);
       else
         cta_apply_q_df(Wd, h, c, h, td, Ud, r_new, h);
       cta_join_from_df(U, Ud, static_cast<int64_t>(h) * r_new);
@@ -272,7 +327,10 @@ __device__ __noinline__ int left_svd(View X, int h, int c, double delta, int max
         U[t] = i < c ? Uc[i + static_cast<int64_t>(jj) * c] : 0.0;
       }
       __syncthreads();
-      cta_apply_q(W, h, c, h, tau, U, r_new, h);
+      if (wy64.on)
+        cta_apply_q_wy(W, h, c, wy64.Ts, wy64.stage, U, r_new, h, sh);
+      else
+        cta_apply_q(W, h, c, h, tau, U, r_new, h);
     }
     if (!certified)
       record_bond(bs, sorted, c, r_new);
@@ -626,30 +684,57 @@ __device__ __noinline__ void balance(double* ar, CoreSlot* S, int d, Bump bump, 
     total += S[k].rp;
   double* cn = bump.take(2 * (total + 1));  // norms -> scl, then 1 / scl
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  double my_log = 0.0, my_cnt = 0.0;
+  // Squared column norms: lanes along a row (the contiguous direction), the
+  // rows spread over the warps, whose partial sums meet in shared memory.
+  double* part = &sh.gemm_a[0][0];  // kWarps x 32
   int64_t base = 0;
   for (int k = 0; k < d - 1; ++k)
   {
     const int h = S[k].r * S[k].n, c = S[k].rp;
     const double* p = ar + S[k].off;
-    for (int col = w; col < c; col += kWarps)
+    int cg = 1;
+    while (cg < c && cg < 32)
+      cg <<= 1;
+    const int rpw = 32 / cg;
+    for (int c0 = 0; c0 < c; c0 += cg)
     {
+      const int col = c0 + (lane & (cg - 1));
       double s = 0.0;
-      for (int i = lane; i < h; i += 32)
-        s += p[static_cast<int64_t>(i) * c + col] * p[static_cast<int64_t>(i) * c + col];
-      s = warp_sum(s);
-      const double nc = sqrt(s);
-      if (lane == 0)
-      {
-        cn[base + col] = nc;
-        if (nc > 0.0)
+      if (col < c)
+        for (int i = w * rpw + lane / cg; i < h; i += kWarps * rpw)
         {
-          my_log += log(nc);
-          my_cnt += 1.0;
+          const double x = p[static_cast<int64_t>(i) * c + col];
+          s = fma(x, x, s);
         }
+      for (int o = cg; o < 32; o <<= 1)
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane < cg)
+        part[w * 32 + lane] = s;
+      __syncthreads();
+      if (threadIdx.x < cg && col < c)
+      {
+        double t = part[threadIdx.x];
+#pragma unroll
+        for (int q = 1; q < kWarps; ++q)
+          t += part[q * 32 + threadIdx.x];
+        cn[base + col] = t;
       }
+      __syncthreads();
     }
     base += c;
+  }
+  // A thread per column from here: a root and a logarithm are ~80 FP64
+  // instructions each, which a warp per column took one column at a time.
+  double my_log = 0.0, my_cnt = 0.0;
+  for (int64_t t = threadIdx.x; t < total; t += blockDim.x)
+  {
+    const double nc = sqrt(cn[t]);
+    cn[t] = nc;
+    if (nc > 0.0)
+    {
+      my_log += log(nc);
+      my_cnt += 1.0;
+    }
   }
   const double tot_log = cta_sum(my_log, sh);
   const double tot_cnt = cta_sum(my_cnt, sh);
@@ -1480,7 +1565,7 @@ __global__ void __launch_bounds__(kThreads, MinBlocks) round_kernel(RoundJob job
 {
   __shared__ CtaShared sh;
   extern __shared__ double dyn_smem[];
-  const Smem sm{dyn_smem, job.smem_doubles};
+  const Smem sm{dyn_smem, job.smem_doubles, job.form_doubles};
   double* scratch = job.scratch + static_cast<int64_t>(blockIdx.x) * job.scratch_stride;
   for (;;)
   {

@@ -27,7 +27,7 @@ __device__ __forceinline__ void reflector_scalars(double s, double ax, double* n
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(ax + t));
   const double e = fma(-t, y, 1.0);  // n = t (1 - e)^(-1/2), rs = y (1 - e)^(-1/2)
   const double q = e * fma(0.375, e, 0.5);
-  *n = fma(t, q, t);
+  *n = t + fma(t, q, fma(s, y, -t));
   *rs = fma(y, q, y);
   const double f = fma(-*n, r, fma(-ax, r, 1.0));  // 1 / (ax + n) = r (1 + f + f^2 + ...)
   *inv = fma(r, fma(f, f, f), r);

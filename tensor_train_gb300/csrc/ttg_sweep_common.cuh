@@ -43,6 +43,10 @@ struct Smem
 {
   double* p;
   int64_t cap;
+  // Matrices of more doubles than this are factored in blocks in df64 when
+  // a panel's staging fits in as many.  Fixed by the batch's size, while cap
+  // follows the CTAs per SM: the two forms round differently.
+  int64_t form;
 };
 
 __device__ void record_bond(BondStat* bs, const double* sorted, int nsv, int r_new)

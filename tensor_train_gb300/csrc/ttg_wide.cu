@@ -357,7 +357,8 @@ __device__ bool wide_jacobi(const WideJob& job, E* A, int p, int q, int64_t lda,
   const int NB = nblk + (nblk & 1), npairs = NB / 2;
   E* As = reinterpret_cast<E*>(sm.p);
   E* Vs = As + static_cast<int64_t>(p) * 2 * b;
-  S* ns = reinterpret_cast<S*>(Vs + (V ? static_cast<int64_t>(q) * 2 * b : 0));
+  using N = typename JOps<E>::N;
+  N* ns = reinterpret_cast<N*>(Vs + (V ? static_cast<int64_t>(q) * 2 * b : 0));
   if (me == 0)
     for (int s = threadIdx.x; s < max_sweeps; s += blockDim.x)
     {

@@ -146,14 +146,20 @@ struct PanelShared
 // lanes of a warp.
 __device__ __forceinline__ void panel_t_column(PanelShared& ps, int i)
 {
-  const int l = threadIdx.x & 31;
+  // Two lanes per row, each half of the sum.
+  const int lane = threadIdx.x & 31, l = lane & (kPb - 1), half = lane / kPb;
   const double nt = -ps.tau[i];
+  const double g = nt * ps.G[l + i * kPb];  // lane q's term is -tau_i G(q, i)
   double acc = 0.0;
-  if (l < i)
-    for (int q = l; q < i; ++q)
-      acc = fma(ps.T[l + q * kPb], nt * ps.G[q + i * kPb], acc);
-  __syncwarp();
-  if (l < kPb)
+  for (int q0 = 0; q0 < i; q0 += 2)  // the same trips on every lane
+  {
+    const int q = q0 + half;
+    const double gq = __shfl_sync(0xffffffffu, g, q);
+    if (l <= q && q < i)
+      acc = fma(ps.T[l + q * kPb], gq, acc);
+  }
+  acc += __shfl_xor_sync(0xffffffffu, acc, kPb);
+  if (half == 0)
     ps.T[l + i * kPb] = l < i ? acc : (l == i ? -nt : 0.0);
   __syncwarp();
 }
