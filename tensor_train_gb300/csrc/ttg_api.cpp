@@ -278,7 +278,9 @@ struct ttg_plan
   int grid = 1;
   int cps = 2;          // resident CTAs per SM of the sweep kernel instantiation
   int scratch_ctas = 1; // CTAs the scratch slabs were allocated for
+  int64_t items_hint = 0;  // TTs of the whole call that this plan is a part of
   int smem_doubles = 0;
+  int form_doubles = 0;  // df64 factorisations of larger matrices are blocked
   // products computed on the device before the sweep (naive apply-round):
   struct Apply
   {
@@ -624,6 +626,39 @@ int32_t setup_wide(ttg_plan& P)
   return TTG_OK;
 }
 
+// CTAs per SM of the per-TT sweep.  One alone keeps a step's matrices in its
+// 200 KB of shared memory and is through a TT soonest; several hide each
+// other's waits.  So few TTs per SM, or large ones, run one or two at a time
+// (the last ones' latency decides), many small ones three or four.  Measured
+// on uneven batches of 200 to 3500 TTs (ranks to 96, mean core 12k doubles,
+// and to 40, 2.3k; ms with 1 / 2 CTAs per SM against 3 mixed, 4 FP64): FP64 to
+// rank 96, 500 TTs 54 / - / 131, 2000 TTs 176 / - / 206, 3500 TTs 4 best; FP64
+// to 40, 700 TTs - / 17 / 30, 1500 TTs 4 best; mixed to 96, 500 TTs 52 / - /
+// 71, 1000 TTs - / 62 / 76, 3500 TTs 3 best; mixed to 40, 330 TTs 11 / 13 / -,
+// 700 TTs - / 14 / 18, 1500 TTs 3 best.
+int sweep_ctas_per_sm(const ttg_plan& P, int64_t items, int sms)
+{
+  if (items <= sms || P.job_kind < 0)
+    return 1;
+  double size = 0.0, cores = 0.0;
+  for (int32_t t : P.order)
+    if (t >= 0 && t < static_cast<int32_t>(P.tts.size()))
+      for (int k = 0; k < P.tts[t].d; ++k)
+      {
+        const CoreSlot& c = P.slots[P.tts[t].first + k];
+        size += static_cast<double>(c.r) * c.n * c.rp;
+        cores += 1.0;
+      }
+  const bool large = size > 6000.0 * std::max(cores, 1.0);
+  const bool mixed = P.opts.precision == TTG_PREC_MIXED;
+  const double per_sm = static_cast<double>(items) / sms;
+  if (per_sm <= (mixed ? (large ? 4.0 : 3.0) : (large ? 16.0 : 4.0)))
+    return 1;
+  if (per_sm <= (mixed && large ? 16.0 : 8.0))
+    return 2;
+  return mixed ? 3 : 4;
+}
+
 int32_t layout_and_alloc(ttg_plan& P)
 {
   static const cudaError_t optin = round_smem_optin(kSmemOnePerSm);
@@ -631,27 +666,22 @@ int32_t layout_and_alloc(ttg_plan& P)
     return fail(TTG_ERR_CUDA, std::string("round kernel shared-memory opt-in: ") +
                                   cudaGetErrorString(optin));
   const int sms = std::max(device().sms, 1);
-  P.smem_doubles = P.grid > sms ? kSmemTwoPerSm : kSmemOnePerSm;
-  P.cps = P.grid > sms ? 2 : 1;
-  // Large batches get scratch for up to 4 CTAs per SM (autotuner candidates).
-  // FP64 sweeps start at 4 per SM (DFMA-bound: more resident TTs keep the
-  // pipe fed); mixed sweeps at 3, whose 56 KB of shared staging still holds
-  // the blocked df64 Householder panels -- the autotuner's picks on the
-  // uneven 4096-TT batch.
+  const int64_t items = static_cast<int64_t>(P.order.size());
+  P.cps = sweep_ctas_per_sm(P, std::max(items, P.items_hint), sms);
+  P.grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(items, int64_t{P.cps} * sms)));
+  constexpr int kSmem[5] = {0, kSmemOnePerSm, kSmemTwoPerSm, kSmemThreePerSm, kSmemFourPerSm};
+  P.smem_doubles = kSmem[P.cps];
+  // Which form a df64 factorisation takes depends on its size and the batch's
+  // alone, not on the CTAs per SM (which are a matter of speed, and tuned):
+  // the forms round differently, and a mixed batch of hundreds of TTs has
+  // singular values close enough together (1e-7) to show it.
+  P.form_doubles = kSmem[items <= sms ? 1 : (items >= 3LL * sms && P.job_kind >= 0 ? 3 : 2)];
+  // Scratch for every launch the autotuner may try: up to 2 CTAs per SM, 4 for
+  // larger batches.
   P.scratch_ctas = P.grid;
-  if (static_cast<int64_t>(P.order.size()) > 2LL * sms && P.job_kind >= 0)
-  {
-    P.scratch_ctas = static_cast<int>(std::min<int64_t>(static_cast<int64_t>(P.order.size()),
-                                                        4LL * sms));
-    const bool mixed = P.opts.precision == TTG_PREC_MIXED;
-    const int cps = mixed ? 3 : 4;
-    if (static_cast<int64_t>(P.order.size()) >= static_cast<int64_t>(cps) * sms)
-    {
-      P.grid = cps * sms;
-      P.cps = cps;
-      P.smem_doubles = mixed ? kSmemThreePerSm : kSmemFourPerSm;
-    }
-  }
+  if (P.job_kind >= 0)
+    P.scratch_ctas = std::max(
+      P.grid, static_cast<int>(std::min<int64_t>(items, (items > 2LL * sms ? 4LL : 2LL) * sms)));
   size_t o = 0;
   P.off_arena = o;
   o = align256(o + sizeof(double) * static_cast<size_t>(P.arena_doubles));
@@ -741,7 +771,7 @@ RoundJob make_job(ttg_plan& P)
   j.max_rank = P.opts.max_rank;
   j.max_sweeps = P.opts.max_sweeps > 0 ? P.opts.max_sweeps : 40;
   j.smem_doubles = P.smem_doubles;
-  j.form_doubles = P.smem_doubles;
+  j.form_doubles = P.form_doubles;
   j.mixed = P.opts.precision == TTG_PREC_MIXED ? 1 : 0;
   j.a_idx = reinterpret_cast<const int32_t*>(d + P.off_aidx);
   j.b_idx = reinterpret_cast<const int32_t*>(d + P.off_bidx);
@@ -774,12 +804,6 @@ int32_t check_opts(const ttg_round_options* o, const char* op)
   if (o->method < 0 || o->method > TTG_METHOD_SKETCH)
     return fail(TTG_ERR_METHOD, std::string(op) + ": unknown method " + std::to_string(o->method));
   return TTG_OK;
-}
-
-int finish_grid(int64_t items)
-{
-  const int sms = std::max(device().sms, 1);
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(items, 2LL * sms)));
 }
 
 // job_kind >= 0 replaces the sweep the options select (right_orthogonalize,
@@ -852,7 +876,6 @@ int32_t build_round_plan(ttg_plan& P, int32_t count, const ttg_tensor* ins,
   for (auto& c : cost)
     P.order.push_back(c.second);
   P.scratch_stride = need;
-  P.grid = finish_grid(static_cast<int64_t>(P.order.size()));
   return layout_and_alloc(P);
 }
 
@@ -1898,6 +1921,7 @@ static int32_t round_batch_pipelined(int32_t count, const ttg_tensor* ins,
   auto launch = [&](int c) -> int32_t {
     Chunk& k = *ch[c];
     k.lease = std::make_unique<PoolLease>(k.P, c & 1);
+    k.P.items_hint = count;
     if (int32_t e = build_round_plan(k.P, static_cast<int32_t>(k.in.size()), k.in.data(), opts, op))
       return e;
     trace.mark("pack");
