@@ -529,10 +529,16 @@ int32_t setup_wide(ttg_plan& P)
   };
   const size_t cc = sizeof(double) * static_cast<size_t>(c_max * c_max);
   const size_t cm = sizeof(double) * static_cast<size_t>(core_max);
+  const size_t twb =
+    8 * kWidePb * kWidePb * static_cast<size_t>((c_max + kWidePb - 1) / kWidePb);
+  // A second set of reflectors, for the Q that is formed during the next QR,
+  // where the blocked QR (whose tiles lie in shared memory) can take every
+  // core: 31 MB at most.
+  const bool later = want_whole && core_max <= int64_t{grid} * smem;
   const size_t oW = take(cm), oU = take(cm), oP = take(cm), oA = take(cm), oR = take(cc),
                oV = take(cc), oF = take(cc), oT1 = take(cc), oT2 = take(cc),
                opart = take(16 * static_cast<size_t>(grid) + 16), oumax = take(8),
-               oTw = take(8 * kWidePb * kWidePb * static_cast<size_t>((c_max + kWidePb - 1) / kWidePb)),
+               oTw = take(twb), oW2 = take(later ? cm : 8), oTw2 = take(later ? twb : 8),
                otau = take(8 * c_max), osig = take(8 * c_max),
                osorted = take(8 * c_max), oord = take(4 * c_max), ocn = take(8 * (cols_max + 1)),
                oival = take(64), orot = take(4 * ms), orel = take(4 * ms),
@@ -541,7 +547,7 @@ int32_t setup_wide(ttg_plan& P)
                oFs = take(stream ? 8 * static_cast<size_t>(f_max) : 8);
   // The exchange packets come last, so that one strided fill zeroes every
   // team's.
-  const size_t opk = take(sizeof(uint4) * static_cast<size_t>(wide_packets(c_max)));
+  const size_t opk = take(sizeof(uint4) * static_cast<size_t>(wide_packets(c_max, later)));
   // One such block per team, then the teams' barrier words.
   const size_t team_bytes = o;
   const size_t obar = team_bytes * static_cast<size_t>(teams_max);
@@ -572,6 +578,8 @@ int32_t setup_wide(ttg_plan& P)
   j.T2 = reinterpret_cast<double*>(b + oT2);
   j.part = reinterpret_cast<double*>(b + opart);
   j.Tw = reinterpret_cast<double*>(b + oTw);
+  j.W2 = later ? reinterpret_cast<double*>(b + oW2) : nullptr;
+  j.Tw2 = reinterpret_cast<double*>(b + oTw2);
   j.packets = reinterpret_cast<uint4*>(b + opk);
   j.c_max = c_max;
   j.umax = reinterpret_cast<unsigned long long*>(b + oumax);
@@ -949,8 +957,9 @@ int32_t plan_run(ttg_plan& P, cudaStream_t st)
     if (P.wide)
     {
       TTG_CUDA(cudaMemsetAsync(P.wjob.bar, 0, sizeof(GridBar) * P.wide_teams, st));
+      const int64_t packets = wide_packets(P.wjob.c_max, P.wjob.W2 != nullptr);
       TTG_CUDA(cudaMemset2DAsync(P.wjob.packets, static_cast<size_t>(P.wjob.team_bytes), 0,
-                                 sizeof(uint4) * static_cast<size_t>(wide_packets(P.wjob.c_max)),
+                                 sizeof(uint4) * static_cast<size_t>(packets),
                                  static_cast<size_t>(P.wide_teams), st));
       WideJob j = P.wjob;
       j.teams = P.wide_teams;

@@ -123,9 +123,9 @@ __host__ __device__ __forceinline__ df64 df_fma(df64 a, df64 b, df64 c)
 
 // ---------------------------------------------------------------------------
 // FP64 <-> df64 conversions with a power-of-two scale, from the IEEE bit
-// patterns on the integer and FP32 pipes.  Conversions by
-// casts would take four and three instructions of the FP64 pipe per element
-// (conversions and an add), and GB300's FP64 pipe retires 2 lanes per clock per SM against the
+// patterns on the integer and FP32 pipes.  Casts would take four
+// and three instructions of the FP64 pipe per element (conversions and an
+// add), and GB300's FP64 pipe retires 2 lanes per clock per SM against the
 // FP32 pipes' 128: in the mixed path those conversions, not the df64
 // arithmetic, would bound the step.
 // ---------------------------------------------------------------------------

@@ -140,9 +140,11 @@ struct GridBar
 constexpr int kWidePb = 16;
 constexpr int kWidePanelSlabs = 32;
 constexpr int kWideTrailSlabs = 16;
-inline int64_t wide_packets(int64_t c_max)
+inline int64_t wide_packets(int64_t c_max, bool later)
 {
-  return 2 * (kWidePanelSlabs + 1) * kWidePb + 2 * kWideTrailSlabs * c_max * kWidePb;
+  // panel products; a block's products; those of the Q formed meanwhile
+  return 2 * (kWidePanelSlabs + 1) * kWidePb +
+         (later ? 4 : 2) * kWideTrailSlabs * c_max * kWidePb;
 }
 
 // Whole-GPU rounding of a few large TTs (wide_round_kernel): the arena,
@@ -175,6 +177,7 @@ struct WideJob
   int64_t smem_doubles;
   double eps;
   double* W;           // core_max: reflectors
+  double* W2;          // core_max: the other QR's, while its Q is formed; or null
   double* Ub;          // core_max: U / work columns
   double* Pb;          // core_max: contraction output
   double* A;           // core_max: Jacobi matrix
@@ -191,6 +194,7 @@ struct WideJob
   int* ival;           // [0] = truncation rank of the current bond
   double* part;        // two partial sums per CTA
   double* Tw;          // kWidePb^2 per block of reflectors
+  double* Tw2;         // the other QR's
   uint4* packets;      // wide_packets(c_max): zeroed before each launch
   int64_t c_max;
   unsigned long long* umax;  // grid-wide max of |x| bit patterns

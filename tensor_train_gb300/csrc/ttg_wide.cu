@@ -62,9 +62,25 @@ struct WideSmem
   double* p;
   int64_t cap;  // doubles
   OzState* oz;  // TMEM accumulator and MMA barrier of this CTA (null: FP64 tiles only)
-  uint32_t* seq;  // next exchange tag, the same on every thread of the team
-  bool* blocked;  // whether W holds the last QR in the blocked form
+  // Per thread, the same on every thread of the team:
+  uint32_t* seq;    // next exchange tag
+  uint32_t* q_seq;  // next tag of the Q formed meanwhile
+  bool* blocked;    // whether W holds the last QR in the blocked form
+  WideQ* later;     // the Q that the next QR's idle CTAs form
+  WideJob* team;    // the team's job, for the exchange of its work buffers
 };
+
+// Doubles at the end of the shared memory that a Q formed meanwhile holds,
+// and the CTAs from which on it is formed (those below work on the panels).
+constexpr int64_t kLaterCap = 14336;
+constexpr int kLaterFrom = kWidePanelSlabs;
+
+
+// Brings a Q put off to its end.
+__device__ bool wide_q_now(const WideJob& job, WideSmem sm)
+{
+  return !sm.later->on || (wide_q_end(job, *sm.later) && grid_sync(job));
+}
 
 // dst[0..n) = src[0..n), spread over the grid.
 __device__ void wide_copy(const WideJob& job, double* dst, const double* src, int64_t n)
@@ -246,9 +262,36 @@ __device__ int wide_qr(const WideJob& job, View X, int h, int c, WideSmem sm, Ct
                        bool* ok)
 {
   const int P = job.size, me = job.rank;
-  *sm.blocked = wide_blocked_fits(h, c, P, sm.cap);
+  WideQ& later = *sm.later;
+  // The Q put off keeps its tile and the last QR's reflectors until the end
+  // of this QR, if this one's tiles fit beside it.
+  int64_t cap = sm.cap - (later.on ? kLaterCap : 0);
+  if (later.on && !wide_blocked_fits(h, c, P, cap))
+  {
+    if (!wide_q_now(job, sm))
+    {
+      *ok = false;
+      return 0;
+    }
+    cap = sm.cap;
+  }
+  *sm.blocked = wide_blocked_fits(h, c, P, cap);
   if (!*sm.blocked)
     return wide_qr_columns(job, X, h, c, sm, sh, ok);
+  if (later.on)
+  {
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+      double* t = sm.team->W;
+      sm.team->W = sm.team->W2;
+      sm.team->W2 = t;
+      t = sm.team->Tw;
+      sm.team->Tw = sm.team->Tw2;
+      sm.team->Tw2 = t;
+    }
+    __syncthreads();
+  }
   const int k = h < c ? h : c;
   const int64_t stride = static_cast<int64_t>(P) * blockDim.x;
   const int64_t first = me * static_cast<int64_t>(blockDim.x) + threadIdx.x;
@@ -274,15 +317,25 @@ __device__ int wide_qr(const WideJob& job, View X, int h, int c, WideSmem sm, Ct
         const int64_t l = j0 + e / j0;
         job.R[i + l * k] = job.W[l * h + i];
       }
+    // Meanwhile, the blocks of the Q put off: as many per panel as leave none
+    // at the last one.
+    if (later.on)
+    {
+      const int panels = (k - j0 + kPb - 1) / kPb;
+      for (int n = (later.next + panels) / panels; n > 0 && *ok; --n)
+        *ok = wide_q_block(job, later);
+    }
     seq += kPb;
     *ok = grid_sync(job) && *ok;
     if (*ok && j0 + nb < c)
     {
-      *ok = wide_trail(job, h, c, j0, nb, seq, sm.p, sm.cap);
+      *ok = wide_trail(job, h, c, j0, nb, seq, sm.p, cap);
       *ok = grid_sync(job) && *ok;
     }
     seq += 1;
   }
+  if (*ok && later.on)
+    *ok = wide_q_end(job, later);
   if (*ok && c > k)
   {
     for (int64_t e = first; e < static_cast<int64_t>(k) * (c - k); e += stride)
@@ -298,16 +351,55 @@ __device__ int wide_qr(const WideJob& job, View X, int h, int c, WideSmem sm, Ct
 // out(i, l) = out[i*o_rs + l*o_cs] = (H_0 ... H_{kref-1} [B; 0])(i, l) for
 // l < ncols; B column-major (nb x ncols, ld nb), nb <= h, or the identity
 // (eye).  Column by column when the QR was (column l on CTA l mod P; y is a
-// length-h work column).  Returns false on a failed wait.
+// length-h work column).  put_off: out may be written as late as the end of
+// the next wide_qr or wide_q_now, which has to follow.  Returns false on a failed wait.
 __device__ bool wide_apply_q(const WideJob& job, int h, int kref, const double* B, int nb,
                              int ncols, double* out, int64_t o_rs, int64_t o_cs, bool eye,
-                             WideSmem sm, CtaShared& sh)
+                             WideSmem sm, CtaShared& sh, bool put_off = false)
 {
   if (*sm.blocked)
   {
-    const uint32_t seq = *sm.seq;
+    WideQ q{};
+    q.W = job.W;
+    q.Tw = job.Tw;
+    q.B = B;
+    q.out = out;
+    q.o_rs = o_rs;
+    q.o_cs = o_cs;
+    q.h = h;
+    q.kref = kref;
+    q.nb_rows = nb;
+    q.ncols = ncols;
+    q.eye = eye;
+    // Q itself (the identity's) is not needed before the next QR is through,
+    // whose panels leave all but 32 CTAs idle: with as many more to spare they
+    // form it meanwhile, a block or two per panel.  d=40 rank 257: 155 -> 141
+    // ms; matvec d=20 rank 256: 49.9 -> 44.5; streaming: 11.0 -> 10.65; right-
+    // canonical d=15 rank 83: 9.4 -> 8.8.
+    const int64_t spare = job.size - kLaterFrom;
+    if (put_off && eye && job.W2 && spare >= kLaterFrom &&
+        trail_cut(h, ncols, static_cast<int>(spare), kLaterCap, 2).St > 0)
+    {
+      q.rank = job.rank - kLaterFrom < 0 ? -1 : job.rank - kLaterFrom;
+      q.size = static_cast<int>(spare);
+      q.region = 1;
+      q.seq = *sm.q_seq;
+      *sm.q_seq += static_cast<uint32_t>((kref + kPb - 1) / kPb);
+      q.sm = sm.p + sm.cap - kLaterCap;
+      q.cap = kLaterCap;
+      *sm.later = q;
+      wide_q_begin(*sm.later);
+      return true;
+    }
+    q.rank = job.rank;
+    q.size = job.size;
+    q.region = 0;
+    q.seq = *sm.seq;
     *sm.seq += static_cast<uint32_t>((kref + kPb - 1) / kPb);
-    return wide_q(job, h, kref, B, nb, ncols, out, o_rs, o_cs, eye, seq, sm.p, sm.cap);
+    q.sm = sm.p;
+    q.cap = sm.cap;
+    wide_q_begin(q);
+    return wide_q_end(job, q);
   }
   const int P = job.size, me = job.rank;
   for (int l = me; l < ncols; l += P)
@@ -726,7 +818,7 @@ __device__ bool wide_right_orth(const WideJob& job, CoreSlot* S, int d, WideSmem
       return false;
     // core_k <- Q^T (Q column-major w x kk is the core's row-major layout);
     // prev (hp x kk) = left_unfold(prev) R^T.
-    if (!wide_apply_q(job, w, kk, nullptr, 0, kk, cs, 1, w, true, sm, sh))
+    if (!wide_apply_q(job, w, kk, nullptr, 0, kk, cs, 1, w, true, sm, sh, k > 1))
       return false;
     if (!wide_gemm(job, hp, kk, r, View{ps, r, 1}, View{job.R, kk, 1}, job.Pb, kk, 1, sm, sh, false,
                    kTriLowerB))
@@ -880,17 +972,29 @@ __device__ __noinline__ bool wide_certify(const WideJob& job, int c, int h, doub
   return true;
 }
 
+// Where a step's U (h x r_new) goes when all singular values are kept: to
+// out(i, j) = out[i rs + j cs] (rs = 0: r_new, cs = 0: h), and with `later`
+// as late as the next wide_left_svd, which has to follow.
+struct WideU
+{
+  double* out;
+  int64_t rs, cs;
+  bool later;
+  bool done = false;     // U went there; else it is in job.Ub (column-major)
+  bool f_upper = false;  // F is the upper triangular R
+};
+
 // Truncated SVD of X (h x c) over the grid, as left_svd of the per-TT
 // kernel (detail/truncate.hpp:61-99 branches): *r_new_out, U in job.Ub
-// (column-major, h x r_new), diag(s) V^T rows in job.F (row-major, r_new x
-// c); *f_upper: F is the upper triangular R.  X must not alias the work buffers (A, W, R, V, F, Ub, Pb, T1, T2).
+// (column-major, h x r_new) or u.out (which may be X's storage), diag(s) V^T
+// rows in job.F (row-major, r_new x c).  X must not alias the work buffers
+// (A, W, R, V, F, Ub, Pb, T1, T2).
 __device__ bool wide_left_svd(const WideJob& job, View X, int h, int c, double delta, TTInfo& T,
                               BondStat* bs, WideSmem sm, CtaShared& sh, int* r_new_out,
-                              bool* f_upper = nullptr)
+                              WideU& u)
 {
   const int me = job.rank;
-  if (f_upper)
-    *f_upper = false;
+  u.done = u.f_upper = false;
   const bool lead = (me == 0 && threadIdx.x == 0);
   const int nsv = h < c ? h : c;
   const double floor2 = 1e-6 * delta * delta / static_cast<double>(nsv > 1 ? nsv : 1);
@@ -916,13 +1020,13 @@ __device__ bool wide_left_svd(const WideJob& job, View X, int h, int c, double d
     {
       // Every singular value is kept: U = Q, F = R.
       r_new = c;
-      if (f_upper)
-        *f_upper = true;
+      u.f_upper = u.done = true;
       const int64_t cc = static_cast<int64_t>(c) * c;
       for (int64_t e = job.rank * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < cc;
            e += static_cast<int64_t>(job.size) * blockDim.x)
         job.F[(e % c) * c + e / c] = job.R[e];
-      if (!wide_apply_q(job, h, c, nullptr, 0, c, job.Ub, 1, h, true, sm, sh))
+      if (!wide_apply_q(job, h, c, nullptr, 0, c, u.out, u.rs ? u.rs : c, u.cs ? u.cs : h, true, sm,
+                        sh, u.later))
         return false;
       WSYNC();
     }
@@ -960,6 +1064,8 @@ __device__ bool wide_left_svd(const WideJob& job, View X, int h, int c, double d
       WSYNC();
     }
   }
+  else if (!wide_q_now(job, sm))
+    return false;
   else if (h >= c)
   {
     for (int64_t e = job.rank * static_cast<int64_t>(blockDim.x) + threadIdx.x;
@@ -1087,15 +1193,16 @@ __device__ bool wide_round_tt(const WideJob& job, int tti, WideSmem sm, CtaShare
     double* ns = ar + S[k + 1].off;
     BondStat* bs = job.bond_stats ? job.bond_stats + T.first + k : nullptr;
     int r_new = 1;
-    bool upper = false;
-    if (!wide_left_svd(job, View{cs, c, 1}, h, c, delta, T, bs, sm, sh, &r_new, &upper))
+    WideU u{cs, 0, 1, k < d - 2};
+    if (!wide_left_svd(job, View{cs, c, 1}, h, c, delta, T, bs, sm, sh, &r_new, u))
       return false;
     // next (r_new x wn) = F right_unfold(next); core_k <- U (row-major).
     if (!wide_gemm(job, r_new, wn, c, View{job.F, c, 1}, View{ns, wn, 1}, job.Pb, wn, 1, sm, sh, false,
-                   upper ? kTriUpperA : kTriNone))
+                   u.f_upper ? kTriUpperA : kTriNone))
       return false;
     WSYNC();
     wide_copy(job, ns, job.Pb, static_cast<int64_t>(r_new) * wn);
+    if (!u.done)
     {
       const int64_t stride = static_cast<int64_t>(job.size) * blockDim.x;
       for (int64_t e = job.rank * static_cast<int64_t>(blockDim.x) + threadIdx.x;
@@ -1146,7 +1253,7 @@ __device__ bool wide_round_right_tt(const WideJob& job, int tti, WideSmem sm, Ct
       return false;
     // core_k <- Q (h x kk, row-major); next (kk x wn) = R right_unfold(next),
     // R (kk x rp) column-major in job.R.
-    if (!wide_apply_q(job, h, kk, nullptr, 0, kk, cs, kk, 1, true, sm, sh))
+    if (!wide_apply_q(job, h, kk, nullptr, 0, kk, cs, kk, 1, true, sm, sh, k < d - 2))
       return false;
     if (!wide_gemm(job, kk, wn, rp, View{job.R, 1, kk}, View{ns, wn, 1}, job.Pb, wn, 1, sm, sh, false,
                    kTriUpperA))
@@ -1173,17 +1280,18 @@ __device__ bool wide_round_right_tt(const WideJob& job, int tti, WideSmem sm, Ct
     double* cs = ar + S[k].off;
     double* ps = ar + S[k - 1].off;
     int r_new = 1;
-    bool upper = false;
-    if (!wide_left_svd(job, View{cs, 1, w}, w, r, delta, T, nullptr, sm, sh, &r_new, &upper))
+    WideU u{cs, 1, 0, k > 1};
+    if (!wide_left_svd(job, View{cs, 1, w}, w, r, delta, T, nullptr, sm, sh, &r_new, u))
       return false;
     // prev (hp x r_new) = left_unfold(prev) F^T, F (r_new x r) row-major in
     // job.F; core_k <- U^T, whose row-major layout is U's column-major one.
     if (!wide_gemm(job, hp, r_new, r, View{ps, r, 1}, View{job.F, 1, r}, job.Pb, r_new, 1, sm, sh,
-                   false, upper ? kTriLowerB : kTriNone))
+                   false, u.f_upper ? kTriLowerB : kTriNone))
       return false;
     WSYNC();
     wide_copy(job, ps, job.Pb, static_cast<int64_t>(hp) * r_new);
-    wide_copy(job, cs, job.Ub, static_cast<int64_t>(w) * r_new);
+    if (!u.done)
+      wide_copy(job, cs, job.Ub, static_cast<int64_t>(w) * r_new);
     if (lead)
     {
       set_ranks(S[k], r_new, rp);
@@ -1297,14 +1405,16 @@ __device__ bool wide_stream_tt(const WideJob& job, int item, WideSmem sm, CtaSha
       break;
     }
     int r_new = 1;
-    if (!wide_left_svd(job, View{Cj, ccols, 1}, hrows, ccols, delta, TO, nullptr, sm, sh, &r_new))
+    WideU u{os, 0, 1, k < d - 2};
+    if (!wide_left_svd(job, View{Cj, ccols, 1}, hrows, ccols, delta, TO, nullptr, sm, sh, &r_new, u))
       return false;
     // core_k <- U (row-major hrows x r_new); F <- diag(s) V^T.
-    WIDE_FOR(e, static_cast<int64_t>(hrows) * r_new)
-    {
-      const int64_t i = e / r_new, j = e % r_new;
-      os[e] = job.Ub[i + j * hrows];
-    }
+    if (!u.done)
+      WIDE_FOR(e, static_cast<int64_t>(hrows) * r_new)
+      {
+        const int64_t i = e / r_new, j = e % r_new;
+        os[e] = job.Ub[i + j * hrows];
+      }
     wide_copy(job, job.Fs, job.F, static_cast<int64_t>(r_new) * ccols);
     if (lead)
       set_ranks(SO[k], alpha, r_new);
@@ -1333,16 +1443,18 @@ __global__ void __launch_bounds__(kThreads, 1) wide_round_kernel(WideJob job)
     tc::fence_after_sync();
     oz.tmem = tmem_base;
   }
-  uint32_t seq = 1;
+  uint32_t seq = 1, q_seq = 1;
   bool blocked = false;
-  const WideSmem sm{dyn_smem, job.smem_doubles, job.tc ? &oz : nullptr, &seq, &blocked};
+  WideQ later{};
+  __shared__ WideJob tj;  // the team's view of the job, read by every thread
+  const WideSmem sm{dyn_smem, job.smem_doubles, job.tc ? &oz : nullptr, &seq, &q_seq, &blocked, &later,
+                    &tj};
   // Teams: the grid splits into `teams` groups of equal size; group g owns
   // its own work buffers (one block of team_bytes each) and barrier word, and
   // rounds items g, g + teams, ... (the order is longest first).
   const int teams = job.teams > 0 ? job.teams : 1;
   const int tsize = static_cast<int>(gridDim.x) / teams;
   const int team = static_cast<int>(blockIdx.x) / tsize;
-  __shared__ WideJob tj;  // the team's view of the job, read by every thread
   if (team < teams && threadIdx.x == 0)
   {
     tj = job;

@@ -120,15 +120,19 @@ __device__ __forceinline__ double packets_sum(const WideJob& job, const uint4* p
 }
 
 // Slots: panel products (slab, column), the panel row's own entries, and the
-// trailing products (slab, column, reflector).
+// products of a block's application (slab, column, reflector), in one region
+// for the sweep's own and one for a Q formed meanwhile.
 __device__ __forceinline__ uint4* panel_slot(const WideJob& job, uint32_t tag, int slab, int l)
 {
   return job.packets + ((tag & 1u) * (kWidePanelSlabs + 1) + slab) * kPb + l;
 }
-__device__ __forceinline__ uint4* trail_slot(const WideJob& job, uint32_t tag, int slab, int col, int i)
+__device__ __forceinline__ uint4* trail_slot(const WideJob& job, int region, uint32_t tag, int slab,
+                                             int col, int i)
 {
   return job.packets + 2 * (kWidePanelSlabs + 1) * kPb +
-         ((static_cast<int64_t>(tag & 1u) * kWideTrailSlabs + slab) * job.c_max + col) * kPb + i;
+         ((static_cast<int64_t>(2 * region + (tag & 1u)) * kWideTrailSlabs + slab) * job.c_max + col) *
+           kPb +
+         i;
 }
 
 // -- panel --------------------------------------------------------------------
@@ -395,7 +399,8 @@ __device__ TrailCut trail_cut(int hp, int m, int P, int64_t cap, int nv)
 template <int G, bool kTrans, class FCol>
 __device__ __forceinline__ bool block_apply_g(const WideJob& job, const double* Vs, int ldv, double* Bs,
                                               int ldb, int nr, int nc, const double* Ts, double* Ws,
-                                              double* Zs, int St, int slab, uint32_t tag, FCol col)
+                                              double* Zs, int St, int slab, int region, uint32_t tag,
+                                              FCol col)
 {
   const int t = threadIdx.x, gl = t & (G - 1), q0 = t / G;
   constexpr int kCols = kThreads / G;
@@ -427,7 +432,7 @@ __device__ __forceinline__ bool block_apply_g(const WideJob& job, const double* 
         if (G < 32 || (gl & 1) == 0)
         {
           if (St > 1)
-            packet_put(trail_slot(job, tag, slab, col(q), i0 + e), acc[e], tag);
+            packet_put(trail_slot(job, region, tag, slab, col(q), i0 + e), acc[e], tag);
           else
             Ws[q * kPb + i0 + e] = acc[e];
         }
@@ -437,7 +442,7 @@ __device__ __forceinline__ bool block_apply_g(const WideJob& job, const double* 
   if (St > 1)
     for (int e = t; e < nc * kPb; e += kThreads)
     {
-      const uint4* p = trail_slot(job, tag, 0, col(e / kPb), e % kPb);
+      const uint4* p = trail_slot(job, region, tag, 0, col(e / kPb), e % kPb);
       const int64_t stride = job.c_max * kPb;
       double v = packets_sum<8>(job, p, stride, St < 8 ? St : 8, tag, &fail);
       if (St > 8)
@@ -496,14 +501,17 @@ __device__ __forceinline__ bool block_apply_g(const WideJob& job, const double* 
 template <bool kTrans, class FCol>
 __device__ bool block_apply(const WideJob& job, const double* Vs, int ldv, double* Bs, int ldb, int nr,
                             int nc, const double* Ts, double* Ws, double* Zs, int St, int slab,
-                            uint32_t tag, FCol col)
+                            int region, uint32_t tag, FCol col)
 {
   // Lanes per column: as few as keep all 256 threads at work.
   if (nc > 16)
-    return block_apply_g<8, kTrans>(job, Vs, ldv, Bs, ldb, nr, nc, Ts, Ws, Zs, St, slab, tag, col);
+    return block_apply_g<8, kTrans>(job, Vs, ldv, Bs, ldb, nr, nc, Ts, Ws, Zs, St, slab, region,
+                                    tag, col);
   if (nc > 8)
-    return block_apply_g<16, kTrans>(job, Vs, ldv, Bs, ldb, nr, nc, Ts, Ws, Zs, St, slab, tag, col);
-  return block_apply_g<32, kTrans>(job, Vs, ldv, Bs, ldb, nr, nc, Ts, Ws, Zs, St, slab, tag, col);
+    return block_apply_g<16, kTrans>(job, Vs, ldv, Bs, ldb, nr, nc, Ts, Ws, Zs, St, slab, region,
+                                     tag, col);
+  return block_apply_g<32, kTrans>(job, Vs, ldv, Bs, ldb, nr, nc, Ts, Ws, Zs, St, slab, region,
+                                     tag, col);
 }
 
 // 8 bytes from global to shared memory, in flight until copies_wait; zeros
@@ -522,18 +530,18 @@ __device__ __forceinline__ void copies_wait()
 
 // Starts the copies of V's rows [r0, r0 + nr) of the block at j0 (zero above
 // row j0 and past nb) and of the block's T into shared memory.
-__device__ __forceinline__ void load_block(const WideJob& job, int h, int j0, int nb, int r0, int nr,
-                                           double* Vs, int ldv, double* Ts)
+__device__ __forceinline__ void load_block(const double* W, const double* Tw, int h, int j0, int nb,
+                                           int r0, int nr, double* Vs, int ldv, double* Ts)
 {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int i = w; i < kPb; i += kWarps)
   {
-    const double* col = job.W + static_cast<int64_t>(i < nb ? j0 + i : j0) * h + r0;
+    const double* col = W + static_cast<int64_t>(i < nb ? j0 + i : j0) * h + r0;
     for (int r = lane; r < nr; r += 32)
       copy_async(Vs + i * ldv + r, col + r, i < nb && r0 + r >= j0);
   }
   for (int e = threadIdx.x; e < kPb * kPb; e += kThreads)
-    copy_async(Ts + e, job.Tw + static_cast<int64_t>(j0 / kPb) * kPb * kPb + e, true);
+    copy_async(Ts + e, Tw + static_cast<int64_t>(j0 / kPb) * kPb * kPb + e, true);
 }
 
 // W's columns from j0 + nb on <- (I - V T^T V^T) W, V the block at j0.
@@ -558,14 +566,14 @@ __device__ __noinline__ bool wide_trail(const WideJob& job, int h, int c, int j0
   double* Zs = Ws + kPb * cut.nc;
   double* Ts = Zs + kPb * cut.nc;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  load_block(job, h, j0, nb, r0, nr, Vs, ld, Ts);
+  load_block(job.W, job.Tw, h, j0, nb, r0, nr, Vs, ld, Ts);
   double* B = job.W + static_cast<int64_t>(c0 + q0) * h + r0;
   for (int q = w; q < nc; q += kWarps)
     for (int r = lane; r < nr; r += 32)
       copy_async(Bs + q * ld + r, B + static_cast<int64_t>(q) * h + r, true);
   copies_wait();
   __syncthreads();
-  if (!block_apply<true>(job, Vs, ld, Bs, ld, nr, nc, Ts, Ws, Zs, cut.St, slab, tag,
+  if (!block_apply<true>(job, Vs, ld, Bs, ld, nr, nc, Ts, Ws, Zs, cut.St, slab, 0, tag,
                          [&](int q) { return q0 + q; }))
     return false;
   for (int q = w; q < nc; q += kWarps)
@@ -575,73 +583,133 @@ __device__ __noinline__ bool wide_trail(const WideJob& job, int h, int c, int j0
   return true;
 }
 
-// out(i, l) = (H_0 ... H_{kref-1} [B; 0])(i, l), l < ncols, from the blocks in
-// W; B column-major (nb_rows x ncols) or, with eye, the identity.  No grid
-// barrier inside; the tags used are seq .. seq + number of blocks.
-__device__ __noinline__ bool wide_q(const WideJob& job, int h, int kref, const double* B, int nb_rows,
-                                    int ncols, double* out, int64_t o_rs, int64_t o_cs, bool eye,
-                                    uint32_t seq, double* sm, int64_t cap)
+// Q = H_0 ... H_{kref-1} [B; 0] (h x ncols) from the explicit blocks in W, to
+// out(i, l) = out[i o_rs + l o_cs]; B column-major (nb_rows x ncols) or, with
+// eye, the identity.  Formed by `size` CTAs of the team, of which this one is
+// `rank` (< 0: takes no part), block by block from the last; a CTA's tile
+// stays in the `cap` doubles at sm in between, so that the blocks can be
+// spread over other work (no grid barrier inside).  Tags seq .. seq + blocks.
+struct WideQ
 {
-  const TrailCut cut = trail_cut(h, ncols, job.size, cap, 2);
-  const int slab = job.rank % cut.St, g = job.rank / cut.St;
-  if (g >= cut.Gt)
-    return true;
-  const int r0 = slab * cut.rows;
-  const int nr = h - r0 < cut.rows ? h - r0 : cut.rows;
+  bool on;
+  int next;  // next block; the same on every CTA of the team
+  const double *W, *Tw, *B;
+  double* out;
+  int64_t o_rs, o_cs;
+  int h, kref, nb_rows, ncols, rank, size, region;
+  bool eye;
+  uint32_t seq;
+  double* sm;
+  int64_t cap;
+  // this CTA's tile
+  TrailCut cut;
+  int slab, g, r0, nr, nc;
+  int ready, buf;  // block whose V is in (or on its way to) buffer buf; -1
+};
+
+__device__ __forceinline__ double* wide_q_tile(const WideQ& q)
+{
+  return q.sm + 2 * kPb * (q.cut.rows | 1);  // behind two slabs of V
+}
+
+__device__ __noinline__ void wide_q_begin(WideQ& q)
+{
+  q.on = true;
+  q.next = (q.kref + kPb - 1) / kPb - 1;
+  q.ready = -1;
+  q.buf = 0;
+  if (q.rank < 0)
+    return;
+  q.cut = trail_cut(q.h, q.ncols, q.size, q.cap, 2);
+  q.slab = q.rank % q.cut.St;
+  q.g = q.rank / q.cut.St;
+  if (q.g >= q.cut.Gt)
+  {
+    q.rank = -1;
+    return;
+  }
+  q.r0 = q.slab * q.cut.rows;
+  q.nr = q.h - q.r0 < q.cut.rows ? q.h - q.r0 : q.cut.rows;
   // Columns g, g + Gt, ...: with the identity start a block touches columns
   // from its own first on, so every group gets some of each.
-  const int nc = (ncols - g + cut.Gt - 1) / cut.Gt;
-  const int ld = cut.rows | 1;
-  double* Vs = sm;  // two slabs
-  double* Bs = Vs + 2 * kPb * ld;
-  double* Ws = Bs + cut.nc * ld;
-  double* Zs = Ws + kPb * cut.nc;
-  double* Ts = Zs + kPb * cut.nc;  // two blocks' T
+  q.nc = (q.ncols - q.g + q.cut.Gt - 1) / q.cut.Gt;
+}
+
+// B's tile into shared memory.
+__device__ __forceinline__ void wide_q_fill(WideQ& q)
+{
+  const int ld = q.cut.rows | 1;
+  double* Bs = wide_q_tile(q);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int q = w; q < nc; q += kWarps)
+  for (int c = w; c < q.nc; c += kWarps)
   {
-    const int l = g + cut.Gt * q;
-    for (int r = lane; r < nr; r += 32)
+    const int l = q.g + q.cut.Gt * c;
+    for (int r = lane; r < q.nr; r += 32)
     {
-      const int gr = r0 + r;
-      Bs[q * ld + r] = eye ? (gr == l ? 1.0 : 0.0)
-                           : (gr < nb_rows ? B[gr + static_cast<int64_t>(l) * nb_rows] : 0.0);
+      const int gr = q.r0 + r;
+      Bs[c * ld + r] = q.eye ? (gr == l ? 1.0 : 0.0)
+                             : (gr < q.nb_rows ? q.B[gr + static_cast<int64_t>(l) * q.nb_rows] : 0.0);
     }
   }
-  const int blocks = (kref + kPb - 1) / kPb;
+}
+
+// The next block's application to this CTA's tile.
+__device__ __noinline__ bool wide_q_block(const WideJob& job, WideQ& q)
+{
+  const int b = q.next--;
+  if (q.rank < 0)
+    return true;
+  if (b == (q.kref + kPb - 1) / kPb - 1)
+    wide_q_fill(q);  // not before: the shared memory is in use until here
   // First of this group's columns that block b touches.
-  auto first_col = [&](int b) {
-    return eye && b * kPb > g ? (b * kPb - g + cut.Gt - 1) / cut.Gt : 0;
+  const int qa = q.eye && b * kPb > q.g ? (b * kPb - q.g + q.cut.Gt - 1) / q.cut.Gt : 0;
+  if (qa >= q.nc)
+    return true;
+  const int ld = q.cut.rows | 1;
+  double* Bs = wide_q_tile(q);
+  double* Ws = Bs + q.cut.nc * ld;
+  double* Zs = Ws + kPb * q.cut.nc;
+  double* Ts = Zs + kPb * q.cut.nc;  // two blocks' T
+  auto load = [&](int blk, int buf) {
+    const int j0 = blk * kPb;
+    load_block(q.W, q.Tw, q.h, j0, q.kref - j0 < kPb ? q.kref - j0 : kPb, q.r0, q.nr,
+               q.sm + buf * kPb * ld, ld, Ts + buf * kPb * kPb);
   };
-  auto load = [&](int b, int buf) {
-    const int j0 = b * kPb;
-    load_block(job, h, j0, kref - j0 < kPb ? kref - j0 : kPb, r0, nr, Vs + buf * kPb * ld, ld,
-               Ts + buf * kPb * kPb);
-  };
-  int b = blocks - 1;
-  while (b >= 0 && first_col(b) >= nc)
-    --b;
-  if (b >= 0)
-    load(b, 0);
-  for (int buf = 0; b >= 0; --b, buf ^= 1)
-  {
-    copies_wait();
-    __syncthreads();
-    if (b > 0)
-      load(b - 1, buf ^ 1);  // in flight while this block is applied
-    const int qa = first_col(b);
-    if (!block_apply<false>(job, Vs + buf * kPb * ld, ld, Bs + qa * ld, ld, nr, nc - qa,
-                            Ts + buf * kPb * kPb, Ws, Zs, cut.St, slab,
-                            seq + static_cast<uint32_t>(blocks - 1 - b),
-                            [&](int q) { return g + cut.Gt * (qa + q); }))
-      return false;
-  }
+  if (q.ready != b)
+    load(b, q.buf);
+  copies_wait();
   __syncthreads();
-  for (int q = w; q < nc; q += kWarps)
+  if (b > 0)
+    load(b - 1, q.buf ^ 1);  // in flight while this block is applied
+  q.ready = b - 1;
+  const uint32_t tag = q.seq + static_cast<uint32_t>((q.kref + kPb - 1) / kPb - 1 - b);
+  const int g = q.g, Gt = q.cut.Gt;
+  const bool ok = block_apply<false>(job, q.sm + q.buf * kPb * ld, ld, Bs + qa * ld, ld, q.nr,
+                                     q.nc - qa, Ts + q.buf * kPb * kPb, Ws, Zs, q.cut.St, q.slab,
+                                     q.region, tag, [&](int c) { return g + Gt * (qa + c); });
+  q.buf ^= 1;
+  return ok;
+}
+
+// All blocks left, and the tile to its place.
+__device__ __noinline__ bool wide_q_end(const WideJob& job, WideQ& q)
+{
+  while (q.next >= 0)
+    if (!wide_q_block(job, q))
+      return false;
+  q.on = false;
+  if (q.rank < 0)
+    return true;
+  copies_wait();
+  __syncthreads();
+  const int ld = q.cut.rows | 1;
+  const double* Bs = wide_q_tile(q);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int c = w; c < q.nc; c += kWarps)
   {
-    const int64_t l = g + cut.Gt * q;
-    for (int r = lane; r < nr; r += 32)
-      out[(r0 + r) * o_rs + l * o_cs] = Bs[q * ld + r];
+    const int64_t l = q.g + q.cut.Gt * c;
+    for (int r = lane; r < q.nr; r += 32)
+      q.out[(q.r0 + r) * q.o_rs + l * q.o_cs] = Bs[c * ld + r];
   }
   __syncthreads();
   return true;
