@@ -438,7 +438,8 @@ constexpr int kSmemThreePerSm = 7168;  // 56 KB
 constexpr int kSmemFourPerSm = 4864;   // 38 KB
 
 // Whole-GPU schedule: chosen for round jobs (method svd, both gauges) by
-// the options, or automatically for at most 4 TTs with a bond rank >= 64.
+// the options, or automatically for at most 4 TTs with a bond rank >= 64, for a
+// lone medium one and, in teams, for a few medium FP64 ones.
 // Work buffers are sized for the largest core and rank of the TTs swept.
 int32_t setup_wide(ttg_plan& P)
 {
@@ -459,7 +460,7 @@ int32_t setup_wide(ttg_plan& P)
     }
   else
     swept = P.order;
-  int64_t core_max = 1, c_max = 1, cols_max = 1, s_max = 1, f_max = 1;
+  int64_t core_max = 1, c_max = 1, cols_max = 1, s_max = 1, f_max = 1, size_sum = 0, cores = 0;
   if (stream)
     for (int it : P.order)
     {
@@ -483,7 +484,10 @@ int32_t setup_wide(ttg_plan& P)
     for (int k = 0; k < ti.d; ++k)
     {
       const CoreSlot& c = P.slots[ti.first + k];
-      core_max = std::max<int64_t>(core_max, static_cast<int64_t>(c.r) * c.n * c.rp);
+      const int64_t size = static_cast<int64_t>(c.r) * c.n * c.rp;
+      core_max = std::max(core_max, size);
+      size_sum += size;
+      ++cores;
       c_max = std::max<int64_t>(c_max, std::max(c.r, c.rp));
       cols += c.rp;
     }
@@ -493,11 +497,31 @@ int32_t setup_wide(ttg_plan& P)
   const bool force_whole = P.opts.schedule == TTG_SCHED_WHOLE_GPU;
   const bool force_teams = P.opts.schedule == TTG_SCHED_TEAMS;
   const bool big = c_max >= 64;
-  // Whole grid on one TT at a time: forced, or AUTO for a few large TTs.
+  // Whole grid on one TT at a time: forced, or AUTO for a few large TTs.  AUTO
+  // also spreads a lone TT whose largest core has 2048 doubles (n = 4, rank
+  // 23): over a CTA per 256 of them, 16 to half the GPU, so that calls from
+  // several threads still run side by side.  One CTA against 16 / 36 / 76, ms:
+  // d=10 n=4 rank 16 sums FP64 1.24 : 1.35 / 1.35 / 1.26, updates 3.29 : 3.58 /
+  // 3.59 / 3.54; rank 24 sums 2.63 : 2.48 / 2.41 / 2.26; rank 32 updates 7.00 :
+  // 6.58 / 6.54 / 6.44, mixed 4.85 : 3.88 / 3.85 / 3.79; rank 48, d=16, 27.5 :
+  // 23.4 / 23.0 / 22.7, mixed 20.0 : 12.9 / 12.5 / 12.2; d=6 n=20 rank 48 sums
+  // 14.9 : 3.6 / 3.2 / 2.8; streaming products of 2304 doubles 3.48 : 2.21.
   // Teams: forced, or offered to the autotuner for 5..256 large TTs (the
-  // default stays one CTA per TT).
-  const bool want_whole = force_whole || (!force_teams && items <= 4 && big);
-  const bool offer_teams = force_teams || (!force_whole && items > 4 && items <= 256 && big);
+  // default stays one CTA per TT), or AUTO for a few FP64 TTs whose mean core
+  // has 2048 doubles: a team each, of at least 5 CTAs.  One CTA per TT against
+  // teams, uneven batches of ranks to 16 / 40 / 64 / 96, ms: 8 TTs 1.88 : 2.28
+  // / 4.1 : 3.6 / 11.9 : 6.5 / 17.7 : 5.9; 30 TTs 3.1 : 3.6 / 7.4 : 6.0 / 14.7 :
+  // 9.1 / 43.0 : 18.2; 38 TTs 3.8 : 5.1 / 8.2 : 9.0 / 17.6 : 13.3 / 49.0 : 25.7.
+  // (Mixed ones stay: their singular vectors would move by 2e-14 over the gap.)
+  const bool is_auto = P.opts.schedule == TTG_SCHED_AUTO && P.items_hint <= items;
+  const bool lone = is_auto && items == 1 && !big && core_max >= 2048;
+  const bool few = is_auto && items > 1 && items <= std::max(device().sms, 1) / 5 && !stream &&
+                   !(items <= 4 && big) && c_max <= 112 && size_sum >= 2048 * cores &&
+                   P.opts.precision != TTG_PREC_MIXED;
+  const int64_t lone_grid = std::max<int64_t>(core_max / 256, 16);
+  const bool want_whole = force_whole || (!force_teams && ((items <= 4 && big) || lone));
+  const bool want_teams = force_teams || few;
+  const bool offer_teams = want_teams || (!force_whole && items > 4 && items <= 256 && big);
   if (stream)
     core_max = std::max(core_max, s_max);
   if (!want_whole && !offer_teams)
@@ -513,6 +537,8 @@ int32_t setup_wide(ttg_plan& P)
   const cudaError_t e = wide_round_setup(static_cast<int>(smem), &grid);
   if (e != cudaSuccess)
     return fail(TTG_ERR_CUDA, std::string("whole-GPU round setup: ") + cudaGetErrorString(e));
+  if (lone)
+    grid = static_cast<int>(std::min<int64_t>(grid / 2, lone_grid));
   if (grid < 2)
     return TTG_OK;
   // Team counts: up to one team per item, at least 4 CTAs per team, 32 teams.
@@ -534,7 +560,7 @@ int32_t setup_wide(ttg_plan& P)
   // A second set of reflectors, for the Q that is formed during the next QR,
   // where the blocked QR (whose tiles lie in shared memory) can take every
   // core: 31 MB at most.
-  const bool later = want_whole && core_max <= int64_t{grid} * smem;
+  const bool later = want_whole && grid >= 2 * kWidePanelSlabs && core_max <= int64_t{grid} * smem;
   const size_t oW = take(cm), oU = take(cm), oP = take(cm), oA = take(cm), oR = take(cc),
                oV = take(cc), oF = take(cc), oT1 = take(cc), oT2 = take(cc),
                opart = take(16 * static_cast<size_t>(grid) + 16), oumax = take(8),
@@ -566,6 +592,7 @@ int32_t setup_wide(ttg_plan& P)
   j.max_sweeps = ms;
   j.jblock = jb;
   j.smem_doubles = smem;
+  j.one_cta = lone || few;
   j.eps = P.opts.eps;
   j.W = reinterpret_cast<double*>(b + oW);
   j.Ub = reinterpret_cast<double*>(b + oU);
@@ -624,7 +651,7 @@ int32_t setup_wide(ttg_plan& P)
     P.wide = true;
     P.wide_teams = 1;
   }
-  else if (force_teams)
+  else if (want_teams)
   {
     P.wide = true;
     P.wide_teams = teams_max;

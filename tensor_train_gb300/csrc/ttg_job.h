@@ -175,6 +175,9 @@ struct WideJob
   double* S2;
   double* Fs;          // streaming: the running F factor
   int64_t smem_doubles;
+  // 1: Jacobi sweeps in one CTA where the matrix fits, in the per-TT order of
+  // rotations (plans that AUTO would else run per TT).
+  int32_t one_cta;
   double eps;
   double* W;           // core_max: reflectors
   double* W2;          // core_max: the other QR's, while its Q is formed; or null
