@@ -135,7 +135,8 @@ typedef struct ttg_tensor {
 
 /* Value of `owned` of an input whose cores do not follow one another in one
  * buffer: core k starts at data[offsets[k]] (its size is that of its shape),
- * offsets[d] is not read.  Cores need not be copied together to be passed. */
+ * offsets[d] is not read.  Cores need not be copied together to be passed.
+ * ttg_free() leaves such a tensor alone. */
 #define TTG_CORES_APART 0x5ca7a
 
 /* ---- library ---------------------------------------------------------- */

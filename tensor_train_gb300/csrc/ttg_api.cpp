@@ -1266,7 +1266,8 @@ int64_t ttg_kernel_launches(void) { return g_launches.load(); }
 
 void ttg_free(ttg_tensor* t)
 {
-  if (!t || !t->owned)
+  // An input's `owned` may say that its cores lie apart: not the library's.
+  if (!t || !t->owned || t->owned == TTG_CORES_APART)
     return;
   std::free(t->ranks);
   std::free(t->rows);
