@@ -958,7 +958,7 @@ int32_t plan_run(ttg_plan& P, cudaStream_t st)
     TTG_CUDA(cudaMemsetAsync(d + P.off_bad, 0, sizeof(int), st));
     const Shape& s = P.shapes[0];
     launch_eval(P.eval_merges, reinterpret_cast<const EvalSeg*>(d + P.off_segs),
-                P.eval_layout.left, static_cast<int>(P.eval_segs.size()),
+                P.eval_layout.left, static_cast<int>(P.eval_layout.cut.size()) - 1,
                 reinterpret_cast<const int*>(d + P.off_modes), s.d,
                 reinterpret_cast<const int*>(d + P.off_idx), P.M,
                 reinterpret_cast<double*>(d + P.off_out), *std::max_element(s.r.begin(), s.r.end()),
@@ -2608,38 +2608,6 @@ int32_t ttg_plan_create_matvec_round(const ttg_tensor* a, const ttg_tensor* x,
 // ---------------------------------------------------------------------------
 // eval_batch, inner, norm.
 // ---------------------------------------------------------------------------
-// Whether products of neighbouring cores stay inside FP64's range wherever
-// the products with a row vector do: every partial sum of the cores' exponents
-// (of the largest entry, plus half the rank's for the sum over it) within 2^800
-// of every other, and no infinity or NaN.  The index-by-index products of such
-// a train neither overflow nor lose anything above 2^-1000 of its scale, and a
-// table spans at most 14 sites, 4 bits each.
-static bool eval_products_safe(const Shape& s)
-{
-  double sum = 0.0, lo = 0.0, hi = 0.0;
-  for (int k = 0; k < s.d; ++k)
-  {
-    const double* x = s.data + s.src_off[k];
-    uint64_t top = 0;
-    for (int64_t i = 0; i < s.size[k]; ++i)
-    {
-      uint64_t u;
-      std::memcpy(&u, x + i, sizeof(u));
-      u &= 0x7ff0000000000000ull;
-      top = u > top ? u : top;
-    }
-    const int e = static_cast<int>(top >> 52);
-    if (e == 0x7ff)
-      return false;
-    if (e == 0)
-      continue;  // a zero core: every product with it is zero
-    sum += e - 1023 + 0.5 * std::log2(static_cast<double>(s.r[k + 1]));
-    lo = std::min(lo, sum);
-    hi = std::max(hi, sum);
-  }
-  return hi - lo <= 800.0;
-}
-
 static int32_t build_eval_plan(ttg_plan& P, const ttg_tensor* a, const int32_t* idx, int32_t M,
                                int32_t M_all)
 {
@@ -2670,8 +2638,6 @@ static int32_t build_eval_plan(ttg_plan& P, const ttg_tensor* a, const int32_t* 
   for (int k = 0; k < s.d; ++k)
     modes[k] = s.mode(k);
   P.eval_layout = plan_eval(s.r.data(), modes.data(), s.d, M_all);
-  if (P.eval_layout.tables && !eval_products_safe(s))
-    plain_eval(P.eval_layout, modes.data(), s.d);
   const int nseg = static_cast<int>(P.eval_layout.cut.size()) - 1;
   TTG_CUDA(eval_smem_optin(nseg, s.d, rmax, P.rcap));
   // layout: [arena | segments | modes | idx] prefix, then [out | bad | tables].
@@ -2679,7 +2645,7 @@ static int32_t build_eval_plan(ttg_plan& P, const ttg_tensor* a, const int32_t* 
   P.off_arena = o;
   o = align256(o + sizeof(double) * static_cast<size_t>(P.arena_doubles));
   P.off_segs = o;
-  o = align256(o + sizeof(EvalSeg) * static_cast<size_t>(nseg));
+  o = align256(o + sizeof(EvalSeg) * static_cast<size_t>(nseg + s.d));
   P.off_modes = o;
   o = align256(o + sizeof(int32_t) * static_cast<size_t>(s.d));
   P.off_order = o;

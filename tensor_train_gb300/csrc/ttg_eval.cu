@@ -14,6 +14,13 @@
 // such a call's values may differ from a smaller one's in their last bits).
 // The cut is picked by counting FMAs: an index then costs one matrix per
 // segment instead of one per site, and a table costs its own FMAs.
+//
+// A product formed ahead of its turn can leave FP64's range where the
+// left-to-right products do not (four sites of 1e-100 after one of 1e250).
+// So every entry formed out of order is looked at as it is stored
+// (out_of_range: its exponent, and its terms where it is tiny), a table's
+// entry that fails becomes a NaN, and an index that meets one, or whose value
+// is not finite, is done again site by site from the left.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -32,25 +39,48 @@ namespace
 constexpr int kEvalWarps = 8;  // per CTA, fewer where the vectors need the room
 constexpr size_t kEvalSmemMax = 227 * 1024;
 
+// Whether the sum y of the products x(i) p(i), i < m, formed before the
+// factors to its left were known, may lack something that the left-to-right
+// order keeps: it is within 2^24 of the largest double or beyond, or it is
+// below 2^-900 and one of its own terms is (a larger entry has lost less than
+// 2^-122 of itself; a small sum of larger terms, or of zeros, is what it is).
+template <class FX, class FP>
+__device__ __forceinline__ bool out_of_range(double y, int m, FX x, FP p)
+{
+  const int e = (__double2hiint(y) >> 20) & 0x7ff;
+  if (e > 1023 + 1000)
+    return true;
+  if (e >= 1023 - 900)
+    return false;
+  for (int i = 0; i < m; ++i)
+  {
+    const double u = x(i), v = p(i);
+    if (u != 0.0 && v != 0.0 && fabs(u * v) < 0x1p-900)
+      return true;
+  }
+  return false;
+}
+
 // T[(i1 N2 + i2)][a][b] = sum_c A(i1, a, c) B(i2, c, b): the products of all
 // pairs of two tables (or cores), one GEMM of (N1 ra) x (N2 rb) x K in
-// 32 x 32 tiles.
+// 32 x 32 tiles.  mark: entries out of range become NaN.
 __global__ void __launch_bounds__(256) merge_kernel(EvalMerge m)
 {
   __shared__ double sm[GridTile<2>::kDoubles];
   const int M = m.N1 * m.ra, N = m.N2 * m.rb;
   const int tn = (N + 31) / 32;
   const int64_t tiles = static_cast<int64_t>((M + 31) / 32) * tn;
+  auto A = [&](int row, int c) {
+    return m.A[(row / m.ra) * m.iA + (row % m.ra) * m.aA + c * m.cA];
+  };
+  auto B = [&](int c, int col) { return m.B[(col / m.rb) * m.iB + c * m.aB + (col % m.rb)]; };
   for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x)
-    grid_tile<2>(static_cast<int>(t / tn) * 32, static_cast<int>(t % tn) * 32, M, N, 0, m.K,
-                 [&](int row, int c) {
-                   return m.A[(row / m.ra) * m.iA + (row % m.ra) * m.aA + c * m.cA];
-                 },
-                 [&](int c, int col) {
-                   return m.B[(col / m.rb) * m.iB + c * m.aB + (col % m.rb)];
-                 },
+    grid_tile<2>(static_cast<int>(t / tn) * 32, static_cast<int>(t % tn) * 32, M, N, 0, m.K, A, B,
                  [&](int row, int col, double v) {
                    const int64_t i = static_cast<int64_t>(row / m.ra) * m.N2 + col / m.rb;
+                   if (m.mark && out_of_range(v, m.K, [&](int c) { return A(row, c); },
+                                              [&](int c) { return B(c, col); }))
+                     v = __longlong_as_double(0x7ff8000000000000ll);
                    m.T[(i * m.ra + row % m.ra) * m.rb + col % m.rb] = v;
                  },
                  sm, m.cA == 1, m.rb == 1);
@@ -58,11 +88,18 @@ __global__ void __launch_bounds__(256) merge_kernel(EvalMerge m)
 
 // y[j] = sum_i x[i] p[i * si + j * sj] for j < n, i < m, by the C lanes of a
 // group (bl = lane in the group): each sum in ascending i, two j per lane at
-// a time where there are that many.
-template <int C>
-__device__ __forceinline__ void group_mv(const double* p, int64_t si, int64_t sj, const double* x,
+// a time where there are that many.  kCheck: true when one of this lane's y is
+// out of range.
+template <int C, bool kCheck>
+__device__ __forceinline__ bool group_mv(const double* p, int64_t si, int64_t sj, const double* x,
                                          int m, double* y, int n, int bl)
 {
+  bool lost = false;
+  auto check = [&](double v, const double* q) {
+    if (kCheck)
+      lost = lost || out_of_range(v, m, [&](int i) { return x[i]; },
+                                  [&](int i) { return q[i * si]; });
+  };
   int j0 = 0;
   for (; j0 + C < n; j0 += 2 * C)
   {
@@ -78,8 +115,12 @@ __device__ __forceinline__ void group_mv(const double* p, int64_t si, int64_t sj
       acc2 = fma(f, b[i * si], acc2);
     }
     y[j] = acc;
+    check(acc, a);
     if (j + C < n)
+    {
       y[j + C] = acc2;
+      check(acc2, b);
+    }
   }
   if (j0 < n)
   {
@@ -90,13 +131,17 @@ __device__ __forceinline__ void group_mv(const double* p, int64_t si, int64_t sj
     for (int i = 0; i < m; ++i)
       acc = fma(x[i], a[i * si], acc);
     if (j0 + bl < n)
+    {
       y[j0 + bl] = acc;
+      check(acc, a);
+    }
   }
+  return lost;
 }
 
 // C lanes per multi-index.  segs[0, nl): the row vector's segments, the first
 // a vector; segs[nl, nseg): the column vector's, the last a vector (none for
-// a single site).  Shared memory: three vectors of rcap doubles per group
+// a single site); segs[nseg, nseg + d): the single sites.  Shared memory: three vectors of rcap doubles per group
 // and, with kStage, the segments, the modes and each group's d indices (a
 // train too long for that reads them from global memory).
 template <int C, bool kStage>
@@ -159,6 +204,7 @@ __global__ void __launch_bounds__(32 * kEvalWarps)
     double* v = s0 + rcap;
     double* x = s0 + 2 * rcap;
     int rq = 1;
+    bool lost = false;
     if (nl < nseg)
     {
       const EvalSeg& e = segs[nseg - 1];
@@ -170,7 +216,7 @@ __global__ void __launch_bounds__(32 * kEvalWarps)
       for (int q = nseg - 2; q >= nl; --q)
       {
         const EvalSeg& g = segs[q];
-        group_mv<C>(entry(g), 1, g.a_stride, s, g.rp, x, g.r, bl);
+        lost |= group_mv<C, true>(entry(g), 1, g.a_stride, s, g.rp, x, g.r, bl);
         rq = g.r;
         __syncwarp();
         double* t = s;
@@ -188,7 +234,7 @@ __global__ void __launch_bounds__(32 * kEvalWarps)
     for (int q = 1; q < nl; ++q)
     {
       const EvalSeg& g = segs[q];
-      group_mv<C>(entry(g), g.a_stride, 1, v, g.r, x, g.rp, bl);
+      group_mv<C, false>(entry(g), g.a_stride, 1, v, g.r, x, g.rp, bl);
       __syncwarp();
       double* t = v;
       v = x;
@@ -205,6 +251,27 @@ __global__ void __launch_bounds__(32 * kEvalWarps)
     }
     else
       acc = v[0];
+    const unsigned again = __ballot_sync(0xffffffffu, lost || !isfinite(acc));
+    if (again)  // from the left, site by site (by the whole warp; others keep theirs)
+    {
+      __syncwarp();
+      const EvalSeg* sites = segs_g + nseg;
+      const double* p = entry(sites[0]);
+      for (int b = bl; b < sites[0].rp; b += C)
+        v[b] = p[b];
+      __syncwarp();
+      for (int k = 1; k < d; ++k)
+      {
+        const EvalSeg& g = sites[k];
+        group_mv<C, false>(entry(g), g.a_stride, 1, v, g.r, x, g.rp, bl);
+        __syncwarp();
+        double* t = v;
+        v = x;
+        x = t;
+      }
+      if (again & group_mask)
+        acc = v[0];
+    }
     if (bl == 0 && live)
     {
       out[smp] = ok ? acc : __longlong_as_double(0x7ff8000000000000ll);
@@ -342,7 +409,6 @@ EvalLayout plan_eval(const int* r, const int* n, int d, int64_t M)
     const int s = L.cut[i], e = L.cut[i + 1];
     if (e - s < 2)
       continue;
-    L.tables = true;
     const bool right = static_cast<int>(i) >= L.left;
     int64_t Nt = right ? n[d - 1] : n[s];
     for (int j = 1; j < e - s; ++j)
@@ -355,18 +421,8 @@ EvalLayout plan_eval(const int* r, const int* n, int d, int64_t M)
   return L;
 }
 
-void plain_eval(EvalLayout& L, const int* n, int d)
-{
-  L.cut.resize(static_cast<size_t>(d) + 1);
-  for (int k = 0; k <= d; ++k)
-    L.cut[static_cast<size_t>(k)] = k;
-  L.left = eval_split(n, d);
-  L.tables = false;
-  L.table_doubles = 0;
-}
-
-// Segments and the merges that fill their tables, for cores at ar + off[k]
-// and tables from `tab` on.
+// Segments, then the single sites, and the merges that fill the segments'
+// tables, for cores at ar + off[k] and tables from `tab` on.
 void lay_out_eval(const EvalLayout& L, const int* r, const int* n, const int64_t* off, int d,
                   const double* ar, double* tab, std::vector<EvalSeg>& segs,
                   std::vector<EvalMerge>& merges)
@@ -394,6 +450,7 @@ void lay_out_eval(const EvalLayout& L, const int* r, const int* n, const int64_t
     for (int j = 1; j < e - s; ++j)
     {
       EvalMerge m{};
+      m.mark = suffix || s > 0;  // the row vectors are the left-to-right products
       const int k = suffix ? d - 1 - j : s + j;
       const int64_t ck_i = r[k + 1], ck_a = static_cast<int64_t>(n[k]) * r[k + 1];
       if (suffix)
@@ -438,6 +495,9 @@ void lay_out_eval(const EvalLayout& L, const int* r, const int* n, const int64_t
     g.a_stride = as;
     segs.push_back(g);
   }
+  for (int k = 0; k < d; ++k)
+    segs.push_back(EvalSeg{ar + off[k], r[k + 1], static_cast<int64_t>(n[k]) * r[k + 1], r[k], r[k + 1],
+                           k, 1});
 }
 
 namespace

@@ -19,7 +19,8 @@ struct EvalSeg
   int32_t r, rp, site, nsites;
 };
 
-// T[(i1 N2 + i2)][a][b] = sum_{c < K} A(i1, a, c) B(i2, c, b).
+// T[(i1 N2 + i2)][a][b] = sum_{c < K} A(i1, a, c) B(i2, c, b); mark: NaN where
+// that left FP64's range.
 struct EvalMerge
 {
   const double* A;
@@ -27,7 +28,7 @@ struct EvalMerge
   const double* B;
   int64_t iB, aB;
   double* T;
-  int32_t N1, ra, K, N2, rb;
+  int32_t N1, ra, K, N2, rb, mark;
 };
 
 // Cut points 0 = cut[0] < ... < d of the segments; a segment of two or more
@@ -36,14 +37,12 @@ struct EvalLayout
 {
   std::vector<int> cut;
   int left = 0;
-  bool tables = false;
   int64_t table_doubles = 0;
 };
 
 // The cheapest cut for M multi-indices of a train of ranks r[0..d] and modes
-// n[0..d), and the cut without tables.
+// n[0..d).
 EvalLayout plan_eval(const int* r, const int* n, int d, int64_t M);
-void plain_eval(EvalLayout& L, const int* n, int d);
 void lay_out_eval(const EvalLayout& L, const int* r, const int* n, const int64_t* off, int d,
                   const double* ar, double* tab, std::vector<EvalSeg>& segs,
                   std::vector<EvalMerge>& merges);
