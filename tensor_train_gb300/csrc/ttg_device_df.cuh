@@ -394,11 +394,7 @@ struct JOps<double>
 };
 // df64: nothing on the FP64 pipe (a warp's instruction holds it for 64 clocks;
 // the rotation in FP64, with its roots and divisions, was ~80 of them).  The
-// rank-96 update round: 22.7 -> 20.1 ms; 456 uneven trains: 115 -> 105 ms.  The
-// tangent is FP32's, then one Newton step on ga t^2 + (be - al) t - ga in
-// df64 (left at FP32's 1e-7 it leaves a pair of nearly equal columns short of
-// orthogonal by more than the sweeps' tolerance can see); the cosine is one
-// third-order step in df64 from the FP32 reciprocal root.
+// rank-96 update round: 22.7 -> 20.1 ms; 456 uneven trains: 115 -> 105 ms.
 template <>
 struct JOps<df64>
 {
@@ -420,29 +416,8 @@ struct JOps<df64>
     const float g = fabsf(ga.hi);
     if (g == 0.0f || g <= static_cast<float>(tol) * size)
       return false;
-    const df64 diff = df_sub(be, al);
-    const float z = diff.hi / (2.0f * ga.hi);
-    const float az = fabsf(z);
-    float t = az > 1.0e9f ? 0.5f / az : 1.0f / (az + sqrtf(fmaf(z, z, 1.0f)));
-    t = z >= 0.0f ? t : -t;
-    const float tt = t * t;
-    float te = fmaf(t, t, -tt);
-    const df64 f = df_fma(diff, df64{t, 0.0f},
-                          df_mul(ga, df_add(df64{tt, te}, df64{-1.0f, 0.0f})));
-    const float tl = -f.hi / fmaf(2.0f * ga.hi, t, diff.hi);
-    te = fmaf(2.0f * t, tl, te);  // (t + tl)^2 = tt + te
-    // e = 1 - (1 + (t + tl)^2) y^2 with y ~ c, from exact sums and products.
-    const float y = rsqrtf(1.0f + tt);
-    const float yy = y * y, ye = fmaf(y, y, -yy);
-    const float p = tt * yy, pe = fmaf(tt, yy, -p);
-    const df64 d1 = two_sum(1.0f, -yy), d = two_sum(d1.hi, -p);
-    const float lo = (d1.lo + d.lo) - ((pe + ye) + fmaf(tt, ye, te * yy));
-    // c = y (1 - e)^(-1/2) = y + y e / 2 + 3/8 y e^2, e = d.hi + lo.
-    const float e = d.hi + lo, h = 0.5f * d.hi;
-    const float yh = y * h, yhe = fmaf(y, h, -yh);
-    const df64 c1 = fast_two_sum(y, yh);
-    const df64 c = fast_two_sum(c1.hi, c1.lo + fmaf(y, fmaf(0.375f * e, e, 0.5f * lo), yhe));
-    const df64 tan = fast_two_sum(t, tl);
+    df64 tan, c;
+    df_rotation(al, be, ga, &tan, &c);
     const df64 s = df_mul(c, tan);
     *r = Rot{c, s, df_neg(s)};
     *na = df_fma(df_neg(tan), ga, al);

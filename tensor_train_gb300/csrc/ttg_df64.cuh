@@ -220,6 +220,44 @@ __host__ __device__ __forceinline__ df64 df_sqrt(df64 a)
   return fast_two_sum(y, d / (y + y));
 }
 
+// The rotation that makes two columns orthogonal from their squared norms al,
+// be and product ga != 0: *tan and *c = 1 / sqrt(1 + tan^2), on the FP32 pipes.
+// The tangent is FP32's, then one Newton step on ga t^2 + (be - al) t - ga
+// in df64 (left at FP32's 1e-7 it leaves a pair of nearly equal columns short
+// of orthogonal by more than the sweeps' tolerance can see): it is off by 4e-14
+// of itself, which the next rotation of the pair takes up.  The cosine is one
+// third-order step in df64 from the FP32 reciprocal root, to 2^-48: a column's
+// length has no later correction.
+__host__ __device__ __forceinline__ void df_rotation(df64 al, df64 be, df64 ga, df64* tan, df64* cosine)
+{
+  const df64 diff = df_sub(be, al);
+  const float z = diff.hi / (2.0f * ga.hi);
+  const float az = fabsf(z);
+  float t = az > 1.0e9f ? 0.5f / az : 1.0f / (az + sqrtf(fmaf(z, z, 1.0f)));
+  t = z >= 0.0f ? t : -t;
+  float tt = t * t;
+  float te = fmaf(t, t, -tt);
+  const df64 f = df_fma(diff, df64{t, 0.0f},
+                        df_mul(ga, df_add(df64{tt, te}, df64{-1.0f, 0.0f})));
+  const df64 tn = fast_two_sum(t, -f.hi / fmaf(2.0f * ga.hi, t, diff.hi));
+  // tan^2 = tt + te (of the sum: the step's own size, up to 4 ulp of t, would
+  // leave te no bits to spare).
+  tt = tn.hi * tn.hi;
+  te = fmaf(2.0f * tn.hi, tn.lo, fmaf(tn.hi, tn.hi, -tt));
+  // e = 1 - (1 + tan^2) y^2 with y ~ c, from exact sums and products.
+  const float y = rsqrtf(1.0f + tt);
+  const float yy = y * y, ye = fmaf(y, y, -yy);
+  const float p = tt * yy, pe = fmaf(tt, yy, -p);
+  const df64 d1 = two_sum(1.0f, -yy), d = two_sum(d1.hi, -p);
+  const float lo = (d1.lo + d.lo) - ((pe + ye) + fmaf(tt, ye, te * yy));
+  // c = y (1 - e)^(-1/2) = y + y e / 2 + 3/8 y e^2, e = d.hi + lo.
+  const float e = d.hi + lo, h = 0.5f * d.hi;
+  const float yh = y * h, yhe = fmaf(y, h, -yh);
+  const df64 c1 = fast_two_sum(y, yh);
+  *cosine = fast_two_sum(c1.hi, c1.lo + fmaf(y, fmaf(0.375f * e, e, 0.5f * lo), yhe));
+  *tan = tn;
+}
+
 __device__ __forceinline__ df64 df_shfl_xor(df64 a, int o)
 {
   return df64{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
