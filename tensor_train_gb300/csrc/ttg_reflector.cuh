@@ -3,6 +3,7 @@
 // products.
 #pragma once
 
+#include <cfloat>
 #include <cuda_runtime.h>
 
 namespace ttg
@@ -39,6 +40,13 @@ __device__ __forceinline__ bool not_negative(double x)  // -0.0 counts as 0
 {
   const long long b = __double_as_longlong(x);
   return b >= 0 || (b << 1) == 0;
+}
+// Whether a column has anything below its diagonal: tail2 > DBL_MIN for a sum
+// of squares, and true for a NaN of either sign (inf - inf is 0xfff8... on a
+// host), so that it reaches R and the norm.
+__device__ __forceinline__ bool has_tail(double tail2)
+{
+  return (__double_as_longlong(tail2) & 0x7fffffffffffffffll) > __double_as_longlong(DBL_MIN);
 }
 __device__ __forceinline__ double copy_sign(double mag, bool positive)
 {

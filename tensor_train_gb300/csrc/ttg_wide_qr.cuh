@@ -28,7 +28,6 @@
 // Reflector convention as cta_householder_qr (Eigen's makeHouseholder).
 #pragma once
 
-#include <cfloat>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -261,7 +260,7 @@ __device__ __noinline__ bool wide_panel(const WideJob& job, int h, int k, int j0
       const double tail2 = ps.d[i], x0 = ps.row[i];
       const bool up = not_negative(x0);
       double beta = x0, tau = 0.0, inv = 0.0, wi = 0.0;
-      if (__double_as_longlong(tail2) > __double_as_longlong(DBL_MIN))  // tail2 >= 0, or a NaN
+      if (has_tail(tail2))
       {
         double n, rs;
         const double ax = fabs(x0);

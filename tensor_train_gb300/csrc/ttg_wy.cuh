@@ -14,7 +14,6 @@
 // updates.
 #pragma once
 
-#include <cfloat>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -106,7 +105,7 @@ __device__ __noinline__ void wy_panel(double* P, int64_t ldp, int hp, int nb, Wy
       const double tail2 = ps.d[i], x0 = ps.row[i];
       const bool up = not_negative(x0);
       double beta = x0, tau = 0.0, inv = 0.0, wi = 0.0;
-      if (__double_as_longlong(tail2) > __double_as_longlong(DBL_MIN))  // tail2 >= 0, or a NaN
+      if (has_tail(tail2))
       {
         double n, rs;
         const double ax = fabs(x0);
