@@ -24,6 +24,7 @@
 #include "ttg_job.h"
 #include "ttg_eval.h"
 #include "ttg_kernels.h"
+#include "ttg_tune.h"
 
 using namespace ttg;
 
@@ -429,14 +430,6 @@ double est_cost(const Shape& s)
   return c;
 }
 
-// Dynamic shared memory of the sweep kernel: two CTAs per SM share the
-// SM's 228 KB (each also has ~17 KB of static shared state) when the grid
-// is larger than the SM count, one CTA gets ~200 KB otherwise.
-constexpr int kSmemTwoPerSm = 11776;  // 92 KB
-constexpr int kSmemOnePerSm = 25600;  // 200 KB
-constexpr int kSmemThreePerSm = 7168;  // 56 KB
-constexpr int kSmemFourPerSm = 4864;   // 38 KB
-
 // Whole-GPU schedule: chosen for round jobs (method svd, both gauges) by
 // the options, or automatically for at most 4 TTs with a bond rank >= 64, for a
 // lone medium one and, in teams, for a few medium FP64 ones.
@@ -704,13 +697,12 @@ int32_t layout_and_alloc(ttg_plan& P)
   const int64_t items = static_cast<int64_t>(P.order.size());
   P.cps = sweep_ctas_per_sm(P, std::max(items, P.items_hint), sms);
   P.grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(items, int64_t{P.cps} * sms)));
-  constexpr int kSmem[5] = {0, kSmemOnePerSm, kSmemTwoPerSm, kSmemThreePerSm, kSmemFourPerSm};
-  P.smem_doubles = kSmem[P.cps];
+  P.smem_doubles = kSmemPerSm[P.cps];
   // Which form a df64 factorisation takes depends on its size and the batch's
   // alone, not on the CTAs per SM (which are a matter of speed, and tuned):
   // the forms round differently, and a mixed batch of hundreds of TTs has
   // singular values close enough together (1e-7) to show it.
-  P.form_doubles = kSmem[items <= sms ? 1 : (items >= 3LL * sms && P.job_kind >= 0 ? 3 : 2)];
+  P.form_doubles = kSmemPerSm[items <= sms ? 1 : (items >= 3LL * sms && P.job_kind >= 0 ? 3 : 2)];
   // Scratch for every launch the autotuner may try: up to 2 CTAs per SM, 4 for
   // larger batches.
   P.scratch_ctas = P.grid;
@@ -1320,11 +1312,39 @@ int32_t ttg_plan_run(ttg_plan* P, void* stream)
   return plan_run(*P, static_cast<cudaStream_t>(stream));
 }
 
-// Autotuner: times each launch configuration of the plan's sweep on the
-// plan itself (every run restarts from the pristine inputs) and keeps the
-// fastest.  Per-TT schedule: one CTA per SM with 200 KB of shared staging,
-// or two per SM with 92 KB each.  Whole-GPU schedule: Jacobi block widths
-// 2, 4 and 8 columns, and the per-TT schedule as a contender.
+// The launch configurations of the plan.
+static std::vector<TuneConfig> plan_configs(const ttg_plan& P)
+{
+  TuneInput in;
+  in.items = static_cast<int>(P.order.size());
+  in.sms = std::max(device().sms, 1);
+  in.scratch_ctas = P.scratch_ctas;
+  const bool stream = P.job_kind == kJobStreamMatvec || P.job_kind == kJobStreamMatmat;
+  int64_t rows = 1;  // of the tallest matrix factored (streaming: not known here)
+  for (int t : P.order)
+    for (int k = 0; !stream && k < P.tts[t].d; ++k)
+    {
+      const CoreSlot& c = P.slots[P.tts[t].first + k];
+      rows = std::max({rows, static_cast<int64_t>(c.r) * c.n, static_cast<int64_t>(c.n) * c.rp});
+    }
+  if (P.opts.precision == TTG_PREC_MIXED)
+  {
+    in.form_doubles = P.form_doubles;
+    in.panel_doubles = stream ? INT32_MAX : rows * kWyB;
+  }
+  in.can_wide = P.wide_grid > 0 && P.wjob.W != nullptr;
+  in.c_max = P.wjob.c_max;
+  in.wide_grid = P.wide_grid;
+  in.wide_teams_max = P.wide_teams_max;
+  in.tensor_cores = P.wjob.mixed && P.wjob.tc;
+  in.jblock = P.wjob.jblock;
+  in.tc = P.wjob.tc;
+  return tune_configs(in);
+}
+
+// Autotuner: times each launch configuration of the plan's sweep
+// (ttg_tune.h) on the plan itself (every run restarts from the pristine inputs)
+// and keeps the fastest.
 int32_t ttg_plan_autotune(ttg_plan* P, void* stream, int32_t* choice)
 {
   if (!P)
@@ -1335,51 +1355,8 @@ int32_t ttg_plan_autotune(ttg_plan* P, void* stream, int32_t* choice)
     return TTG_OK;
   P->drop_graph();
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int sms = std::max(device().sms, 1);
-  const int items = static_cast<int>(P->order.size());
-  struct Cand
-  {
-    int code;  // 1/2: per TT, CTAs per SM; 100 + b (+ 1000 with tensor cores): whole GPU
-    bool wide;
-    int grid, smem, jblock, tc, cps, teams = 1;
-  };
-  std::vector<Cand> cands;
-  const int g1 = std::max(1, std::min(items, sms)), g2 = std::max(1, std::min(items, 2 * sms));
-  cands.push_back({1, false, g1, kSmemOnePerSm, P->wjob.jblock, P->wjob.tc, 1});
-  if (g2 > g1)
-    cands.push_back({2, false, g2, kSmemTwoPerSm, P->wjob.jblock, P->wjob.tc, 2});
-  const int g3 = std::max(1, std::min(items, 3 * sms)), g4 = std::max(1, std::min(items, 4 * sms));
-  if (g3 > g2 && g3 <= P->scratch_ctas)
-    cands.push_back({3, false, g3, kSmemThreePerSm, P->wjob.jblock, P->wjob.tc, 3});
-  if (g4 > g3 && g4 <= P->scratch_ctas)
-    cands.push_back({4, false, g4, kSmemFourPerSm, P->wjob.jblock, P->wjob.tc, 4});
-  const bool can_wide = P->wide_grid > 0 && P->wjob.W != nullptr;
+  const std::vector<TuneConfig> cands = plan_configs(*P);
   const int teams0 = P->wide_teams;
-  if (can_wide)
-  {
-    int64_t c_max = 1;
-    for (int t : P->order)
-      for (int k = 0; k < P->tts[t].d; ++k)
-      {
-        const CoreSlot& c = P->slots[P->tts[t].first + k];
-        c_max = std::max<int64_t>(c_max, std::max(c.r, c.rp));
-      }
-    if (P->wide_teams_max <= 1)
-    {
-      // The sliced-BF16 tensor-core tiles are tried only when they were
-      // opted into (TTG_WIDE_TENSOR_CORES=1): they are no faster on these
-      // barrier-bound sweeps and carry ~1e-12 instead of FP64 rounding per
-      // product, which reached 2.6e-10 on the d=40 rank-257 round.
-      for (int tcv = 0; tcv <= (P->wjob.mixed && P->wjob.tc ? 1 : 0); ++tcv)
-        for (int b : {2, 4, 8})
-          if ((6 * c_max + 2) * b <= kSmemOnePerSm)
-            cands.push_back({100 + b + 1000 * tcv, true, P->wide_grid, kSmemOnePerSm, b, tcv, 1, 1});
-    }
-    else
-      for (int t : {4, 8, 16, 32})
-        if (t <= P->wide_teams_max)
-          cands.push_back({10000 + t, true, P->wide_grid, kSmemOnePerSm, P->wjob.jblock, 0, 1, t});
-  }
   const bool wide0 = P->wide;
   const int grid0 = P->grid, smem0 = P->smem_doubles, jb0 = P->wjob.jblock, tc0 = P->wjob.tc,
             cps0 = P->cps;
@@ -1387,7 +1364,7 @@ int32_t ttg_plan_autotune(ttg_plan* P, void* stream, int32_t* choice)
   int bi = -1;
   for (size_t i = 0; i < cands.size(); ++i)
   {
-    const Cand& c = cands[i];
+    const TuneConfig& c = cands[i];
     P->wide = c.wide;
     P->grid = c.grid;
     P->smem_doubles = c.smem;
@@ -1431,7 +1408,7 @@ int32_t ttg_plan_autotune(ttg_plan* P, void* stream, int32_t* choice)
     P->wide_teams = teams0;
     return TTG_OK;
   }
-  const Cand& c = cands[static_cast<size_t>(bi)];
+  const TuneConfig& c = cands[static_cast<size_t>(bi)];
   P->wide = c.wide;
   P->grid = c.grid;
   P->smem_doubles = c.smem;

@@ -134,6 +134,9 @@ struct GridBar
   int err;
 };
 
+// Reflectors per block of the per-TT df64 QR (ttg_wy_df.cuh).
+constexpr int kWyB = 8;
+
 // Blocked QR of the whole-GPU kernel (ttg_wide_qr.cuh): reflectors per block,
 // most row slabs of a panel and of a block's application, and the exchange
 // packets (16 bytes each) of one team for ranks up to c_max.

@@ -27,13 +27,12 @@
 
 #include "ttg_device.cuh"
 #include "ttg_device_df.cuh"
+#include "ttg_job.h"
 
 namespace ttg
 {
 namespace
 {
-
-constexpr int kWyB = 8;  // reflectors per block
 
 // Shared staging the blocked routines need for m rows (in doubles).
 __device__ __forceinline__ int64_t wy_stage_need(int m)
