@@ -304,14 +304,16 @@ int32_t ttg_plan_upload(ttg_plan* plan, void* stream);
  * (the deep copy of round(const tt&), round/tt_round.hpp:129-134) and runs
  * the sweep on it.  Idempotent: repeated runs give the same result. */
 int32_t ttg_plan_run(ttg_plan* plan, void* stream);
-/* Autotuner: times the plan's launch configurations on the plan itself
- * (per-TT schedule: 1, 2, 3 or 4 CTAs per SM, i.e. 200, 92, 56 or 38 KB of
- * shared staging and 128, 128, 85 or 64 registers per thread; whole-GPU schedule: Jacobi block widths 2/4/8, and the per-TT
- * schedule as a contender; on the mixed path also with and without the
- * sliced-BF16 tensor-core contractions) and keeps the fastest.  *choice
- * (optional): 1-4 = per TT with that many CTAs per SM, 100 + b = whole
- * GPU with block width b (+1000 with tensor-core contractions), 10000 + t =
- * t teams of CTAs, 0 = nothing to tune.  Synchronises `stream`; drops a captured
+/* Autotuner: times the plan's launch configurations on the plan itself and
+ * keeps the fastest, the one that it has among them (per-TT schedule: 1, 2, 3 or
+ * 4 CTAs per SM, i.e. 200, 92, 56 or 38 KB of shared staging and 128, 128, 85 or
+ * 64 registers per thread, in mixed precision those that factor every matrix in
+ * the same form; whole-GPU schedule: Jacobi block widths 2/4/8, and the per-TT
+ * schedule as a contender; with TTG_WIDE_TENSOR_CORES=1 also the sliced-BF16
+ * tensor-core contractions of the mixed path; teams of CTAs: 4, 8, 16, 32).
+ * *choice (optional): 1-4 = per TT with that many CTAs per SM, 100 + b = whole
+ * GPU with block width b (+1000 with tensor-core contractions), 10000 + t = t
+ * teams of CTAs, 0 = nothing to tune.  Synchronises `stream`; drops a captured
  * graph (capture again afterwards). */
 int32_t ttg_plan_autotune(ttg_plan* plan, void* stream, int32_t* choice);
 /* enable != 0: capture one run (deep copy from the pristine inputs, the

@@ -1337,6 +1337,9 @@ static std::vector<TuneConfig> plan_configs(const ttg_plan& P)
   in.wide_grid = P.wide_grid;
   in.wide_teams_max = P.wide_teams_max;
   in.tensor_cores = P.wjob.mixed && P.wjob.tc;
+  in.wide = P.wide;
+  in.cps = P.cps;
+  in.teams = P.wide_teams;
   in.jblock = P.wjob.jblock;
   in.tc = P.wjob.tc;
   return tune_configs(in);
@@ -1356,15 +1359,7 @@ int32_t ttg_plan_autotune(ttg_plan* P, void* stream, int32_t* choice)
   P->drop_graph();
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const std::vector<TuneConfig> cands = plan_configs(*P);
-  const int teams0 = P->wide_teams;
-  const bool wide0 = P->wide;
-  const int grid0 = P->grid, smem0 = P->smem_doubles, jb0 = P->wjob.jblock, tc0 = P->wjob.tc,
-            cps0 = P->cps;
-  float best = 0.0f;
-  int bi = -1;
-  for (size_t i = 0; i < cands.size(); ++i)
-  {
-    const TuneConfig& c = cands[i];
+  auto use = [&](const TuneConfig& c) {
     P->wide = c.wide;
     P->grid = c.grid;
     P->smem_doubles = c.smem;
@@ -1372,7 +1367,8 @@ int32_t ttg_plan_autotune(ttg_plan* P, void* stream, int32_t* choice)
     P->wjob.tc = c.tc;
     P->cps = c.cps;
     P->wide_teams = c.teams;
-    float ms = 0.0f;
+  };
+  auto timed = [&](float* ms) -> int32_t {
     for (int rep = 0; rep < 2; ++rep)  // warm, then timed
     {
       TTG_CUDA(cudaEventRecord(P->ev0, st));
@@ -1380,7 +1376,7 @@ int32_t ttg_plan_autotune(ttg_plan* P, void* stream, int32_t* choice)
         return e;
       TTG_CUDA(cudaEventRecord(P->ev1, st));
       TTG_CUDA(cudaEventSynchronize(P->ev1));
-      TTG_CUDA(cudaEventElapsedTime(&ms, P->ev0, P->ev1));
+      TTG_CUDA(cudaEventElapsedTime(ms, P->ev0, P->ev1));
     }
     if (P->wide)
     {
@@ -1391,33 +1387,28 @@ int32_t ttg_plan_autotune(ttg_plan* P, void* stream, int32_t* choice)
         if (bar.err)
           return fail(TTG_ERR_TIMEOUT, "autotune: a grid barrier wait timed out");
     }
-    if (bi < 0 || ms < best)
+    return TTG_OK;
+  };
+  size_t pick = 0;
+  float best = 0.0f;
+  for (size_t i = 0; i < cands.size(); ++i)
+  {
+    use(cands[i]);
+    float ms = 0.0f;
+    if (int32_t e = timed(&ms))
+    {
+      use(cands[0]);
+      return e;
+    }
+    if (i == 0 || ms < best)
     {
       best = ms;
-      bi = static_cast<int>(i);
+      pick = i;
     }
   }
-  if (bi < 0)
-  {
-    P->wide = wide0;
-    P->grid = grid0;
-    P->smem_doubles = smem0;
-    P->wjob.jblock = jb0;
-    P->wjob.tc = tc0;
-    P->cps = cps0;
-    P->wide_teams = teams0;
-    return TTG_OK;
-  }
-  const TuneConfig& c = cands[static_cast<size_t>(bi)];
-  P->wide = c.wide;
-  P->grid = c.grid;
-  P->smem_doubles = c.smem;
-  P->wjob.jblock = c.jblock;
-  P->wjob.tc = c.tc;
-  P->cps = c.cps;
-  P->wide_teams = c.teams;
+  use(cands[pick]);
   if (choice)
-    *choice = c.code;
+    *choice = cands[pick].code;
   return TTG_OK;
 }
 

@@ -38,7 +38,9 @@ struct TuneInput
   int wide_grid = 0, wide_teams_max = 1;
   bool tensor_cores = false;
   int64_t c_max = 1;  // largest rank
-  int jblock = 1, tc = 0;
+  // as the plan stands
+  int cps = 1, jblock = 1, tc = 0, teams = 1;
+  bool wide = false;
 };
 
 // Whether CTAs with `smem` doubles take the same form of every factorisation
@@ -50,15 +52,28 @@ inline bool keeps_form(const TuneInput& in, int smem)
   return std::min<int64_t>(in.form_doubles, in.panel_doubles) <= smem;
 }
 
+// The plan's own configuration first, so that tuning cannot leave it slower.
 inline std::vector<TuneConfig> tune_configs(const TuneInput& in)
 {
+  const int grid0 = std::max(1, std::min(in.items, in.cps * in.sms));
   std::vector<TuneConfig> out;
+  if (!in.wide)
+    out.push_back({in.cps, false, grid0, kSmemPerSm[in.cps], in.jblock, in.tc, in.cps});
+  else if (in.teams > 1)
+    out.push_back({10000 + in.teams, true, in.wide_grid, kSmemOnePerSm, in.jblock, in.tc, 1, in.teams});
+  else
+    out.push_back({100 + in.jblock + 1000 * in.tc, true, in.wide_grid, kSmemOnePerSm, in.jblock,
+                   in.tc, 1, 1});
+  auto add = [&](const TuneConfig& c) {
+    if (c.code != out[0].code)
+      out.push_back(c);
+  };
   int last = 0;
   for (int cps = 1; cps <= 4; ++cps)
   {
     const int grid = std::max(1, std::min(in.items, cps * in.sms));
     if (grid > last && (cps <= 2 || grid <= in.scratch_ctas) && keeps_form(in, kSmemPerSm[cps]))
-      out.push_back({cps, false, grid, kSmemPerSm[cps], in.jblock, in.tc, cps});
+      add({cps, false, grid, kSmemPerSm[cps], in.jblock, in.tc, cps});
     last = grid;
   }
   if (in.can_wide && in.wide_teams_max <= 1)
@@ -70,12 +85,12 @@ inline std::vector<TuneConfig> tune_configs(const TuneInput& in)
     for (int tc = 0; tc <= (in.tensor_cores ? 1 : 0); ++tc)
       for (int b : {2, 4, 8})
         if ((6 * in.c_max + 2) * b <= kSmemOnePerSm)
-          out.push_back({100 + b + 1000 * tc, true, in.wide_grid, kSmemOnePerSm, b, tc, 1, 1});
+          add({100 + b + 1000 * tc, true, in.wide_grid, kSmemOnePerSm, b, tc, 1, 1});
   }
   else if (in.can_wide)
     for (int t : {4, 8, 16, 32})
       if (t <= in.wide_teams_max)
-        out.push_back({10000 + t, true, in.wide_grid, kSmemOnePerSm, in.jblock, 0, 1, t});
+        add({10000 + t, true, in.wide_grid, kSmemOnePerSm, in.jblock, 0, 1, t});
   return out;
 }
 

@@ -54,6 +54,52 @@ int main()
       if (c.wide)
         CHECK((6 * c_max + 2) * c.jblock <= c.smem);
   }
+  // The plan's own configuration is among them, first, and each only once: the
+  // teams that a few FP64 trains start in (one each, 2 to 30), a lone train over
+  // part of the GPU, and any number of CTAs per SM.
+  for (int items = 2; items <= 30; ++items)
+  {
+    TuneInput in;
+    in.items = items;
+    in.sms = in.scratch_ctas = sms;
+    in.can_wide = in.wide = true;
+    in.wide_grid = sms;
+    in.c_max = 96;
+    in.jblock = 4;
+    in.teams = in.wide_teams_max = items;
+    const auto all = tune_configs(in);
+    CHECK(all[0].wide && all[0].teams == items && all[0].code == 10000 + items);
+    int per_tt = 0;
+    for (size_t i = 1; i < all.size(); ++i)
+    {
+      CHECK(all[i].code != all[0].code);
+      per_tt += !all[i].wide;
+    }
+    CHECK(per_tt == 1);
+  }
+  for (int b : {1, 2, 4, 8})
+  {
+    TuneInput in;
+    in.items = 1;
+    in.sms = in.scratch_ctas = sms;
+    in.can_wide = in.wide = true;
+    in.wide_grid = 16;
+    in.c_max = 48;
+    in.jblock = b;
+    const auto all = tune_configs(in);
+    CHECK(all[0].wide && all[0].teams == 1 && all[0].code == 100 + b && all[0].grid == 16);
+    CHECK(all.size() == (b == 1 ? 5u : 4u));
+  }
+  for (int cps = 1; cps <= 4; ++cps)
+  {
+    TuneInput in;
+    in.items = 5000;
+    in.sms = sms;
+    in.scratch_ctas = 4 * sms;
+    in.cps = cps;
+    const auto all = tune_configs(in);
+    CHECK(all[0].code == cps && all[0].grid == cps * sms && all.size() == 4u);
+  }
   std::printf(g_fail ? "FAILED\n" : "OK\n");
   return g_fail ? 1 : 0;
 }
