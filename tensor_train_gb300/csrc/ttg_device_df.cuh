@@ -637,11 +637,16 @@ struct CertOps<double>
   static __device__ __forceinline__ double mul(double a, double b) { return a * b; }
   static __device__ __forceinline__ double neg(double a) { return -a; }
   static __device__ __forceinline__ double sub(double a, double b) { return a - b; }
-  // One third-order step from the hardware's approximation: a rounding of the
-  // elimination like any other (the library's division is three times the
-  // instructions, on the path of every pivot).
+  // One third-order step (Householder's iteration) from the hardware's
+  // approximation, to 1.1 2^-53: a rounding of the elimination like any other
+  // (the library's division is three times the instructions, on the path of
+  // every pivot).  The approximation takes a subnormal for zero and returns
+  // one as zero: near the ends of the range the library divides.
   static __device__ __forceinline__ double recip(double a)
   {
+    const int ex = (__double2hiint(a) >> 20) & 0x7ff;
+    if (ex < 23 || ex > 2023)
+      return 1.0 / a;
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
     const double e = ::fma(-a, r, 1.0);

@@ -15,10 +15,14 @@ namespace
 // n = |x|, rs = 1 / n, inv = 1 / (ax + n).  One third-order step
 // (Householder's iteration: the error of the start cubed) from the hardware's
 // approximations of the reciprocal root and the reciprocal, which hold at
-// least 20 bits: 2^-60 before the last rounding.  What counts is the number
-// of FP64 instructions (64 clocks each) that every other thread waits for:
-// with the library's root and two divisions the step took 1.39 us per column,
-// with these 0.6 us.
+// least 20 bits.  Before the last rounding that leaves 2^-58 of n and rs (e up
+// to 2^-19, 5/16 e^3 dropped) and 2^-57 of inv (f up to 2^-19, f^3 dropped, and
+// f's own rounding, 2^-54): each within 1.1 (n, rs) and 2.6 (inv) of 2^-53.
+// What counts is the number of FP64 instructions (64 clocks each) that every
+// other thread waits for: with the library's root and two divisions the step
+// took 1.39 us per column, with these 0.6 us; the term that t's rounding leaves
+// out of e is one of them (without it n and rs are off by 1.5 and 1.2; d=15
+// rank-83 round 8.8 -> 9.0 ms).
 __device__ __forceinline__ void reflector_scalars(double s, double ax, double* n, double* rs,
                                                   double* inv)
 {
@@ -26,9 +30,12 @@ __device__ __forceinline__ void reflector_scalars(double s, double ax, double* n
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
   const double t = s * y;  // ~n
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(ax + t));
-  const double e = fma(-t, y, 1.0);  // n = t (1 - e)^(-1/2), rs = y (1 - e)^(-1/2)
+  const double d = fma(s, y, -t);
+  // e = 1 - s y^2, with what the rounding of t left out:
+  // n = s y (1 - e)^(-1/2), rs = y (1 - e)^(-1/2).
+  const double e = fma(-d, y, fma(-t, y, 1.0));
   const double q = e * fma(0.375, e, 0.5);
-  *n = t + fma(t, q, fma(s, y, -t));
+  *n = t + fma(t, q, d);
   *rs = fma(y, q, y);
   const double f = fma(-*n, r, fma(-ax, r, 1.0));  // 1 / (ax + n) = r (1 + f + f^2 + ...)
   *inv = fma(r, fma(f, f, f), r);
