@@ -23,7 +23,7 @@ SOURCES = ["ttg_kernels.cu", "ttg_wide.cu", "ttg_api.cpp", "ttg_host.cpp", "ttg_
 HEADERS = ["ttg_device.cuh", "ttg_device_df.cuh", "ttg_df64.cuh", "ttg_job.h", "ttg_kernels.h",
            "ttg_tc.cuh", "ttg_sweep_common.cuh", "ttg_ozaki.cuh", "ttg_wy_df.cuh", "ttg_gemm_live.h",
            "ttg_gridbar.cuh", "ttg_gemm_grid.cuh", "ttg_mlp_back.cuh", "ttg_eval.h", "ttg_wide_qr.cuh",
-           "ttg_reflector.cuh", "ttg_wy.cuh", "ttg_tune.h"]
+           "ttg_reflector.cuh", "ttg_wy.cuh", "ttg_tune.h", "ttg_inner.h"]
 
 
 def _nvcc() -> str:

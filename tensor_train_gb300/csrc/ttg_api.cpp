@@ -23,6 +23,7 @@
 #include "../../include/ttg.h"
 #include "ttg_job.h"
 #include "ttg_eval.h"
+#include "ttg_inner.h"
 #include "ttg_kernels.h"
 #include "ttg_tune.h"
 
@@ -2430,39 +2431,6 @@ int32_t ttg_matmat(const ttg_tensor* A, const ttg_tensor* B, ttg_tensor* out)
   return apply_round_common(A, B, nullptr, out, nullptr, true, 0, "matmat");
 }
 
-// frob_norm_apply (algebra/tt_matrix_frob_norm_apply.hpp:36-98): the
-// product cores (matvec_core, or matmat_core packed as 3-axis cores of mode
-// m*n) are formed in the arena by the apply kernels, then one CTA runs the
-// contract_inner_step chain of the product with itself.  The product stays
-// on the device (the reference avoids holding it for host-memory reasons;
-// it is sum_k r_k^A r_k^x m_k r_{k+1}^A r_{k+1}^x doubles of HBM here).
-// Buffers of the inner-product chain of the TTs a and b (ttg_inner.cu): env
-// (doubles of one environment), the scratch [partials | T | value and barrier
-// word] and the largest tile count of one product.
-struct InnerSizes
-{
-  int64_t env = 1, tmp = 1, tiles = 1;
-  int64_t scratch() const { return 2 * kInnerSlices * env + a32(tmp) + 32; }
-};
-
-static InnerSizes inner_sizes(const CoreSlot* a, const CoreSlot* b, int d)
-{
-  InnerSizes z;
-  auto t16 = [](int64_t n) { return (n + 15) / 16; };
-  for (int k = 0; k < d; ++k)
-  {
-    const int64_t n = a[k].n;
-    z.env = std::max({z.env, static_cast<int64_t>(a[k].r) * b[k].r,
-                      static_cast<int64_t>(a[k].rp) * b[k].rp});
-    z.tmp = std::max(z.tmp, b[k].r * n * a[k].rp);
-    z.tiles = std::max({z.tiles, t16(b[k].r) * t16(n * a[k].rp),
-                        std::min<int64_t>(kInnerSlices, (b[k].r * n + 31) / 32) * t16(a[k].rp) *
-                          t16(b[k].rp)});
-  }
-  z.env = a32(z.env);
-  return z;
-}
-
 // Runs the chain on the plan's scratch (sized by InnerSizes) over the cores
 // in `arena` and waits for the value.
 static int32_t run_inner(ttg_plan& P, const double* arena, const CoreSlot* SA, const CoreSlot* SB,
@@ -2471,8 +2439,7 @@ static int32_t run_inner(ttg_plan& P, const double* arena, const CoreSlot* SA, c
   double* scratch = reinterpret_cast<double*>(static_cast<char*>(P.dev.p) + P.off_scratch);
   double* tail = scratch + P.scratch_stride - 8;  // value, then the barrier word
   GridBar* bar = reinterpret_cast<GridBar*>(tail + 1);
-  TTG_CUDA(launch_inner(arena, SA, SB, d, static_cast<int>(std::min<int64_t>(z.tiles, INT32_MAX)),
-                        std::max(device().sms, 1), scratch, z.env, bar, tail, st));
+  TTG_CUDA(launch_inner(arena, SA, SB, d, z, scratch, bar, tail, st));
   g_launches += 1;
   struct
   {
@@ -2487,6 +2454,12 @@ static int32_t run_inner(ttg_plan& P, const double* arena, const CoreSlot* SA, c
   return TTG_OK;
 }
 
+// frob_norm_apply (algebra/tt_matrix_frob_norm_apply.hpp:36-98): the
+// product cores (matvec_core, or matmat_core packed as 3-axis cores of mode
+// m*n) are formed in the arena by the apply kernels, then the grid runs the
+// contract_inner_step chain of the product with itself.  The product stays
+// on the device (the reference avoids holding it for host-memory reasons;
+// it is sum_k r_k^A r_k^x m_k r_{k+1}^A r_{k+1}^x doubles of HBM here).
 int32_t ttg_frob_norm_apply(const ttg_tensor* a, const ttg_tensor* x, double* out)
 {
   g_err.clear();
@@ -2519,7 +2492,8 @@ int32_t ttg_frob_norm_apply(const ttg_tensor* a, const ttg_tensor* x, double* ou
   if (int32_t st = build_apply_plan(P, A, X, false, nullptr))
     return st;
   const TTInfo ty = P.tts[P.out_tts[0]];
-  const InnerSizes z = inner_sizes(&P.slots[ty.first], &P.slots[ty.first], ty.d);
+  const InnerSizes z = inner_sizes(&P.slots[ty.first], &P.slots[ty.first], ty.d,
+                                  std::max(device().sms, 1));
   P.scratch_stride = z.scratch();
   if (int32_t st = layout_and_alloc(P))
     return st;
@@ -2712,7 +2686,8 @@ int32_t ttg_inner(const ttg_tensor* a, const ttg_tensor* b, double* out)
   P.shapes = {A, B};
   add_tensor(P, A, true, nullptr);
   add_tensor(P, B, true, nullptr);
-  const InnerSizes z = inner_sizes(&P.slots[P.tts[0].first], &P.slots[P.tts[1].first], A.d);
+  const InnerSizes z = inner_sizes(&P.slots[P.tts[0].first], &P.slots[P.tts[1].first], A.d,
+                                  std::max(device().sms, 1));
   P.scratch_stride = z.scratch();
   P.grid = 1;
   P.job_kind = -1;

@@ -16,6 +16,7 @@
 
 #include "ttg_gemm_grid.cuh"
 #include "ttg_gridbar.cuh"
+#include "ttg_inner.h"
 #include "ttg_kernels.h"
 
 namespace ttg
@@ -26,28 +27,18 @@ namespace
 constexpr int kInnerThreads = 256;
 constexpr long long kInnerWaitCycles = 4000000000ll;  // ~2 s
 
-// Slices of the inner dimension K of an (M x N) environment: enough tiles
-// for the grid, at most kInnerSlices, none shorter than a 32-deep slab.
-__host__ __device__ inline int inner_slices(int M, int N, int K, int grid)
-{
-  const int64_t tiles = static_cast<int64_t>((M + 15) / 16) * ((N + 15) / 16);
-  int64_t s = grid / tiles;
-  s = s < (K + 31) / 32 ? s : (K + 31) / 32;
-  s = s < kInnerSlices ? s : kInnerSlices;
-  return s < 1 ? 1 : static_cast<int>(s);
-}
-
 __global__ void __launch_bounds__(kInnerThreads)
   inner_kernel(const double* __restrict__ ar, const CoreSlot* __restrict__ SA,
-               const CoreSlot* __restrict__ SB, int d, double* scratch, int64_t env_cap, GridBar* bar,
+               const CoreSlot* __restrict__ SB, int d, double* scratch, int64_t env, GridBar* bar,
                double* out)
 {
   __shared__ double sm[GridTile<1>::kDoubles];
   const int P = static_cast<int>(gridDim.x), me = static_cast<int>(blockIdx.x);
   double* E = scratch;
-  double* En = scratch + kInnerSlices * env_cap;
-  double* T = scratch + 2 * kInnerSlices * env_cap;
-  int slices = 0;  // partials of E; 0: the 1 x 1 start
+  double* En = scratch + env;
+  double* T = scratch + 2 * env;
+  int slices = 0;  // partials of E, `size` doubles each; 0: the 1 x 1 start
+  int64_t size = 0;
   for (int k = 0; k < d; ++k)
   {
     const int ra = SA[k].r, n = SA[k].n, rap = SA[k].rp;
@@ -65,7 +56,7 @@ __global__ void __launch_bounds__(kInnerThreads)
                      const double* e = E + static_cast<int64_t>(a) * rb + b;
                      double v = __ldcg(e);
                      for (int s = 1; s < slices; ++s)
-                       v += __ldcg(e + s * env_cap);
+                       v += __ldcg(e + s * size);
                      return v;
                    },
                    [&](int a, int j) { return ca[a * w + j]; },
@@ -74,13 +65,14 @@ __global__ void __launch_bounds__(kInnerThreads)
       return;
     const int K = rb * n;
     slices = inner_slices(rap, rbp, K, P);
+    size = static_cast<int64_t>(rap) * rbp;
     const int per = (K + slices - 1) / slices;
     const int tm = (rap + 15) / 16, tn2 = (rbp + 15) / 16;
     for (int t = me; t < tm * tn2 * slices; t += P)
     {
       const int s = t / (tm * tn2), q = t % (tm * tn2);
       const int k0 = s * per, k1 = k0 + per < K ? k0 + per : K;
-      double* Es = En + s * env_cap;
+      double* Es = En + s * size;
       grid_tile<1>((q / tn2) * 16, (q % tn2) * 16, rap, rbp, k0, k1,
                    [&](int a, int p) { return __ldcg(T + static_cast<int64_t>(p) * rap + a); },
                    [&](int p, int b) { return cb[static_cast<int64_t>(p) * rbp + b]; },
@@ -97,25 +89,23 @@ __global__ void __launch_bounds__(kInnerThreads)
   {
     double v = __ldcg(E);
     for (int s = 1; s < slices; ++s)
-      v += __ldcg(E + s * env_cap);
+      v += __ldcg(E + s * size);
     *out = v;
   }
 }
 
 }  // namespace
 
-cudaError_t launch_inner(const double* ar, const CoreSlot* SA, const CoreSlot* SB, int d, int tiles,
-                         int sms, double* scratch, int64_t env_cap, GridBar* bar, double* out,
+cudaError_t launch_inner(const double* ar, const CoreSlot* SA, const CoreSlot* SB, int d,
+                         const InnerSizes& z, double* scratch, GridBar* bar, double* out,
                          cudaStream_t stream)
 {
-  int grid = tiles < sms ? tiles : sms;
-  if (grid < 1)
-    grid = 1;
   cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(GridBar), stream);
   if (e != cudaSuccess)
     return e;
-  void* args[] = {&ar, &SA, &SB, &d, &scratch, &env_cap, &bar, &out};
-  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(inner_kernel), dim3(grid),
+  int64_t env = z.env;
+  void* args[] = {&ar, &SA, &SB, &d, &scratch, &env, &bar, &out};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(inner_kernel), dim3(z.grid),
                                      dim3(kInnerThreads), args, 0, stream);
 }
 

@@ -19,13 +19,11 @@ cudaError_t launch_wide_round(const WideJob& job, int grid, cudaStream_t stream)
 cudaError_t wide_round_setup(int smem_doubles, int* max_grid);
 void launch_apply_core(const double* A, const double* X, double* Y, int r, int m, int p, int rp,
                        int s, int nout, int sp, cudaStream_t stream);
-// Partial environments of the inner-product chain (ttg_inner.cu).
-constexpr int kInnerSlices = 4;
-// <a, b> of two TTs in `ar` into *out (cooperative).  tiles: the most 16 x 16
-// output tiles of any one product (inner_tiles); scratch: inner_scratch
+// <a, b> of two TTs in `ar` into *out (cooperative).  scratch: z.scratch()
 // doubles; bar: the launch's barrier word, whose err the caller reads.
-cudaError_t launch_inner(const double* ar, const CoreSlot* SA, const CoreSlot* SB, int d, int tiles,
-                         int sms, double* scratch, int64_t env_cap, GridBar* bar, double* out,
+struct InnerSizes;  // ttg_inner.h
+cudaError_t launch_inner(const double* ar, const CoreSlot* SA, const CoreSlot* SB, int d,
+                         const InnerSizes& z, double* scratch, GridBar* bar, double* out,
                          cudaStream_t stream);
 cudaError_t round_smem_optin(int smem_doubles);
 void launch_fp64_peak(double* out, int iters, int grid, int block, cudaStream_t stream);
