@@ -37,6 +37,13 @@ __global__ void __launch_bounds__(kInnerThreads)
   double* E = scratch;
   double* En = scratch + env;
   double* T = scratch + 2 * env;
+  // A chain of one CTA needs no barrier word (d = 300, rank 1: 2.56 -> 1.59 ms).
+  auto wait_all = [&] {
+    if (P > 1)
+      return grid_barrier(bar, P, kInnerWaitCycles);
+    __syncthreads();
+    return true;
+  };
   int slices = 0;  // partials of E, `size` doubles each; 0: the 1 x 1 start
   int64_t size = 0;
   for (int k = 0; k < d; ++k)
@@ -61,7 +68,7 @@ __global__ void __launch_bounds__(kInnerThreads)
                    },
                    [&](int a, int j) { return ca[a * w + j]; },
                    [&](int b, int j, double v) { T[b * w + j] = v; }, sm, false, false);
-    if (!grid_barrier(bar, P, kInnerWaitCycles))
+    if (!wait_all())
       return;
     const int K = rb * n;
     slices = inner_slices(rap, rbp, K, P);
@@ -79,7 +86,7 @@ __global__ void __launch_bounds__(kInnerThreads)
                    [&](int a, int b, double v) { Es[static_cast<int64_t>(a) * rbp + b] = v; }, sm,
                    false, false);
     }
-    if (!grid_barrier(bar, P, kInnerWaitCycles))
+    if (!wait_all())
       return;
     double* x = E;
     E = En;
