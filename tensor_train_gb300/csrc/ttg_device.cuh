@@ -101,14 +101,19 @@ __device__ __forceinline__ void cta_fill(double* p, int64_t n, double v)
 // f(i, j) for i < m, j < n by groups of lanes along i (8, 16 or 32 by m):
 // neighbouring lanes get neighbouring i, and no index is divided (a 64-bit
 // division per element made the copies of a 64 x 16 step cost as much as its
-// contraction).
+// contraction).  Where there are fewer columns than groups, several groups
+// share one: a group per column left a 16384 x 1 copy to one warp of eight.
 template <class F>
 __device__ __forceinline__ void cta_each(int m, int n, F f)
 {
   const int G = m > 16 ? 32 : (m > 8 ? 16 : 8);
-  const int gl = threadIdx.x & (G - 1);
-  for (int j = threadIdx.x / G; j < n; j += kThreads / G)
-    for (int i = gl; i < m; i += G)
+  const int groups = kThreads / G, q = threadIdx.x / G;
+  int lg = 0;  // 2^lg groups per column
+  while ((2 << lg) <= groups && n <= groups >> (lg + 1))
+    ++lg;
+  const int step = G << lg;
+  for (int j = q >> lg; j < n; j += groups >> lg)
+    for (int i = static_cast<int>(threadIdx.x & (G - 1)) + G * (q & ((1 << lg) - 1)); i < m; i += step)
       f(i, j);
 }
 
