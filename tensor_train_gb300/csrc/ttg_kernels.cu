@@ -54,15 +54,29 @@ __device__ void gemm_sel(bool mixed, int M, int N, int K, View A, View B, double
 // Where the blocked FP64 Householder routines keep their blocks' T and, for a
 // matrix in global memory, the panel they work on: in the `room` doubles of
 // shared memory at `free` (which for a matrix in shared memory start with
-// it); off when these do not fit.
+// it); off when these do not fit, or the unblocked routines are faster.
 struct Wy
 {
   bool on;
   double* Ts;
   double* stage;
 };
+// The blocked panel takes a column's products with 8 lanes per panel column,
+// whatever their number, so a narrow tall matrix leaves most of the CTA idle
+// where the unblocked column norm and updates use all of it.  FP64 d=10 sweeps
+// of n r x r unfoldings, blocked over unblocked time: 1 column 1.2 (4 rows) to
+// 2.0 (from 2000); 2 columns 1.05 (64 rows) to 1.8; 3: 0.93 (63 rows), 1.07
+// (126); 4: 0.86 (64), 0.99 (192), 1.2 (384); 6: 0.93 (252), 1.12 (384); 8: 0.88
+// (256), 1.04 (384), 1.16 (2048); 9: 0.87 (252), 1.03 (378); 12: 0.93 (384), 0.99
+// (768), 1.04 (2040).
+__device__ __forceinline__ bool wy_faster(int h, int c)
+{
+  return c >= 16 || (c >= 3 && h <= (c >= 12 ? 80 : 40) * c);
+}
 __device__ __forceinline__ Wy wy_place(int h, int c, double* free, int64_t room)
 {
+  if (!wy_faster(h, c))
+    return Wy{false, nullptr, nullptr};
   const int64_t hc = static_cast<int64_t>(h) * c, t = wy_t_need(h < c ? h : c);
   if (hc + t <= room)
     return Wy{true, free + hc, nullptr};
