@@ -76,8 +76,9 @@ typedef enum ttg_precision { TTG_PREC_FP64 = 0, TTG_PREC_MIXED = 1 } ttg_precisi
  * many TTs in flight, or the whole GPU on one TT at a time (cooperative
  * launch; for a few large TTs).  AUTO picks the whole GPU when a call
  * holds at most 4 TTs with a bond rank of 64 or more, part of it for a lone TT
- * with a core of 2048 doubles or more, and a team per TT for 2 to 30 FP64 TTs
- * of such mean cores and ranks to 112. */
+ * with a core of 2048 doubles and a mean core of 1024 (mixed precision and
+ * streaming products: 640), and a team per TT for 2 to 30 FP64 TTs of mean
+ * cores of 2048 doubles and ranks to 112. */
 typedef enum ttg_schedule {
   TTG_SCHED_AUTO = 0,
   TTG_SCHED_PER_TT = 1,

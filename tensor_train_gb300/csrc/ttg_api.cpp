@@ -471,17 +471,18 @@ int32_t setup_wide(ttg_plan& P)
         f_max = std::max(f_max, (b * bx) * (b * bx));
       }
     }
-  for (int t : swept)
+  for (size_t i = 0; i < swept.size(); ++i)
   {
-    const TTInfo& ti = P.tts[t];
+    const TTInfo& ti = P.tts[swept[i]];
+    const bool counted = !stream || i % 3 == 2;  // not an operand of a product
     int64_t cols = 0;
     for (int k = 0; k < ti.d; ++k)
     {
       const CoreSlot& c = P.slots[ti.first + k];
       const int64_t size = static_cast<int64_t>(c.r) * c.n * c.rp;
       core_max = std::max(core_max, size);
-      size_sum += size;
-      ++cores;
+      size_sum += counted ? size : 0;
+      cores += counted ? 1 : 0;
       c_max = std::max<int64_t>(c_max, std::max(c.r, c.rp));
       cols += c.rp;
     }
@@ -493,8 +494,15 @@ int32_t setup_wide(ttg_plan& P)
   const bool big = c_max >= 64;
   // Whole grid on one TT at a time: forced, or AUTO for a few large TTs.  AUTO
   // also spreads a lone TT whose largest core has 2048 doubles (n = 4, rank
-  // 23): over a CTA per 256 of them, 16 to half the GPU, so that calls from
-  // several threads still run side by side.  One CTA against 16 / 36 / 76, ms:
+  // 23) and whose mean core has 1024 (mixed ones and streaming products, by
+  // their outputs: 640): a small core's step is all grid barriers.  One CTA
+  // against the spread form by mean core, ms: FP64 d=60 n=8 115 2.9 : 4.6, 553
+  // 5.3 : 6.3, 821 7.2 : 7.4, 1146 8.3 : 8.2, 1527 9.8 : 8.9; d=20 n=2 619 3.0 :
+  // 3.2, 966 3.8 : 3.6; mixed d=60 n=8 252 4.4 : 5.4, 553 6.3 : 6.3, 821 8.6 : 7.4;
+  // d=60 n=2 556 9.3 : 10.1, 740 10.6 : 11.0, 1028 13.0 : 11.9; streaming 280 7.4 :
+  // 9.5, 660 2.47 : 2.22, 950 12.9 : 11.7.  It takes a CTA per 256 doubles of the
+  // largest core, 16 to half the GPU, which leaves room for a plan on another
+  // stream (one-shot calls take turns).  One CTA against 16 / 36 / 76, ms:
   // d=10 n=4 rank 16 sums FP64 1.24 : 1.35 / 1.35 / 1.26, updates 3.29 : 3.58 /
   // 3.59 / 3.54; rank 24 sums 2.63 : 2.48 / 2.41 / 2.26; rank 32 updates 7.00 :
   // 6.58 / 6.54 / 6.44, mixed 4.85 : 3.88 / 3.85 / 3.79; rank 48, d=16, 27.5 :
@@ -508,7 +516,9 @@ int32_t setup_wide(ttg_plan& P)
   // 9.1 / 43.0 : 18.2; 38 TTs 3.8 : 5.1 / 8.2 : 9.0 / 17.6 : 13.3 / 49.0 : 25.7.
   // (Mixed ones stay: their singular vectors would move by 2e-14 over the gap.)
   const bool is_auto = P.opts.schedule == TTG_SCHED_AUTO && P.items_hint <= items;
-  const bool lone = is_auto && items == 1 && !big && core_max >= 2048;
+  const int64_t lone_mean = stream || P.opts.precision == TTG_PREC_MIXED ? 640 : 1024;
+  const bool lone = is_auto && items == 1 && !big && core_max >= 2048 &&
+                    size_sum >= lone_mean * cores;
   const bool few = is_auto && items > 1 && items <= std::max(device().sms, 1) / 5 && !stream &&
                    !(items <= 4 && big) && c_max <= 112 && size_sum >= 2048 * cores &&
                    P.opts.precision != TTG_PREC_MIXED;
