@@ -1121,8 +1121,8 @@ int32_t first_bad_status(const ttg_plan& P)
 
 // State of the one-shot entry points, one set per device: the stream they
 // run on, the lock that serialises them, and the buffers they reuse
-// (grow-only, guarded by the lock), so repeated calls do not pay cudaMalloc /
-// cudaHostAlloc again.  Calls on different devices (the multi-device batch
+// (guarded by the lock; PoolLease says what they keep), so repeated calls do not
+// pay cudaMalloc / cudaHostAlloc again.  Calls on different devices (the multi-device batch
 // entries run one host thread per device) proceed in parallel.
 constexpr int kMaxDevices = 64;
 
@@ -1161,8 +1161,14 @@ cudaStream_t lib_stream2()
   return s.stream2;
 }
 
+// What the whole-GPU work buffers, and calls that trim, leave in the pools.
+constexpr size_t kPoolKeep = size_t{1} << 30;
+
 // Lends the device's buffers (slot 0, or slot 1 for the second plan of a
-// pipelined batch) to a plan for one call, and takes them back grown.
+// pipelined batch) to a plan for one call, and takes them back grown.  trim:
+// buffers that this call grew beyond kPoolKeep are freed (an inner product or
+// an evaluation of a few GB is no reason to hold them: allocating them again
+// takes less than the call).
 struct PoolLease
 {
   ttg_plan& P;
@@ -1170,13 +1176,25 @@ struct PoolLease
   DevMem& dev;
   HostPinned& host;
   const bool wide;  // slot 0 also lends the whole-GPU work buffers
-  explicit PoolLease(ttg_plan& p, int slot = 0)
+  const bool trim;
+  const size_t had_dev, had_host;
+  explicit PoolLease(ttg_plan& p, int slot = 0, bool trim_ = false)
     : P(p), D(dev_state()), dev(slot ? D.dev_pool2 : D.dev_pool),
-      host(slot ? D.host_pool2 : D.host_pool), wide(slot == 0)
+      host(slot ? D.host_pool2 : D.host_pool), wide(slot == 0), trim(trim_), had_dev(dev.bytes),
+      had_host(host.bytes)
   {
     swap();
   }
-  ~PoolLease() { swap(); }
+  ~PoolLease()
+  {
+    swap();
+    if (wide && D.wide_pool.bytes > kPoolKeep)
+      D.wide_pool.release();
+    if (trim && dev.bytes > std::max(kPoolKeep, had_dev))
+      dev.release();
+    if (trim && host.bytes > std::max(kPoolKeep, had_host))
+      host.release();
+  }
   void swap()
   {
     std::swap(P.dev.p, dev.p);
@@ -2091,7 +2109,7 @@ int32_t ttg_right_orthogonalize(const ttg_tensor* in, ttg_tensor* out)
   std::lock_guard<std::mutex> lk(dev_state().mu);
   ttg_round_options o{};
   ttg_plan P;
-  PoolLease lease(P);
+  PoolLease lease(P, 0, true);
   P.one_shot = true;
   if (int32_t st = build_round_plan(P, 1, in, &o, "right_orthogonalize", kJobRightOrth))
     return st;
@@ -2120,7 +2138,7 @@ int32_t ttg_left_orthogonalize(const ttg_tensor* in, ttg_tensor* out)
   std::lock_guard<std::mutex> lk(dev_state().mu);
   ttg_round_options o{};
   ttg_plan P;
-  PoolLease lease(P);
+  PoolLease lease(P, 0, true);
   P.one_shot = true;
   if (int32_t st = build_round_plan(P, 1, in, &o, "left_orthogonalize", kJobLeftOrth))
     return st;
@@ -2692,7 +2710,7 @@ int32_t ttg_inner(const ttg_tensor* a, const ttg_tensor* b, double* out)
     return st;
   std::lock_guard<std::mutex> lk(dev_state().mu);
   ttg_plan P;
-  PoolLease lease(P);
+  PoolLease lease(P, 0, true);
   P.shapes = {A, B};
   add_tensor(P, A, true, nullptr);
   add_tensor(P, B, true, nullptr);
@@ -2763,7 +2781,7 @@ int32_t ttg::eval_batch_part(const ttg_tensor* a, const int32_t* idx, int32_t M,
     return st;
   std::lock_guard<std::mutex> lk(dev_state().mu);
   ttg_plan P;
-  PoolLease lease(P);
+  PoolLease lease(P, 0, true);
   if (int32_t st = build_eval_plan(P, a, idx, M, M_all))
     return st;
   if (M == 0)
