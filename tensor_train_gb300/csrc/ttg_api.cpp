@@ -310,6 +310,8 @@ struct ttg_plan
   // (direct, set in layout_and_alloc) instead of through the pinned image.
   bool one_shot = false;
   bool direct = false;
+  // From the first upload until the results were waited for.
+  bool in_flight = false;
   // eval plans
   const int32_t* eval_idx = nullptr;
   int64_t M = 0;
@@ -922,6 +924,7 @@ int32_t build_round_plan(ttg_plan& P, int32_t count, const ttg_tensor* ins,
 int32_t plan_upload(ttg_plan& P, cudaStream_t st)
 {
   char* d = static_cast<char*>(P.dev.p);
+  P.in_flight = true;
   if (!P.direct)
   {
     TTG_CUDA(cudaMemcpyAsync(d + P.off_pristine, P.host.p, P.prefix_bytes, cudaMemcpyHostToDevice,
@@ -1020,6 +1023,7 @@ int32_t plan_download_raw(ttg_plan& P, cudaStream_t st)
     TTG_CUDA(cudaMemcpyAsync(bars.data(), P.wjob.bar, sizeof(GridBar) * bars.size(),
                              cudaMemcpyDeviceToHost, st));
   TTG_CUDA(cudaStreamSynchronize(st));
+  P.in_flight = false;
   if (P.wide)
     for (const GridBar& bar : bars)
       if (bar.err)
@@ -1187,6 +1191,8 @@ struct PoolLease
   }
   ~PoolLease()
   {
+    if (P.in_flight)  // a call that failed half-way: nothing may touch the caller's memory later
+      cudaStreamSynchronize(wide ? lib_stream() : lib_stream2());
     swap();
     if (wide && D.wide_pool.bytes > kPoolKeep)
       D.wide_pool.release();
@@ -1528,6 +1534,7 @@ int32_t ttg_plan_download(ttg_plan* P, void* stream, ttg_tensor* outs, double* v
                              cudaMemcpyDeviceToHost, st));
     TTG_CUDA(cudaMemcpyAsync(&bad, d + P->off_bad, sizeof(int), cudaMemcpyDeviceToHost, st));
     TTG_CUDA(cudaStreamSynchronize(st));
+    P->in_flight = false;
     if (bad)
       return fail(TTG_ERR_INDEX, "eval_at: idx out of range");
     return TTG_OK;
@@ -2476,6 +2483,7 @@ static int32_t run_inner(ttg_plan& P, const double* arena, const CoreSlot* SA, c
   } got{};
   TTG_CUDA(cudaMemcpyAsync(&got, tail, sizeof(got), cudaMemcpyDeviceToHost, st));
   TTG_CUDA(cudaStreamSynchronize(st));
+  P.in_flight = false;
   if (got.bar.err)
     return fail(TTG_ERR_TIMEOUT, std::string(op) + ": a grid barrier wait timed out");
   *out = got.v;
@@ -2655,6 +2663,7 @@ static int32_t build_eval_plan(ttg_plan& P, const ttg_tensor* a, const int32_t* 
 static int32_t eval_upload(ttg_plan& P, cudaStream_t st)
 {
   char* d = static_cast<char*>(P.dev.p);
+  P.in_flight = true;
   TTG_CUDA(cudaMemcpyAsync(d, P.host.p, P.off_order, cudaMemcpyHostToDevice, st));
   if (P.M > 0)
     TTG_CUDA(cudaMemcpyAsync(d + P.off_idx, P.eval_idx,
