@@ -1,6 +1,6 @@
 // FP64 pieces shared by the blocked Householder routines (ttg_wide_qr.cuh,
-// ttg_wy.cuh): the scalars of a reflector and the reduction of a block's 16
-// products.
+// ttg_wy.cuh): the scalars of a reflector, the reduction of a block's 16
+// products and the columns of its T.
 #pragma once
 
 #include <cfloat>
@@ -84,6 +84,32 @@ __device__ __forceinline__ void halving_sum(double (&acc)[16], int gl)
   }
   if (G == 32)
     acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+}
+
+// Column i of a block's T = -tau_i T(0:i, 0:i) G(0:i, i), T(i, i) = tau_i, by
+// the 32 lanes of a warp; G = V^T V above the diagonal, T upper triangular,
+// both 16 x 16 and column-major in ps.
+template <class Shared>
+__device__ __forceinline__ void t_column(Shared& ps, int i)
+{
+  constexpr int kB = 16;
+  static_assert(sizeof(ps.T) == kB * kB * sizeof(double), "16 reflectors per block");
+  // Two lanes per row, each half of the sum.
+  const int lane = threadIdx.x & 31, l = lane & (kB - 1), half = lane / kB;
+  const double nt = -ps.tau[i];
+  const double g = nt * ps.G[l + i * kB];  // lane q's term is -tau_i G(q, i)
+  double acc = 0.0;
+  for (int q0 = 0; q0 < i; q0 += 2)  // the same trips on every lane
+  {
+    const int q = q0 + half;
+    const double gq = __shfl_sync(0xffffffffu, g, q);
+    if (l <= q && q < i)
+      acc = fma(ps.T[l + q * kB], gq, acc);
+  }
+  acc += __shfl_xor_sync(0xffffffffu, acc, kB);
+  if (half == 0)
+    ps.T[l + i * kB] = l < i ? acc : (l == i ? -nt : 0.0);
+  __syncwarp();
 }
 
 }  // namespace

@@ -18,8 +18,8 @@
 //     column group only.  Q's tiles stay in shared memory over all blocks.
 //
 // An exchange is one 16-byte packet per value, {low word, tag, high word,
-// tag}: each 8-byte half says by its tag that it has arrived (8-byte accesses
-// are single), so a reader needs no fence and no flag, only a poll of the
+// tag}, the line of NCCL's low-latency (LL) protocol: each 8-byte half says by
+// its tag that it has arrived (8-byte accesses are single), so a reader needs no fence and no flag, only a poll of the
 // packet itself.  Tags never repeat within a launch, and the packets are
 // zeroed before it.  Packet buffers alternate by the tag's parity: a CTA two
 // exchanges ahead has all packets of the one between, whose senders have read
@@ -145,28 +145,6 @@ struct PanelShared
   double inv[kPb], tau[kPb];
 };
 
-// Column i of T = -tau_i T(0:i, 0:i) G(0:i, i), T(i, i) = tau_i, by the 32
-// lanes of a warp.
-__device__ __forceinline__ void panel_t_column(PanelShared& ps, int i)
-{
-  // Two lanes per row, each half of the sum.
-  const int lane = threadIdx.x & 31, l = lane & (kPb - 1), half = lane / kPb;
-  const double nt = -ps.tau[i];
-  const double g = nt * ps.G[l + i * kPb];  // lane q's term is -tau_i G(q, i)
-  double acc = 0.0;
-  for (int q0 = 0; q0 < i; q0 += 2)  // the same trips on every lane
-  {
-    const int q = q0 + half;
-    const double gq = __shfl_sync(0xffffffffu, g, q);
-    if (l <= q && q < i)
-      acc = fma(ps.T[l + q * kPb], gq, acc);
-  }
-  acc += __shfl_xor_sync(0xffffffffu, acc, kPb);
-  if (half == 0)
-    ps.T[l + i * kPb] = l < i ? acc : (l == i ? -nt : 0.0);
-  __syncwarp();
-}
-
 // Factors columns j0 .. j0 + nb of W (h rows) on the first S CTAs of the
 // team, `rows` rows from j0 on each.  On return W holds the explicit V (from
 // row j0 on), R its entries, job.Tw the block's T.  Tags seq .. seq + nb.
@@ -227,7 +205,7 @@ __device__ __noinline__ bool wide_panel(const WideJob& job, int h, int k, int j0
     }
     // T's previous column while the packets travel (the first CTA's T is used).
     if (me == 0 && w == 6 && i > 0)
-      panel_t_column(ps, i - 1);
+      t_column(ps, i - 1);
     if (S > 1 && t < 8 * kPb)
     {
       const int l = t >> 3, g = t & 7;
@@ -307,7 +285,7 @@ __device__ __noinline__ bool wide_panel(const WideJob& job, int h, int k, int j0
     __syncthreads();
   }
   if (me == 0 && w == 6)
-    panel_t_column(ps, nb - 1);
+    t_column(ps, nb - 1);
   // R's entries and the explicit V.
   for (int i = w; i < nb; i += kWarps)
   {

@@ -43,27 +43,6 @@ __device__ __forceinline__ int64_t wy_t_need(int c)
   return static_cast<int64_t>((c + kWb - 1) / kWb) * kWb * kWb;
 }
 
-// Column i of T = -tau_i T(0:i, 0:i) G(0:i, i), T(i, i) = tau_i (one warp).
-__device__ __forceinline__ void wy_t_column(WyShared& ps, int i)
-{
-  // Two lanes per row, each half of the sum.
-  const int lane = threadIdx.x & 31, l = lane & (kWb - 1), half = lane / kWb;
-  const double nt = -ps.tau[i];
-  const double g = nt * ps.G[l + i * kWb];  // lane q's term is -tau_i G(q, i)
-  double acc = 0.0;
-  for (int q0 = 0; q0 < i; q0 += 2)  // the same trips on every lane
-  {
-    const int q = q0 + half;
-    const double gq = __shfl_sync(0xffffffffu, g, q);
-    if (l <= q && q < i)
-      acc = fma(ps.T[l + q * kWb], gq, acc);
-  }
-  acc += __shfl_xor_sync(0xffffffffu, acc, kWb);
-  if (half == 0)
-    ps.T[l + i * kWb] = l < i ? acc : (l == i ? -nt : 0.0);
-  __syncwarp();
-}
-
 // Householder factorisation of P (hp x nb, nb <= kWb, ld ldp) in place: R on
 // and above the diagonal, the unscaled tails below (v_i = inv_i x_i).  ps:
 // inv, tau and T of the block (zero past nb).  Ends with a barrier.
@@ -96,7 +75,7 @@ __device__ __noinline__ void wy_panel(double* P, int64_t ldp, int hp, int nb, Wy
       }
     }
     else if (w == 6 && i > 0)
-      wy_t_column(ps, i - 1);
+      t_column(ps, i - 1);
     __syncthreads();
     // tau inv = +-1 / n: warp 0 forms what the update waits for, warps 1 and
     // 2 (on other pipes, the same scalars again) the rest.
@@ -152,7 +131,7 @@ __device__ __noinline__ void wy_panel(double* P, int64_t ldp, int hp, int nb, Wy
     __syncthreads();
   }
   if (w == 6)
-    wy_t_column(ps, nb - 1);
+    t_column(ps, nb - 1);
   __syncthreads();
 }
 
