@@ -46,8 +46,11 @@ int32_t fail(int32_t st, const std::string& msg)
   {                                                                                  \
     cudaError_t e_ = (call);                                                         \
     if (e_ != cudaSuccess)                                                           \
+    {                                                                                \
+      cudaGetLastError(); /* this call's alone, not the next one's */                \
       return fail(e_ == cudaErrorMemoryAllocation ? TTG_ERR_OOM : TTG_ERR_CUDA,      \
-                  std::string(#call) + ": " + cudaGetErrorString(e_));              \
+                  std::string(#call) + ": " + cudaGetErrorString(e_));               \
+    }                                                                                \
   } while (0)
 
 struct DeviceInfo

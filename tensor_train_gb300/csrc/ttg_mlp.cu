@@ -157,8 +157,11 @@ int32_t mfail(int32_t st, const std::string& m)
   {                                                                                    \
     cudaError_t e_ = (call);                                                           \
     if (e_ != cudaSuccess)                                                             \
+    {                                                                                  \
+      cudaGetLastError(); /* this call's alone, not the next one's */                  \
       return mfail(e_ == cudaErrorMemoryAllocation ? TTG_ERR_OOM : TTG_ERR_CUDA,       \
-                   std::string(#call) + ": " + cudaGetErrorString(e_));               \
+                   std::string(#call) + ": " + cudaGetErrorString(e_));                \
+    }                                                                                  \
   } while (0)
 
 int32_t ensure_rows(ttg_mlp* m, int rows)
