@@ -286,12 +286,19 @@ __global__ void __launch_bounds__(32 * kEvalWarps)
 // 129 MB L2 beside the vector tables' lines in use; a vector table is read
 // once per index, from HBM at worst.
 constexpr double kMatDoubles = 6.0e6, kMatTotal = 1.3e7, kVecDoubles = 1.7e7;
-// FMAs that one more launch is worth: ~3 us at the chip's 0.6 TFMA/s.
+// FMAs that one more launch is worth: ~3 us at the chip's 0.6 TFMA/s (0 / 5e5 /
+// 2e6 / 8e6, d=30 n=2 rank 16: 3000 indices 0.29 / 0.29 / 0.20 / 0.20 ms, 30 000
+// 0.42 / 0.41 / 0.41 / 0.61).
 constexpr double kLaunchFma = 2.0e6;
 constexpr int kMostSites = 16;
 // Matrix tables from this many indices on; column-vector tables of at most
 // kRightN entries (and never past the middle), so that where the two vectors
-// meet depends on the train alone.
+// meet depends on the train alone.  Matrix tables on : off, ms: d=32 n=4 rank 64
+// 8000 indices 1.45 : 1.93, 32 768 2.76 : 4.91, 2^20 28.9 : 110; rank 16 16 000
+// 0.44 : 0.39, 32 768 0.50 : 0.55, 131 072 0.79 : 1.33; d=12 n=8 rank 24 32 768
+// 0.33 : 0.38.  kRightN of 1 / 256 / 4096 / 65536 / 1e6, 3e5 indices: d=32 n=4 rank
+// 64 12.3 / 19.6 / 18.6 / 10.9 / 12.9 ms, d=10 n=16 rank 30 1.64 / 1.55 / 1.25 / 1.14
+// / 1.15; 3e4 indices 5.2 / 4.9 / 4.5 / 4.8 / 5.0 and 0.49 / 0.44 / 0.41 / 0.43 / 0.43.
 constexpr int64_t kMatM = 1 << 15;
 constexpr double kRightN = 65536;
 
@@ -504,7 +511,10 @@ namespace
 {
 
 // Shape of a launch: lanes per index (the largest rank, 8 to 32), warps per
-// CTA, whether the segments and indices are staged, shared memory.
+// CTA, whether the segments and indices are staged, shared memory.  8 / 16 / 32
+// lanes, d=20 n=4, ms: 33 indices of rank 9 0.116 / 0.106 / 0.106, 24 0.20 / 0.18 /
+// 0.13, 32 0.30 / 0.21 / 0.16 (more lanes shorten one index's chain); 3e5 of rank 8
+// 0.46 / 0.54 / 0.67, 12 0.57 / 0.62 / 0.77, 32 1.27 / 1.31 / 1.37.
 struct EvalShape
 {
   int lanes, warps;
