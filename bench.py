@@ -32,9 +32,9 @@ METRIC = ("TT roundings/sec and matvec_round/sec at rel. err<=1e-8: mixed/learne
 EPS = 1e-8
 SEED0 = 1000
 # DRAM bytes (read + write) of one mixed round_kernel launch on TTs 1000..1607
-# of the batch at the mixed default of 3 CTAs per SM (ncu,
+# of the batch at 3 CTAs per SM, the mixed default of the 4096-TT batch (ncu,
 # profiles/round_kernel_batch608_ncu.md).
-TRAFFIC_608 = 6.161341952e9 + 9.316889088e9
+TRAFFIC_608 = 6.589021184e9 + 9.897978112e9
 
 
 def measured_peaks(path=None):

@@ -235,7 +235,9 @@ int32_t ttg_matmat(const ttg_tensor* A, const ttg_tensor* B, ttg_tensor* out);
 /* ---- evaluation and inner products ------------------------------------
  * Replaces: std::vector<double> eval_batch(const tt&, const int* idx, int M)
  *           (algebra/tt_eval.hpp:86-112); idx is M x d row-major; out has M
- *           entries (caller-owned). */
+ *           entries (caller-owned).  From 32 768 indices on, products of
+ *           neighbouring cores are formed once and looked up: a value's last
+ *           bits may then differ from those of a smaller call. */
 int32_t ttg_eval_batch(const ttg_tensor* a, const int32_t* idx, int32_t M, double* out);
 
 /* Replaces: double inner(const tt&, const tt&) and double norm(const tt&)

@@ -282,7 +282,8 @@ class _Owned:
 
 
 def _take(t: _Tensor):
-    """The cores of an output tensor: arrays on its buffer, which they own."""
+    """The cores of an output tensor: arrays on its one buffer, which lives as
+    long as any of them (copy a core to keep it alone)."""
     d = t.d
     if d == 0:
         lib().ttg_free(C.byref(t))
